@@ -58,7 +58,7 @@ namespace sg {
 
 void launch_mlp_forward(const float *X, uint32_t n, uint32_t F, uint32_t H, const uint16_t *W1, const float *b1,
                         const uint16_t *W2, const float *b2, const uint16_t *w3, const float *b3, float *Z1,
-                        float *Z2, float *P, cudaStream_t st);
+                        float *Z2, float *P, uint32_t *dev_err, cudaStream_t st, int n_sm);
 
 namespace {
 
@@ -442,7 +442,7 @@ void Miner::score(const std::vector<float> &feat, size_t n, std::vector<float> &
     hscore_.reserve(n * 4);
     launch_mlp_forward(X, (uint32_t)n, kDim, sc.hidden, sc.w1.as<uint16_t>(), sc.b1.as<float>(), sc.w2.as<uint16_t>(),
                        sc.b2.as<float>(), sc.w3.as<uint16_t>(), sc.b3.as<float>(), nullptr, nullptr,
-                       score_.as<float>(), st);
+                       score_.as<float>(), h_->dev_err.as<uint32_t>(), st, h_->n_sm);
     ++launches_;
     SG_CUDA_TRY(cudaMemcpyAsync(hscore_.ptr, score_.ptr, n * 4, cudaMemcpyDeviceToHost, st));
     h_->sync();

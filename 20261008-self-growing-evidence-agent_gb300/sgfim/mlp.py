@@ -89,8 +89,7 @@ class Trainer:
         WT = WT.to(self.dev, torch.float32).contiguous() if WT is not None else None
         n = X.shape[0]
         P, Z1, Z2 = self.forward(X, keep=True)
-        for t in self.g.values():
-            t.zero_()
+        torch._foreach_zero_(list(self.g.values()))
         loss = torch.zeros(1, dtype=torch.float32, device=self.dev)
         self.eng.mlp_backward(X.data_ptr(), n, self.in_dim, self.hidden, self.b16["W2"].data_ptr(),
                               self.b16["w3"].data_ptr(), Z1.data_ptr(), Z2.data_ptr(), P.data_ptr(), Y.data_ptr(),
