@@ -140,6 +140,7 @@ void sgfim_close(sgfim_handle *h) {
     h->ds.ext_cooc.release();
     h->ds.ext_d2o.release();
     h->ext.release();
+    h->tx.release();
     h->support_scratch.release();
     h->cand_ptr_dev.release();
     h->cand_items_dev.release();

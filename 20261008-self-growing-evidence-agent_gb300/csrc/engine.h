@@ -165,6 +165,15 @@ struct ExtWorkspace {
     }
 };
 
+// Device buffers of the transactionisation calls.
+struct TxWorkspace {
+    DevBuf rows, cols, small, anom, items;
+    size_t bytes() const { return rows.bytes + cols.bytes + small.bytes + anom.bytes + items.bytes; }
+    void release() {
+        for (DevBuf *b : {&rows, &cols, &small, &anom, &items}) b->release();
+    }
+};
+
 // MLP scorer weights (device) for the learned frontier order.
 struct Scorer {
     bool loaded = false;
@@ -190,6 +199,7 @@ struct sgfim_handle {
     sg::MinerWorkspace mws;
     sg::WindowWorkspace wws;
     sg::ExtWorkspace ext;
+    sg::TxWorkspace tx;
     sg::SupportPlan plan;
     uint64_t launches = 0;
     cudaEvent_t ev_a = nullptr, ev_b = nullptr;
