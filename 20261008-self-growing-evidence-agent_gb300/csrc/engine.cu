@@ -387,7 +387,7 @@ int sgfim_support_batch_device(sgfim_handle *h, const uint64_t *bitmaps, uint32_
         map_ptr = map_ok ? bitmaps : nullptr;
         map_key[0] = d; map_key[1] = n_even; map_key[2] = row_stride;
     }
-    h->support_scratch.reserve(support_scratch_bytes(n_cand), st);
+    h->support_scratch.reserve(support_scratch_bytes(n_cand, d, n_even, h->plan), st);
     SupportScratch sc{h->support_scratch.ptr, h->support_scratch.bytes};
     const SupportPlan &plan = h->plan;
     const uint64_t n_txn = n_words * 64;
@@ -438,7 +438,7 @@ int sgfim_support_batch(sgfim_handle *h, const uint64_t *cand_ptr, const uint32_
     SG_CUDA_TRY(cudaMemcpyAsync(&bad_h, d_bad, 4, cudaMemcpyDeviceToHost, h->stream));
     SG_CUDA_TRY(cudaStreamSynchronize(h->stream));
     if (bad_h) return fail(h, SGFIM_EINVAL, "cand_ptr must be non-decreasing");
-    h->support_scratch.reserve(support_scratch_bytes(n_cand), h->stream);
+    h->support_scratch.reserve(support_scratch_bytes(n_cand, ds.d, ds.n_words, h->plan), h->stream);
     SupportScratch sc{h->support_scratch.ptr, h->support_scratch.bytes};
     const SupportPlan &plan = h->plan;
     const uint64_t before = h->launches;
@@ -459,7 +459,7 @@ int sgfim_support_batch(sgfim_handle *h, const uint64_t *cand_ptr, const uint32_
 
 int sgfim_support_plan_set(sgfim_handle *h, int kernel, uint32_t cands_per_cta, uint32_t waves) {
     if (!h) return SGFIM_EINVAL;
-    if (kernel < SGFIM_KERNEL_AUTO || kernel > SGFIM_KERNEL_LANE_TM) return fail(h, SGFIM_EINVAL, "unknown kernel");
+    if (kernel < SGFIM_KERNEL_AUTO || kernel > SGFIM_KERNEL_PAIR) return fail(h, SGFIM_EINVAL, "unknown kernel");
     h->plan.kernel = kernel;
     h->plan.cands_per_cta = cands_per_cta;
     h->plan.waves = waves;

@@ -30,8 +30,6 @@ struct QueryBatch {
     const uint64_t *arena = nullptr;
     uint64_t arena_stride = 0;
     uint64_t n_q = 0;
-    const uint64_t *n_q_device = nullptr;  // when set, the query count is read on the device
-    const uint32_t *q_index = nullptr;     // optional indirection: query j is q_index[j]
     const uint64_t *q_w0 = nullptr;        // optional first word of each query (words before it are skipped)
     uint32_t *out = nullptr;
     uint64_t empty_value = 0;       // result of an empty query without mask
@@ -59,7 +57,7 @@ void launch_tail_counts(const uint64_t *rows, uint64_t row_stride, uint64_t n_wo
 // shared-memory staged kernel on those and the streaming kernel on the rest.
 enum SupportKernel : int {
     SUPPORT_AUTO = 0, SUPPORT_STAGED = 1, SUPPORT_SORTED = 2, SUPPORT_STREAM = 3, SUPPORT_STAGED4 = 4,
-    SUPPORT_LANE = 5, SUPPORT_LANE_TM = 6
+    SUPPORT_LANE = 5, SUPPORT_LANE_TM = 6, SUPPORT_PAIR = 7
 };
 struct SupportPlan {
     int kernel = SUPPORT_AUTO;
@@ -79,7 +77,8 @@ struct SupportScratch {
     void *base = nullptr;
     size_t bytes = 0;
 };
-size_t support_scratch_bytes(uint64_t n_cand);
+// scratch that lets every kernel the plan may choose run
+size_t support_scratch_bytes(uint64_t n_cand, uint32_t d, uint64_t n_words, const SupportPlan &plan);
 // ev (optional, 4 events): recorded before prep, before the counting kernel,
 // after it, and after the >8-item tail.
 int support_batch_device(const uint64_t *bitmaps, uint32_t d, uint64_t n_words, uint64_t row_stride,
@@ -91,20 +90,31 @@ int support_batch_device(const uint64_t *bitmaps, uint32_t d, uint64_t n_words, 
 // TMA.  Returns -1 when d or the shared-memory layout does not fit (the caller
 // then takes another kernel); otherwise the >8-item candidates are left in
 // *ovf_list / *ovf_count (device) for the streaming kernel.  ev (optional):
-// ev[1] and ev[2] are recorded around the counting kernel.
+// ev[1] and ev[2] are recorded around the counting kernel.  gate (optional, device): the
+// kernels leave everything alone when it holds 0.
 bool lane_supported(uint32_t d);
+// Candidates grouped by their two rarest rows (kernels_pair.cu); -1 when the
+// shape or the scratch does not allow it.  gated: the supports are left alone,
+// and **dense is non-zero on the device, when the data are too dense for it.
+bool pair_supported(uint32_t d, uint64_t n_cand);
+size_t pair_scratch_bytes(uint64_t n_cand, uint32_t d);
+int pair_supports_device(const CUtensorMap *map, const uint64_t *bitmaps, uint32_t d, uint64_t n_words,
+                         uint64_t row_stride, const uint64_t *cand_ptr, const uint32_t *cand_items, uint64_t n_cand,
+                         uint64_t n_txn, uint32_t *out, void *scratch, size_t scratch_bytes, bool gated,
+                         uint32_t *dev_err, cudaStream_t st, int n_sm, const uint32_t **dense, uint32_t **ovf_list,
+                         unsigned long long **ovf_count, uint64_t *launches, cudaEvent_t *ev);
 // The same counting with the records and totals in tensor memory and a ring of
 // shared-memory box slots that loads the next chunk during the current one.
 int lane_tm_supports_device(const CUtensorMap *map, uint32_t d, uint64_t n_words, const uint64_t *cand_ptr,
                             const uint32_t *cand_items, uint64_t n_cand, uint64_t n_txn, uint32_t *out, void *scratch,
                             size_t scratch_bytes, uint32_t waves, uint32_t *dev_err, cudaStream_t st, int n_sm,
                             uint32_t **ovf_list, unsigned long long **ovf_count, uint64_t *launches,
-                            cudaEvent_t *ev);
+                            cudaEvent_t *ev, const uint32_t *gate = nullptr);
 int lane_supports_device(const CUtensorMap *map, uint32_t d, uint64_t n_words, const uint64_t *cand_ptr,
                          const uint32_t *cand_items, uint64_t n_cand, uint64_t n_txn, uint32_t *out, void *scratch,
                          size_t scratch_bytes, uint32_t waves, uint32_t *dev_err, cudaStream_t st, int n_sm,
                          uint32_t **ovf_list, unsigned long long **ovf_count, uint64_t *launches,
-                         cudaEvent_t *ev);
+                         cudaEvent_t *ev, const uint32_t *gate = nullptr);
 // Encode the 2-D tensor map used by the staged kernel (rows x words, u64).
 bool encode_bitmap_map(CUtensorMap *map, const uint64_t *bitmaps, uint32_t d, uint64_t n_words,
                        uint64_t row_stride);

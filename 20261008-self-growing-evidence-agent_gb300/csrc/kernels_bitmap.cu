@@ -172,9 +172,7 @@ __global__ void __launch_bounds__(256) query_kernel(QueryBatch qb) {
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
     const uint64_t n_warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    const uint64_t n_q = qb.n_q_device ? *qb.n_q_device : qb.n_q;
-    for (uint64_t j = warp; j < n_q; j += n_warps) {
-        const uint64_t q = qb.q_index ? qb.q_index[j] : j;
+    for (uint64_t q = warp; q < qb.n_q; q += n_warps) {
         const uint64_t a = qb.q_ptr[q], b = qb.q_ptr[q + 1];
         const uint64_t *mask = nullptr;
         if (qb.mask_slot) {
@@ -252,14 +250,115 @@ void launch_tail_counts(const uint64_t *rows, uint64_t row_stride, uint64_t n_wo
 }
 
 void launch_queries(const QueryBatch &qb, cudaStream_t st, int n_sm) {
-    uint64_t blocks;
-    if (qb.n_q_device) {
-        blocks = (uint64_t)n_sm * 8;
-    } else {
-        if (qb.n_q == 0) return;
-        blocks = std::min<uint64_t>((qb.n_q + 7) / 8, (uint64_t)n_sm * 64);
-    }
+    if (qb.n_q == 0) return;
+    const uint64_t blocks = std::min<uint64_t>((qb.n_q + 7) / 8, (uint64_t)n_sm * 64);
     query_kernel<<<(unsigned)blocks, 256, 0, st>>>(qb);
+    SG_CUDA_TRY(cudaGetLastError());
+}
+
+// ---------------------------------------------------------------- streamed batch supports
+// Supports of CSR candidates straight from L2/HBM: a warp owns one segment of
+// one candidate's rows.  A step covers kStreamU x 64 words, two rows at a time
+// (eight 16-byte loads in flight per lane), and rows are read only where the
+// AND of the rows before them still has a bit.  With more than one segment the
+// warps add into out, which holds zeros (an empty candidate's support comes
+// from its first segment).  Short segments fill the chip
+// when candidates are few and keep its last wave short: over 1,000,000
+// transactions 300 candidates take 23 us and 3,000 130 us (one warp per candidate:
+// 384 and 420 us), 200,000 run at 22 TB/s from L1 and L2.
+constexpr int kStreamU = 4;
+constexpr uint32_t kStreamStep = 64 * kStreamU;   // words a warp covers per step
+
+struct StreamBatch {
+    const uint64_t *rows;
+    uint64_t stride, n_words;
+    uint32_t d;
+    const uint64_t *cand_ptr;
+    const uint32_t *items;
+    uint64_t n;                       // candidates (entries of index, when given)
+    const uint64_t *n_device;         // when set, the count is read on the device
+    const uint32_t *index;            // optional: entry j is candidate index[j]
+    uint64_t n_txn;
+    uint64_t seg_words;               // multiple of 2
+    uint32_t n_seg;
+    uint32_t *out;
+};
+
+__global__ void __launch_bounds__(256) cand_stream_kernel(StreamBatch sb) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t n_warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    const uint64_t total = (sb.n_device ? *sb.n_device : sb.n) * sb.n_seg;
+    for (uint64_t q = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; q < total; q += n_warps) {
+        const uint64_t j = q / sb.n_seg;
+        const uint64_t c = sb.index ? sb.index[j] : j, seg = q - j * sb.n_seg;
+        const uint64_t a = sb.cand_ptr[c], k = sb.cand_ptr[c + 1] - a;
+        uint32_t acc = 0;
+        if (k == 0) {
+            acc = seg == 0 ? (uint32_t)sb.n_txn : 0u;
+        } else {
+            // the first 32 items travel in the lanes
+            const uint32_t mine = lane < k ? sb.items[a + lane] : 0u;
+            bool bad = mine >= sb.d;
+            for (uint64_t i = 32 + lane; i < k; i += 32) bad |= sb.items[a + i] >= sb.d;
+            if (!__any_sync(0xffffffffu, bad)) {
+                const uint64_t w0 = seg * sb.seg_words, w1 = min(sb.n_words, w0 + sb.seg_words);
+                uint32_t part = 0;
+                for (uint64_t base = w0; base < w1; base += kStreamStep) {
+                    const uint64_t *at = sb.rows + base + 2 * lane;
+                    uint4 v[kStreamU];
+                    const uint64_t *r0 = at + (uint64_t)__shfl_sync(0xffffffffu, mine, 0) * sb.stride;
+#pragma unroll
+                    for (int u = 0; u < kStreamU; ++u)
+                        v[u] = base + 64 * u + 2 * lane < w1 ? ld_nc_v4(r0 + 64 * u) : make_uint4(0, 0, 0, 0);
+                    for (uint64_t i = 1; i < k; i += 2) {
+                        const uint64_t i2 = i + 1 < k ? i + 1 : i;   // an odd count ANDs its last row twice
+                        const uint32_t x = i < 32 ? __shfl_sync(0xffffffffu, mine, (int)i) : sb.items[a + i];
+                        const uint32_t y = i2 < 32 ? __shfl_sync(0xffffffffu, mine, (int)i2) : sb.items[a + i2];
+                        const uint64_t *rx = at + (uint64_t)x * sb.stride, *ry = at + (uint64_t)y * sb.stride;
+                        uint4 p[kStreamU], o[kStreamU];
+                        bool any = false;
+#pragma unroll
+                        for (int u = 0; u < kStreamU; ++u) {
+                            const bool live = (v[u].x | v[u].y | v[u].z | v[u].w) != 0;
+                            p[u] = o[u] = make_uint4(0, 0, 0, 0);
+                            if (live) {
+                                p[u] = ld_nc_v4(rx + 64 * u);
+                                o[u] = ld_nc_v4(ry + 64 * u);
+                            }
+                            any |= live;
+                        }
+#pragma unroll
+                        for (int u = 0; u < kStreamU; ++u) v[u] = and4(v[u], and4(p[u], o[u]));
+                        if (!__any_sync(0xffffffffu, any)) break;
+                    }
+#pragma unroll
+                    for (int u = 0; u < kStreamU; ++u) part += popc4(v[u]);
+                }
+                acc = warp_sum(part);
+            }
+        }
+        if (lane == 0) {
+            if (sb.n_seg == 1) sb.out[c] = acc;
+            else if (acc) atomicAdd(&sb.out[c], acc);
+        }
+    }
+}
+
+// All n candidates (index null), or the listed ones, whose outputs hold zeros.
+static void launch_cand_stream(StreamBatch sb, cudaStream_t st, int n_sm) {
+    const uint64_t warps = (uint64_t)n_sm * 128;   // four times what the chip holds at once: short tails
+    const uint64_t most = std::max<uint64_t>(1, (sb.n_words + kStreamStep - 1) / kStreamStep);
+    if (sb.n_device) {
+        sb.n_seg = (uint32_t)std::min<uint64_t>(8, most);
+    } else {
+        if (sb.n == 0) return;
+        sb.n_seg = (uint32_t)std::min<uint64_t>(most, std::max<uint64_t>(1, warps / sb.n));
+        if (sb.n_seg > 1) SG_CUDA_TRY(cudaMemsetAsync(sb.out, 0, sb.n * 4, st));
+    }
+    sb.seg_words = ((sb.n_words + sb.n_seg - 1) / sb.n_seg + kStreamStep - 1) / kStreamStep * kStreamStep;
+    const uint64_t blocks =
+        sb.n_device ? (uint64_t)n_sm * 8 : std::min<uint64_t>((sb.n * sb.n_seg + 7) / 8, (uint64_t)n_sm * 64);
+    cand_stream_kernel<<<(unsigned)blocks, 256, 0, st>>>(sb);
     SG_CUDA_TRY(cudaGetLastError());
 }
 
@@ -283,6 +382,7 @@ __global__ void prep_records_kernel(const uint64_t *__restrict__ cand_ptr, const
         } else if (k > 8) {
             const unsigned long long slot = atomicAdd(ovf_count, 1ull);
             ovf_list[slot] = (uint32_t)c;
+            out[c] = 0;
         } else {
             bool zero = false;
             uint16_t it[8];
@@ -556,6 +656,7 @@ __global__ void sort_count_kernel(const uint64_t *__restrict__ cand_ptr, const u
             out[c] = (uint32_t)n_txn;
         } else if (k > 8) {
             ovf_list[atomicAdd(ovf_count, 1ull)] = (uint32_t)c;
+            out[c] = 0;
         } else {
             uint32_t mn = 0xffffffffu;
             bool zero = false;
@@ -791,7 +892,33 @@ bool encode_bitmap_map(CUtensorMap *map, const uint64_t *bitmaps, uint32_t d, ui
     return r == CUDA_SUCCESS;
 }
 
-size_t support_scratch_bytes(uint64_t n_cand) { return support_scratch_bytes_for(n_cand); }
+// The kernel of an AUTO call (map: the rows can be staged by TMA).
+//
+// Streaming reads every row of every candidate from L2; staging reads the
+// bitmaps once per SM, whatever the number of candidates.  At 1,048,576
+// transactions, in us (streamed / k1_lane_tm), sensor rows and sparse rows alike:
+//   256 rows:    20,000 candidates 546 / 2,082; 60,000 1,489 / 2,665; 200,000 4,719 / 5,427
+//   640 rows:    20,000 701 / 3,002; 60,000 1,978 / 3,581; 200,000 6,206 / 6,354; 600,000 17,857 / 13,709
+//   1,024 rows:  20,000 626 / 3,416; 200,000 6,296 / 6,776; 600,000 18,398 / 14,119
+// and in proportion to the transactions from 20,000 on: the staged kernel pays
+// per box of 256 rows, so the line is a number of candidates and boxes.
+// Above it, calls of 2e9 candidate-words (2.4 ms) or more look whether the data
+// are sparse (kernels_pair.cu), which costs them 40 us when they are not.
+static SupportKernel auto_kernel(uint64_t n_cand, uint32_t d, uint64_t n_words, bool map) {
+    if (!map || d == 0) return SUPPORT_STREAM;
+    const uint64_t boxes = (d + 255) / 256;
+    if (n_cand < 100000 + 30000 * boxes) return SUPPORT_STREAM;
+    if (pair_supported(d, n_cand) && n_cand * n_words >= 2000000000ull) return SUPPORT_PAIR;
+    return lane_supported(d) ? SUPPORT_LANE_TM : SUPPORT_STAGED4;
+}
+
+size_t support_scratch_bytes(uint64_t n_cand, uint32_t d, uint64_t n_words, const SupportPlan &plan) {
+    const size_t base = support_scratch_bytes_for(n_cand);
+    const bool pair = plan.kernel == SUPPORT_PAIR
+                          ? pair_supported(d, n_cand)
+                          : plan.kernel == SUPPORT_AUTO && auto_kernel(n_cand, d, n_words, true) == SUPPORT_PAIR;
+    return pair ? align256(base) + pair_scratch_bytes(n_cand, d) : base;
+}
 
 int support_batch_device(const uint64_t *bitmaps, uint32_t d, uint64_t n_words, uint64_t row_stride,
                          uint64_t n_txn, const uint64_t *cand_ptr, const uint32_t *cand_items, uint64_t n_cand,
@@ -813,37 +940,64 @@ int support_batch_device(const uint64_t *bitmaps, uint32_t d, uint64_t n_words, 
         while (cpc > 1 && smem_fn(d, cpc) > 227 * 1024) cpc = cpc * 3 / 4;
         return smem_fn(d, cpc) <= 227 * 1024 ? cpc : 0;
     };
+    StreamBatch cs{};
+    cs.rows = bitmaps; cs.stride = row_stride; cs.n_words = n_words_even; cs.d = d;
+    cs.cand_ptr = cand_ptr; cs.items = cand_items; cs.n = n_cand; cs.n_txn = n_txn; cs.out = out;
     int kind = plan.kernel;
     if (map == nullptr || d == 0) kind = SUPPORT_STREAM;
-    // measured on GB300 at 1M candidates x 1,024 rows: lane with TMEM records 22.3 ms, lane
-    // with shared-memory records 23.2 ms, staged with 4-lane groups 30.0 ms, staged with 8-lane
-    // groups 30.9 ms, sorted 30.8-46 ms (depending on its grid).  AUTO falls through to the
-    // shared-memory lane form, then STAGED4, when a layout does not fit.
-    if (kind == SUPPORT_AUTO) kind = lane_supported(d) ? SUPPORT_LANE_TM : SUPPORT_STAGED4;
+    // AUTO falls through to the shared-memory lane form, then STAGED4, when a layout does not
+    // fit (1M candidates x 1,024 rows: 22.3 ms with records in TMEM, 23.2 in shared memory, staged
+    // with 4-lane groups 30.0, with 8-lane groups 30.9, sorted 30.8 - 46)
+    const bool gated = kind == SUPPORT_AUTO;
+    if (kind == SUPPORT_AUTO) kind = auto_kernel(n_cand, d, n_words_even, map != nullptr);
+    const uint32_t *gate = nullptr;
+    if (kind == SUPPORT_PAIR) {
+        uint32_t *ovf_l = nullptr;
+        unsigned long long *ovf_c = nullptr;
+        const size_t at = align256(support_scratch_bytes_for(n_cand));   // the lane kernels' scratch comes first
+        mark(0);
+        if (scratch.bytes > at &&
+            pair_supports_device(map, bitmaps, d, n_words_even, row_stride, cand_ptr, cand_items, n_cand, n_txn, out,
+                                 static_cast<char *>(scratch.base) + at, scratch.bytes - at, gated, dev_err, st, n_sm,
+                                 &gate, &ovf_l, &ovf_c, launches, ev) == 0) {
+            StreamBatch tail = cs;
+            tail.n_device = reinterpret_cast<const uint64_t *>(ovf_c);
+            tail.index = ovf_l;
+            launch_cand_stream(tail, st, n_sm);
+            if (launches) *launches += 1;
+            if (!gated) {
+                mark(3);
+                return 0;
+            }
+        }
+        kind = lane_supported(d) ? SUPPORT_LANE_TM : SUPPORT_STAGED4;
+    }
     if (kind == SUPPORT_LANE || kind == SUPPORT_LANE_TM) {
         uint32_t *ovf_l = nullptr;
         unsigned long long *ovf_c = nullptr;
-        mark(0);
+        // after a gated pair call: these kernels run when it found the data dense, and the pair
+        // kernel's events stand
+        if (!gate) mark(0);
+        cudaEvent_t *lane_ev = gate ? nullptr : ev;
         int rc = -1;
         if (kind == SUPPORT_LANE_TM)
             rc = lane_tm_supports_device(map, d, n_words_even, cand_ptr, cand_items, n_cand, n_txn, out,
                                          scratch.base, scratch.bytes, plan.waves ? plan.waves : 1, dev_err, st, n_sm,
-                                         &ovf_l, &ovf_c, launches, ev);
+                                         &ovf_l, &ovf_c, launches, lane_ev, gate);
         if (rc != 0)
             rc = lane_supports_device(map, d, n_words_even, cand_ptr, cand_items, n_cand, n_txn, out, scratch.base,
                                       scratch.bytes, kind == SUPPORT_LANE && plan.waves ? plan.waves : 2, dev_err, st,
-                                      n_sm, &ovf_l, &ovf_c, launches, ev);
+                                      n_sm, &ovf_l, &ovf_c, launches, lane_ev, gate);
         if (rc == 0) {
-            QueryBatch qb;
-            qb.rows = bitmaps; qb.row_stride = row_stride; qb.n_words = n_words_even; qb.d = d;
-            qb.q_ptr = cand_ptr; qb.q_items = cand_items; qb.n_q_device = reinterpret_cast<const uint64_t *>(ovf_c);
-            qb.q_index = ovf_l; qb.out = out; qb.empty_value = n_txn;
-            launch_queries(qb, st, n_sm);
+            if (gate) mark(2);
+            cs.n_device = reinterpret_cast<const uint64_t *>(ovf_c);
+            cs.index = ovf_l;
+            launch_cand_stream(cs, st, n_sm);
             mark(3);
             if (launches) *launches += 1;
             return 0;
         }
-        if (scratch.bytes < support_scratch_bytes(n_cand)) return -1;
+        if (scratch.bytes < support_scratch_bytes_for(n_cand)) return -1;
         kind = SUPPORT_STAGED4;
     }
     if (kind == SUPPORT_SORTED && d > kSortCompactMax) kind = SUPPORT_STAGED;
@@ -857,18 +1011,15 @@ int support_batch_device(const uint64_t *bitmaps, uint32_t d, uint64_t n_words, 
         if (!cpc) kind = SUPPORT_STREAM;
     }
     if (kind == SUPPORT_STREAM) {
-        QueryBatch qb;
-        qb.rows = bitmaps; qb.row_stride = row_stride; qb.n_words = n_words_even; qb.d = d;
-        qb.q_ptr = cand_ptr; qb.q_items = cand_items; qb.n_q = n_cand; qb.out = out; qb.empty_value = n_txn;
         mark(0);
         mark(1);
-        launch_queries(qb, st, n_sm);
+        launch_cand_stream(cs, st, n_sm);
         mark(2);
         mark(3);
         if (launches) *launches += 1;
         return 0;
     }
-    if (scratch.bytes < support_scratch_bytes(n_cand)) return -1;
+    if (scratch.bytes < support_scratch_bytes_for(n_cand)) return -1;
     uint8_t *sb = static_cast<uint8_t *>(scratch.base);
     uint4 *recs = reinterpret_cast<uint4 *>(sb);
     uint32_t *ovf = reinterpret_cast<uint32_t *>(sb + align256(n_cand * 16));
@@ -917,11 +1068,9 @@ int support_batch_device(const uint64_t *bitmaps, uint32_t d, uint64_t n_words, 
         if (launches) *launches += 2;
     }
     // candidates with more than 8 items
-    QueryBatch qb;
-    qb.rows = bitmaps; qb.row_stride = row_stride; qb.n_words = n_words_even; qb.d = d;
-    qb.q_ptr = cand_ptr; qb.q_items = cand_items; qb.n_q_device = reinterpret_cast<const uint64_t *>(ovf_n);
-    qb.q_index = ovf; qb.out = out; qb.empty_value = n_txn;
-    launch_queries(qb, st, n_sm);
+    cs.n_device = reinterpret_cast<const uint64_t *>(ovf_n);
+    cs.index = ovf;
+    launch_cand_stream(cs, st, n_sm);
     mark(3);
     if (launches) *launches += 1;
     return 0;

@@ -63,8 +63,10 @@ __global__ void __launch_bounds__(kLaneTile) lane_hist_kernel(const uint64_t *__
                                                               uint32_t d, uint64_t n_txn, uint32_t *__restrict__ bins,
                                                               uint32_t *__restrict__ ovf_list,
                                                               unsigned long long *__restrict__ ovf_count,
-                                                              uint32_t *__restrict__ out) {
+                                                              uint32_t *__restrict__ out,
+                                                              const uint32_t *__restrict__ gate) {
     __shared__ uint32_t hist[kLaneBins];
+    if (gate && *gate == 0) return;
     if (threadIdx.x < kLaneBins) hist[threadIdx.x] = 0;
     __syncthreads();
     for (uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; c < n; c += (uint64_t)gridDim.x * blockDim.x) {
@@ -77,6 +79,7 @@ __global__ void __launch_bounds__(kLaneTile) lane_hist_kernel(const uint64_t *__
             out[c] = (uint32_t)n_txn;
         } else if (bin == -2) {
             ovf_list[atomicAdd(ovf_count, 1ull)] = (uint32_t)c;
+            out[c] = 0;   // the streaming kernel adds its segments
         } else {
             out[c] = 0;
         }
@@ -92,7 +95,9 @@ __global__ void __launch_bounds__(kLaneTile) lane_scatter_kernel(const uint64_t 
                                                                  const uint32_t *__restrict__ items, uint64_t n,
                                                                  uint32_t d, uint32_t *__restrict__ bins,
                                                                  uint4 *__restrict__ recs,
-                                                                 uint32_t *__restrict__ perm) {
+                                                                 uint32_t *__restrict__ perm,
+                                                                 const uint32_t *__restrict__ gate) {
+    if (gate && *gate == 0) return;
     __shared__ uint32_t start[kLaneBins], tile_n[kLaneBins], tile_base[kLaneBins];
     if (threadIdx.x == 0) {
         uint32_t s = 0;
@@ -444,7 +449,7 @@ int lane_tm_supports_device(const CUtensorMap *map, uint32_t d, uint64_t n_words
                             const uint32_t *cand_items, uint64_t n_cand, uint64_t n_txn, uint32_t *out, void *scratch,
                             size_t scratch_bytes, uint32_t waves, uint32_t *dev_err, cudaStream_t st, int n_sm,
                             uint32_t **ovf_list, unsigned long long **ovf_count, uint64_t *launches,
-                            cudaEvent_t *ev) {
+                            cudaEvent_t *ev, const uint32_t *gate) {
     if (!lane_supported(d) || n_cand == 0 || n_cand > 0xffffffffull) return -1;
     if (scratch_bytes < support_scratch_bytes_for(n_cand)) return -1;
     const uint32_t n_boxes = (d + kLaneRowsPerBox - 1) / kLaneRowsPerBox;
@@ -472,9 +477,10 @@ int lane_tm_supports_device(const CUtensorMap *map, uint32_t d, uint64_t n_words
     SG_CUDA_TRY(cudaMemsetAsync(bins, 0, 2 * kLaneBins * 4, st));
     SG_CUDA_TRY(cudaMemsetAsync(ovf_n, 0, 8, st));
     const unsigned prep_blocks = (unsigned)std::min<uint64_t>((n_cand + kLaneTile - 1) / kLaneTile, (uint64_t)n_sm * 8);
-    lane_hist_kernel<<<prep_blocks, kLaneTile, 0, st>>>(cand_ptr, cand_items, n_cand, d, n_txn, bins, ovf, ovf_n, out);
+    lane_hist_kernel<<<prep_blocks, kLaneTile, 0, st>>>(cand_ptr, cand_items, n_cand, d, n_txn, bins, ovf, ovf_n, out,
+                                                        gate);
     SG_CUDA_TRY(cudaGetLastError());
-    lane_scatter_kernel<<<prep_blocks, kLaneTile, 0, st>>>(cand_ptr, cand_items, n_cand, d, bins, recs, perm);
+    lane_scatter_kernel<<<prep_blocks, kLaneTile, 0, st>>>(cand_ptr, cand_items, n_cand, d, bins, recs, perm, gate);
     SG_CUDA_TRY(cudaGetLastError());
     const size_t smem = lane_tm_smem_bytes(n_slots);
     SG_CUDA_TRY(cudaFuncSetAttribute(k1_lane_tm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -495,7 +501,7 @@ int lane_supports_device(const CUtensorMap *map, uint32_t d, uint64_t n_words, c
                          const uint32_t *cand_items, uint64_t n_cand, uint64_t n_txn, uint32_t *out, void *scratch,
                          size_t scratch_bytes, uint32_t waves, uint32_t *dev_err, cudaStream_t st, int n_sm,
                          uint32_t **ovf_list, unsigned long long **ovf_count, uint64_t *launches,
-                         cudaEvent_t *ev) {
+                         cudaEvent_t *ev, const uint32_t *gate) {
     if (!lane_supported(d) || n_cand == 0 || n_cand > 0xffffffffull) return -1;
     if (scratch_bytes < support_scratch_bytes_for(n_cand)) return -1;
     const uint32_t n_boxes = (d + kLaneRowsPerBox - 1) / kLaneRowsPerBox;
@@ -518,9 +524,10 @@ int lane_supports_device(const CUtensorMap *map, uint32_t d, uint64_t n_words, c
     SG_CUDA_TRY(cudaMemsetAsync(bins, 0, 2 * kLaneBins * 4, st));
     SG_CUDA_TRY(cudaMemsetAsync(ovf_n, 0, 8, st));
     const unsigned prep_blocks = (unsigned)std::min<uint64_t>((n_cand + kLaneTile - 1) / kLaneTile, (uint64_t)n_sm * 8);
-    lane_hist_kernel<<<prep_blocks, kLaneTile, 0, st>>>(cand_ptr, cand_items, n_cand, d, n_txn, bins, ovf, ovf_n, out);
+    lane_hist_kernel<<<prep_blocks, kLaneTile, 0, st>>>(cand_ptr, cand_items, n_cand, d, n_txn, bins, ovf, ovf_n, out,
+                                                        gate);
     SG_CUDA_TRY(cudaGetLastError());
-    lane_scatter_kernel<<<prep_blocks, kLaneTile, 0, st>>>(cand_ptr, cand_items, n_cand, d, bins, recs, perm);
+    lane_scatter_kernel<<<prep_blocks, kLaneTile, 0, st>>>(cand_ptr, cand_items, n_cand, d, bins, recs, perm, gate);
     SG_CUDA_TRY(cudaGetLastError());
     const size_t smem = lane_smem_bytes(n_boxes, (uint32_t)l_cap);
     SG_CUDA_TRY(cudaFuncSetAttribute(k1_lane_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

@@ -170,15 +170,18 @@ int sgfim_cooccurrence(sgfim_handle *h, uint32_t *out, uint32_t d);
  * kernel: SGFIM_KERNEL_*; cands_per_cta: candidates a CTA owns (0 = derived);
  * waves: CTAs per SM over the grid when cands_per_cta is 0 (0 = the kernel's
  * default: 1 for SORTED, 2 for STAGED). */
-#define SGFIM_KERNEL_AUTO 0    /* LANE_TM when the rows fit shared memory (d <= 1,792), else STAGED4 or streaming */
+#define SGFIM_KERNEL_AUTO 0    /* by the number of candidates and rows: STREAM, then LANE_TM (d <= 1,792; STAGED4
+                                  above), or PAIR on large calls whose data are sparse */
 #define SGFIM_KERNEL_STAGED 1  /* TMA-staged chunks, candidates in input order */
 #define SGFIM_KERNEL_SORTED 2  /* TMA-staged chunks, candidates sorted by (k, first item); ids < 1024 */
-#define SGFIM_KERNEL_STREAM 3  /* one warp per candidate, rows streamed from L2/HBM */
+#define SGFIM_KERNEL_STREAM 3  /* a warp per candidate and run of words, rows streamed from L2/HBM */
 #define SGFIM_KERNEL_STAGED4 4 /* TMA-staged chunks, 4-lane groups (32 bytes of a row per lane) */
 #define SGFIM_KERNEL_LANE 5    /* TMA-staged chunks, one lane per candidate, candidates sorted by k
                                   on the device; waves = CTAs per SM (default 2) */
 #define SGFIM_KERNEL_LANE_TM 6 /* LANE with the candidates in tensor memory and the next chunk
                                   loaded during the current one; waves default 1 */
+#define SGFIM_KERNEL_PAIR 7    /* candidates grouped by their two rarest rows, rows read where the AND still
+                                  has a bit */
 int sgfim_support_plan_set(sgfim_handle *h, int kernel, uint32_t cands_per_cta, uint32_t waves);
 
 /* Allocation-free form of sgfim_support_batch_device.  It has no counterpart
