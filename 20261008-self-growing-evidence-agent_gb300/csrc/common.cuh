@@ -102,6 +102,27 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity
     return false;
 }
 
+// The same bound with the limit read once per kernel: on the path of every step
+// of a pipeline the read of err costs a round trip to L2 whenever the first poll
+// fails.  The clock is read after every 16 failed polls.
+__device__ __forceinline__ uint64_t mbar_limit_ns(const uint32_t *err) {
+    const uint32_t us = err ? *reinterpret_cast<const volatile uint32_t *>(err + kCtlWaitUs) : 0u;
+    return (uint64_t)(us ? us : kWaitLimitUsDefault) * 1000ull;
+}
+__device__ __forceinline__ bool mbar_wait_limit(uint64_t *bar, uint32_t parity, uint64_t limit_ns, uint32_t *err) {
+    uint64_t t0 = 0;
+    for (;;) {
+#pragma unroll 1
+        for (int i = 0; i < 16; ++i)
+            if (mbar_try_wait(bar, parity)) return true;
+        const uint64_t t = global_ns();
+        if (t0 == 0) t0 = t;
+        else if (t - t0 > limit_ns) break;
+    }
+    set_device_error(err, DEVERR_MBAR_TIMEOUT);
+    return false;
+}
+
 // 2-D tiled TMA load (global -> this CTA's shared memory), completion on bar.
 __device__ __forceinline__ void tma_load_2d(void *smem_dst, const CUtensorMap *map, int32_t x, int32_t y,
                                             uint64_t *bar) {

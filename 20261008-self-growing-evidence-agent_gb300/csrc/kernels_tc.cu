@@ -21,6 +21,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "tcgen05.cuh"
 
 namespace sg {
 
@@ -32,20 +33,6 @@ constexpr int kTcAtom = 128 * 128;             // one 128-row x 128-byte swizzle
 constexpr int kTcOperand = 2 * kTcAtom;        // two atoms along K per operand
 constexpr int kTcStageBytes = 2 * kTcOperand;  // A and B
 constexpr uint32_t kTcCols = 128;              // TMEM columns (fp32 accumulators)
-
-__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr) {
-    // sm_100 shared-memory matrix descriptor: start >> 4 (bits 0-13), leading
-    // byte offset >> 4 (16-29, unused for swizzled K-major: 1), stride byte
-    // offset >> 4 (32-45: 1024 B between 8-row groups), version 1 (46-47),
-    // base offset 0 (49-51), layout SWIZZLE_128B = 2 (61-63).
-    uint64_t d = 0;
-    d |= (uint64_t)((addr >> 4) & 0x3fff);
-    d |= (uint64_t)1 << 16;
-    d |= (uint64_t)(1024 >> 4) << 32;
-    d |= (uint64_t)1 << 46;
-    d |= (uint64_t)2 << 61;
-    return d;
-}
 
 // Instruction descriptor, kind::f8f6f4: D = f32 (bits 4-5 = 1), A = B = e4m3
 // (bits 7-9, 10-12 = 0), both K-major (bits 15, 16 = 0), N >> 3 at bits
@@ -60,15 +47,6 @@ __device__ __forceinline__ void tc_mma(uint32_t tmem, uint64_t adesc, uint64_t b
         "l"(adesc), "l"(bdesc), "r"(kTcIdesc), "r"(acc)
         : "memory");
 }
-
-__device__ __forceinline__ void tc_commit(uint64_t *bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                     smem_addr(bar))
-                 : "memory");
-}
-
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 
 // 4 bits -> 4 bytes of e4m3 (0x38 = 1.0 where the bit is set).
 __device__ __forceinline__ uint32_t nib4(uint32_t n) { return ((n * 0x00204081u) & 0x01010101u) * 0x38u; }
@@ -455,15 +433,380 @@ __global__ void __launch_bounds__(kT2Threads, 1)
     }
 }
 
+// ---------------------------------------------------------------- fp4, 128 x 256 tiles
+// The same product with 4-bit operands: tcgen05.mma kind::mxf4 (e2m1 with
+// block scales) multiplies K = 64 transactions per instruction at twice the
+// fp8 rate and half its bytes.  Every product is exactly 0 or 1 and the fp32 sums
+// are the same exact integers.
+//
+// What the 256 x 256 form above is bound by is shared memory: per K = 32 it
+// writes 16 KB of expanded operands and the MMAs read 24 KB (320 clocks) for 256
+// clocks of tensor work.  Here A is expanded into tensor memory and only B goes
+// through shared memory: per K = 64 with M = 128, N = 256, 8 KB written and 8 KB
+// read (128 clocks) for 128 clocks of tensor work, and 6 KB of bit slices.  The
+// expansion is cheaper too: the order of the transactions inside
+// a K step does not matter as long as A and B share it, so a 32-bit word becomes
+// four registers by shift and mask, register i holding bits i, i + 4, i + 8, ...
+// as nibbles (5 instructions where the byte form needs 40).
+//
+// Bits arrive by TMA in rows of 64 bytes, two steps at a time.
+//
+// The work is cut into runs of transactions, all tiles of a run next to each
+// other, so the CTAs that read the same rows read them at the same time (from L2:
+// with a tile's runs next to each other the bitmaps came 4 times from HBM).  It is
+// dealt evenly in steps, so a CTA may end one tile and begin the next; counts are added to out and its
+// mirror with coalesced atomics (the mirror through a shared-memory transpose).
+// A diagonal tile's A rows are a half of its B rows: their bits are loaded once.
+//
+// Warp roles, as in the 256 x 256 form: two groups of 12 warps expand the even and
+// the odd steps, a row per thread (eight warps B, four A), and all 24 read the
+// accumulators at a tile's end; warp 24 issues the MMAs, warp 25 the TMA loads.
+//
+// Measured, 1,024 rows x 1,048,576 transactions: 0.30 ms a call (0.525 for the 256 x
+// 256 form); tensor pipe 50%, and shared memory (expansion writes with their
+// conflicts 310 clocks a step, the MMAs' reads 256, bit slices 200) about 75% of a
+// step's 1,070 clocks.  Before: A through shared memory too 0.36 ms; a single group
+// of 12 expansion warps 0.32; stage and phase divided out by the MMA thread every
+// step 0.33.  No difference: 3 or 4 stages, 64- or 128-byte rows, 5 or 7 instructions
+// per expanded word.
+constexpr int kF4GroupWarps = 12;                        // warps that expand one step
+constexpr int kF4ExpWarps = 2 * kF4GroupWarps;
+constexpr int kF4Threads = 32 * (kF4ExpWarps + 2);
+constexpr int kF4RowsA = 128, kF4RowsB = 256;
+constexpr int kF4Words = 8;                              // 64-bit words of a double step: 512 transactions
+constexpr int kF4StageBytes = kF4RowsB * 128;            // B, one step: 32 KB
+constexpr int kF4Stages = 3;
+constexpr int kF4Ring = 5;
+constexpr int kF4RowBytes = kF4Words * 8;
+constexpr int kF4RingBytes = (kF4RowsA + kF4RowsB) * kF4RowBytes;   // 24 KB
+constexpr int kF4Turn = 32 * 17;                         // words of a warp's 32 x 16 transpose buffer
+constexpr uint32_t kF4ScaleCol = 256;                    // block scales: TMEM columns 256..319
+constexpr uint32_t kF4ColA = 320;                        // A: 32 columns (256 values per row) per stage
+constexpr uint64_t kF4MaxSteps = (1u << 20) / (kF4Words * 64);   // double steps summed in one accumulator
+// Double steps of a CTA, at least: its fixed part (tensor memory, barriers, counts
+// to out) is about 2 us, a double step 1 us.  126 rows x 65,536 transactions, a
+// call: 18 us at 2, 20 at 4, 23 at 8, 31 at 16.
+constexpr uint64_t kF4MinSteps = 2;
+// A, B e2m1; scale format ue8m0; N = 256, M = 128; K = 64
+constexpr uint32_t kF4Idesc = (1u << 7) | (1u << 10) | ((256u >> 3) << 17) | (1u << 23) | ((128u >> 4) << 24);
+
+// A from tensor memory, B from shared memory
+__device__ __forceinline__ void tc_mma_f4(uint32_t tmem, uint32_t a, uint64_t bdesc, uint32_t scale_a,
+                                          uint32_t scale_b, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %6, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], [%1], %2, %3, [%4], [%5], p;\n\t}" ::"r"(
+            tmem),
+        "r"(a), "l"(bdesc), "r"(kF4Idesc), "r"(scale_a), "r"(scale_b), "r"(acc)
+        : "memory");
+}
+
+// 128 bits -> four 16-byte pieces (32 values each).  Piece i holds bits i, i + 4,
+// i + 8, ... of the four words as nibbles: bits 0, 1 and 2 stay where they are and
+// read as 0.5, 1 and 2, bit 3 moves to bit 2 (where it would be the sign).  The
+// block scales (one per 32 values) make every product 1: 2 x 2 for piece 0, 1 x 1
+// for piece 1, 1/2 x 1/2 for pieces 2 and 3.
+__device__ __forceinline__ uint4 mask4(const uint4 &x, uint32_t m) {
+    return make_uint4(x.x & m, x.y & m, x.z & m, x.w & m);
+}
+__device__ __forceinline__ void expand_f4(const uint4 &x, uint4 (&p)[4]) {
+    p[0] = mask4(x, 0x11111111u);
+    p[1] = mask4(x, 0x22222222u);
+    p[2] = mask4(x, 0x44444444u);
+    p[3] = mask4(make_uint4(x.x >> 1, x.y >> 1, x.z >> 1, x.w >> 1), 0x44444444u);
+}
+constexpr uint32_t kF4ScaleLow = 0x7f807f80u, kF4ScaleHigh = 0x7e7e7e7eu;   // pieces 0 and 1; 2 and 3 (ue8m0)
+
+struct F4Work {
+    uint32_t d, col_tiles;      // rows; 256-row column tiles
+    uint64_t tiles;
+    uint64_t run, last;         // double steps of a run of transactions, and of the last run
+    uint64_t full;              // double steps of all tiles in the runs before the last
+    uint64_t total;             // double steps of the whole product
+    uint64_t share;             // double steps of a CTA
+};
+
+// The tile and double step at position g of the work, and how many follow in its
+// run (itself included).  Row tile bi (128 rows) meets the column tiles from
+// bi / 2 on.
+__device__ __forceinline__ uint64_t f4_unit(const F4Work &w, uint64_t g, uint32_t &bi, uint32_t &bj, uint64_t &step0) {
+    const uint64_t len = g < w.full ? w.run : w.last;
+    const uint64_t u = g < w.full ? g / w.run : (g - w.full) / w.last;
+    const uint64_t s = g < w.full ? g - u * w.run : g - w.full - u * w.last;
+    const uint64_t r = g < w.full ? u / w.tiles : w.full / (w.tiles * w.run);
+    uint64_t t = g < w.full ? u - r * w.tiles : u;
+    step0 = r * w.run + s;
+    bi = 0;
+    while (t >= w.col_tiles - (bi >> 1)) {
+        t -= w.col_tiles - (bi >> 1);
+        ++bi;
+    }
+    bj = (bi >> 1) + (uint32_t)t;
+    return len - s;
+}
+
+// 128 bits of a row -> 16 TMEM columns of e2m1 values.
+__device__ __forceinline__ void tmem_st_f4(uint32_t taddr, const uint4 &x) {
+    uint4 p[4];
+    expand_f4(x, p);
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+        "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
+        "r"(p[0].x), "r"(p[0].y), "r"(p[0].z), "r"(p[0].w), "r"(p[1].x), "r"(p[1].y), "r"(p[1].z), "r"(p[1].w),
+        "r"(p[2].x), "r"(p[2].y), "r"(p[2].z), "r"(p[2].w), "r"(p[3].x), "r"(p[3].y), "r"(p[3].z), "r"(p[3].w)
+        : "memory");
+}
+
+// 256 bits of a row -> its 128 bytes in stage ST; at[c]: address of piece c in stage 0.
+template <int ST>
+__device__ __forceinline__ void smem_st_f4(uint8_t *base, const uint32_t (&at)[8], const uint4 &x0, const uint4 &x1) {
+    uint4 p[4];
+    expand_f4(x0, p);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) *reinterpret_cast<uint4 *>(base + at[c] + ST * kF4StageBytes) = p[c];
+    expand_f4(x1, p);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) *reinterpret_cast<uint4 *>(base + at[4 + c] + ST * kF4StageBytes) = p[c];
+}
+
+__global__ void __launch_bounds__(kF4Threads, 1)
+    cooc_f4_kernel(const __grid_constant__ CUtensorMap bm_map, F4Work work, uint32_t *__restrict__ out, uint32_t *err) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    __shared__ uint64_t ring_full[kF4Ring], ring_empty[kF4Ring], stage_full[kF4Stages], stage_empty[kF4Stages];
+    __shared__ uint64_t done_bar, free_bar;           // a tile's MMAs are done; its accumulators have been read
+    __shared__ uint32_t tmem_slot;
+    __shared__ volatile uint32_t failed;              // a role gave up on a wait: the others stop
+    __shared__ unsigned long long issued_n;           // ring steps issued (producer)
+    const uint64_t limit = mbar_limit_ns(err);
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    uint8_t *base = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem) + 1023) & ~uintptr_t(1023));
+    uint8_t *ring = base + (size_t)kF4Stages * kF4StageBytes;
+    uint32_t *turn = reinterpret_cast<uint32_t *>(base);   // transposes, while no stage is in use
+    const uint64_t g0 = work.share * blockIdx.x, g1 = min(work.total, g0 + work.share);
+
+    if (warp == 0) tmem_alloc(&tmem_slot, 512);
+    if (tid == 0) {
+        for (int i = 0; i < kF4Ring; ++i) {
+            mbar_init(&ring_full[i], 1);
+            mbar_init(&ring_empty[i], kF4ExpWarps);
+        }
+        for (int i = 0; i < kF4Stages; ++i) {
+            mbar_init(&stage_full[i], kF4GroupWarps);
+            mbar_init(&stage_empty[i], 1);
+        }
+        mbar_init(&done_bar, 1);
+        mbar_init(&free_bar, kF4ExpWarps);
+        fence_mbar_init();
+        failed = 0;
+        issued_n = 0;
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+    if (warp < 4) {   // the scales, the same in every lane: A low, B low, A high, B high
+        const uint32_t at = tmem + ((warp * 32u) << 16) + kF4ScaleCol;
+#pragma unroll 1
+        for (uint32_t c = 0; c < 64; ++c)
+            asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(at + c),
+                         "r"(c < 32 ? kF4ScaleLow : kF4ScaleHigh)
+                         : "memory");
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+
+    // every role walks the same units: ns double steps of a tile
+    // (t: double steps of this CTA before the unit; double step t uses ring slot t % kF4Ring, its
+    // steps 2t and 2t + 1 stages 2t % kF4Stages and the next)
+    uint32_t t = 0;
+    uint32_t mma_st = 0, mma_par = 0;                      // stage and phase of the next MMAs
+    const uint64_t desc0 = smem_desc_sw128(smem_addr(base));
+    uint32_t unit_n = 0;      // units of this CTA so far (done_bar and free_bar phases)
+    bool ok = true;
+    for (uint64_t g = g0; g < g1 && ok; ++unit_n) {
+        uint32_t bi, bj;
+        uint64_t step0;
+        const uint64_t follow = f4_unit(work, g, bi, bj, step0);
+        const uint32_t ns = (uint32_t)min(g1 - g, follow);
+        const bool diag = (bi >> 1) == bj;   // A is half bi & 1 of B
+        if (warp < kF4ExpWarps) {
+            // ---- expansion: threads 0..255 B rows (shared memory), 256..383 A rows (tensor memory)
+            // of the group whose turn the step is
+            const uint32_t group = warp >= kF4GroupWarps ? 1u : 0u, r = tid - group * kF4GroupWarps * 32;
+            const bool is_a = r >= kF4RowsB;
+            const uint32_t src_row = is_a && diag ? r - kF4RowsB + (bi & 1) * kF4RowsA : r;
+            // the bits' 16-byte pieces are swizzled by TMA: piece c of row r at c ^ (r / 2 % 4)
+            const uint32_t sel = (src_row >> 1) & 3;
+            const uint8_t *src = ring + src_row * kF4RowBytes;
+            uint32_t at[8];
+#pragma unroll
+            for (uint32_t c = 0; c < 8; ++c) at[c] = r * 128 + ((c ^ (r & 7)) << 4);
+            const uint32_t a_at = tmem + (((warp & 3) * 32u) << 16) + kF4ColA;
+            for (uint32_t k = t; k < t + ns; ++k) {
+                const uint32_t slot = k % kF4Ring, step = 2 * k + group, use = step / kF4Stages,
+                               st = step - use * kF4Stages;
+                ok = mbar_wait_limit(&ring_full[slot], (k / kF4Ring) & 1, limit, err);
+                uint4 x0 = make_uint4(0, 0, 0, 0), x1 = x0;
+                if (ok) {
+                    x0 = *reinterpret_cast<const uint4 *>(src + slot * kF4RingBytes + (((group * 2) ^ sel) << 4));
+                    x1 = *reinterpret_cast<const uint4 *>(src + slot * kF4RingBytes + (((group * 2 + 1) ^ sel) << 4));
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&ring_empty[slot]);   // the slot's bits are in registers
+                if (ok && use) ok = mbar_wait_limit(&stage_empty[st], (use - 1) & 1, limit, err);
+                if (!__all_sync(0xffffffffu, ok)) {
+                    ok = false;
+                    break;
+                }
+                if (!is_a) {
+                    if (st == 0) smem_st_f4<0>(base, at, x0, x1);
+                    else if (st == 1) smem_st_f4<1>(base, at, x0, x1);
+                    else smem_st_f4<2>(base, at, x0, x1);
+                    fence_proxy_async_smem();
+                } else {
+                    tc_fence_after();
+                    tmem_st_f4(a_at + st * 32, x0);
+                    tmem_st_f4(a_at + st * 32 + 16, x1);
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    tc_fence_before();
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&stage_full[st]);
+            }
+            // ---- the unit's counts: warp w reads TMEM quadrant w % 4, every sixth chunk of 16 columns
+            if (ok) ok = mbar_wait_limit(&done_bar, unit_n & 1, limit, err);
+            // one decision for all expansion warps: they meet at barriers from here on
+            uint32_t bad;
+            asm volatile(
+                "{\n\t.reg .pred p, q;\n\t"
+                "setp.eq.u32 p, %1, 0;\n\t"
+                "barrier.cta.red.or.pred q, 1, %2, p;\n\t"
+                "selp.u32 %0, 1, 0, q;\n\t}"
+                : "=r"(bad)
+                : "r"((uint32_t)ok), "n"(32 * kF4ExpWarps)
+                : "memory");
+            ok = bad == 0;
+            if (!ok) {
+                failed = 1;
+                break;
+            }
+            tc_fence_after();
+            const uint32_t q = warp & 3, d = work.d;
+            const uint32_t row0 = bi * kF4RowsA + q * 32;
+            uint32_t *mine = turn + warp * kF4Turn;
+            for (uint32_t cb = (warp >> 2) * 16; cb < kF4RowsB; cb += kF4ExpWarps * 4) {
+                const uint32_t col0 = bj * kF4RowsB + cb;
+                if (col0 >= d || row0 >= d || col0 + 15 < row0) continue;   // nothing on or above the diagonal
+                uint32_t v[16];
+                tmem_ld16(tmem + ((q * 32u) << 16) + cb, v);
+                tmem_wait_ld();
+                const uint32_t row = row0 + lane;
+                __syncwarp();
+#pragma unroll
+                for (uint32_t c = 0; c < 16; ++c) {
+                    const uint32_t col = col0 + c, cnt = (uint32_t)__uint_as_float(v[c]);
+                    mine[lane * 17 + c] = cnt;
+                    if (cnt && row < d && col < d && col > row) atomicAdd(&out[(uint64_t)col * d + row], cnt);
+                }
+                __syncwarp();
+#pragma unroll 4
+                for (uint32_t r2 = 0; r2 < 32; r2 += 2) {   // two rows of 16 columns per instruction
+                    const uint32_t rr = row0 + r2 + (lane >> 4), col = col0 + (lane & 15);
+                    const uint32_t cnt = mine[(r2 + (lane >> 4)) * 17 + (lane & 15)];
+                    if (cnt && rr < d && col < d && col >= rr) atomicAdd(&out[(uint64_t)rr * d + col], cnt);
+                }
+            }
+            tc_fence_before();
+            // the stages hold transposes until every warp is through
+            asm volatile("bar.sync 1, %0;" ::"n"(32 * kF4ExpWarps) : "memory");
+            if (lane == 0) mbar_arrive(&free_bar);
+        } else if (warp == kF4ExpWarps) {
+            // ---- MMA issue (one thread; its serial chain is on the path of every step, so stage,
+            // phase and descriptors are carried along instead of computed)
+            if (lane == 0) {
+                if (unit_n > 0) ok = mbar_wait_limit(&free_bar, (unit_n - 1) & 1, limit, err);
+                uint32_t acc = 0;
+                for (uint32_t k = 2 * ns; k > 0; --k) {
+                    if (!ok || !mbar_wait_limit(&stage_full[mma_st], mma_par, limit, err)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint64_t bd = desc0 + mma_st * (uint32_t)(kF4StageBytes >> 4);
+                    const uint32_t a0 = tmem + kF4ColA + mma_st * 32, sc = tmem + kF4ScaleCol;
+                    // K steps of 64: pieces 0 and 1, then 2 and 3, of either 128 bits
+                    tc_mma_f4(tmem, a0, bd, sc, sc + 16, acc);
+                    acc = 1;
+                    tc_mma_f4(tmem, a0 + 8, bd + 2, sc + 32, sc + 48, 1u);
+                    tc_mma_f4(tmem, a0 + 16, bd + 4, sc, sc + 16, 1u);
+                    tc_mma_f4(tmem, a0 + 24, bd + 6, sc + 32, sc + 48, 1u);
+                    tc_commit(&stage_empty[mma_st]);
+                    if (++mma_st == kF4Stages) {
+                        mma_st = 0;
+                        mma_par ^= 1;
+                    }
+                }
+                if (!ok) failed = 1;
+                tc_commit(&done_bar);   // also after a failed wait: the MMAs issued still read the stages
+            }
+            ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+        } else {
+            // ---- TMA producer (one thread)
+            if (lane == 0) {
+                const uint32_t bytes = diag ? kF4RowsB * kF4RowBytes : kF4RingBytes;
+                for (uint32_t k = 0; k < ns; ++k) {
+                    const uint32_t slot = (t + k) % kF4Ring, use = (t + k) / kF4Ring;
+                    if (failed || (use && !mbar_wait_limit(&ring_empty[slot], (use - 1) & 1, limit, err))) {
+                        ok = false;
+                        break;
+                    }
+                    uint8_t *dst = ring + (size_t)slot * kF4RingBytes;
+                    mbar_arrive_expect_tx(&ring_full[slot], bytes);
+                    const int32_t x = (int32_t)((step0 + k) * kF4Words);
+                    for (int h = 0; h < 2; ++h)
+                        tma_load_2d(dst + h * 128 * kF4RowBytes, &bm_map, x, (int32_t)(bj * kF4RowsB + h * 128),
+                                    &ring_full[slot]);
+                    if (!diag)
+                        tma_load_2d(dst + kF4RowsB * kF4RowBytes, &bm_map, x, (int32_t)(bi * kF4RowsA), &ring_full[slot]);
+                    issued_n = issued_n + 1;
+                }
+                if (!ok) failed = 1;
+            }
+            ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+        }
+        g += ns;
+        t += ns;
+    }
+    __syncthreads();
+    if (failed) {
+        // let what is in flight land before the CTA's memory goes away: the MMAs issued (the
+        // last commit of done_bar has this CTA's last phase), and the last box of every ring slot
+        mbar_wait_limit(&done_bar, unit_n ? (unit_n - 1) & 1 : 0, limit, err);
+        const uint64_t n1 = issued_n;
+        for (uint64_t k = n1 > (uint64_t)kF4Ring ? n1 - kF4Ring : 0; k < n1; ++k)
+            mbar_wait_limit(&ring_full[k % kF4Ring], (uint32_t)((k / kF4Ring) & 1), limit, err);
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        tc_fence_after();
+        tmem_dealloc(tmem, 512);
+    }
+}
+
 bool encode_bits_map_box(CUtensorMap *map, const uint64_t *bitmaps, uint32_t d, uint64_t n_words,
-                         uint64_t row_stride, uint32_t box_words, uint32_t box_rows);
+                         uint64_t row_stride, uint32_t box_words, uint32_t box_rows,
+                         CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_NONE);
 
 bool encode_bits_map(CUtensorMap *map, const uint64_t *bitmaps, uint32_t d, uint64_t n_words, uint64_t row_stride) {
     return encode_bits_map_box(map, bitmaps, d, n_words, row_stride, 4, 128);
 }
 
 bool encode_bits_map_box(CUtensorMap *map, const uint64_t *bitmaps, uint32_t d, uint64_t n_words,
-                         uint64_t row_stride, uint32_t box_words, uint32_t box_rows) {
+                         uint64_t row_stride, uint32_t box_words, uint32_t box_rows, CUtensorMapSwizzle swizzle) {
     using EncodeFn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                   const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -482,14 +825,52 @@ bool encode_bits_map_box(CUtensorMap *map, const uint64_t *bitmaps, uint32_t d, 
     cuuint32_t box[2] = {box_words, box_rows};
     cuuint32_t estr[2] = {1, 1};
     return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, const_cast<uint64_t *>(bitmaps), dims, strides, box, estr,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 }  // namespace
 
 size_t tc_smem_bytes() { return (size_t)kTcStages * kTcStageBytes + (size_t)kTcRing * kTcBitSlot + 1024; }
+size_t f4_smem_bytes() {
+    static_assert(kF4ExpWarps * kF4Turn * 4 <= kF4Stages * kF4StageBytes, "transposes use the stages' memory");
+    return (size_t)kF4Stages * kF4StageBytes + (size_t)kF4Ring * kF4RingBytes + 1024;
+}
 size_t tc256_smem_bytes() { return (size_t)kT2Stages * kT2StageBytes + (size_t)kT2Ring * kT2BitSlot + 1024; }
+
+int cooc_f4_device(const uint64_t *bitmaps, uint32_t d, uint64_t n_words, uint64_t row_stride, uint32_t *out,
+                   cudaStream_t st, int n_sm, uint32_t *dev_err, uint64_t *launches) {
+    if (d == 0) return 0;
+    if ((reinterpret_cast<uintptr_t>(bitmaps) & 15) || (row_stride & 1)) return -1;
+    CUtensorMap map;
+    if (n_words && !encode_bits_map_box(&map, bitmaps, d, n_words, row_stride, kF4Words, 128,
+                                        CU_TENSOR_MAP_SWIZZLE_64B))
+        return -1;
+    SG_CUDA_TRY(cudaMemsetAsync(out, 0, (size_t)d * d * 4, st));
+    if (n_words == 0) return 0;
+    F4Work w;
+    w.d = d;
+    w.col_tiles = (d + kF4RowsB - 1) / kF4RowsB;
+    const uint32_t row_tiles = (d + kF4RowsA - 1) / kF4RowsA;
+    uint64_t tiles = 0;
+    for (uint32_t bi = 0; bi < row_tiles; ++bi) tiles += w.col_tiles - (bi >> 1);
+    w.tiles = tiles;
+    const uint64_t steps = (n_words + kF4Words - 1) / kF4Words;
+    w.total = tiles * steps;
+    // a CTA's share is a run where runs allow it: most CTAs then have one tile
+    w.share = std::max<uint64_t>(kF4MinSteps, (w.total + n_sm - 1) / n_sm);
+    w.run = std::min<uint64_t>(std::min<uint64_t>(steps, kF4MaxSteps), w.share);
+    const uint64_t grid = (w.total + w.share - 1) / w.share;
+    const uint64_t runs = (steps + w.run - 1) / w.run;
+    w.last = steps - (runs - 1) * w.run;
+    w.full = tiles * w.run * (runs - 1);
+    const size_t smem = f4_smem_bytes();
+    SG_CUDA_TRY(cudaFuncSetAttribute(cooc_f4_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    cooc_f4_kernel<<<(unsigned)grid, kF4Threads, smem, st>>>(map, w, out, dev_err);
+    SG_CUDA_TRY(cudaGetLastError());
+    if (launches) *launches += 1;
+    return 0;
+}
 
 int cooc_tc256_device(const uint64_t *bitmaps, uint32_t d, uint64_t n_words, uint64_t row_stride, uint32_t *out,
                       cudaStream_t st, int n_sm, uint32_t *dev_err, uint64_t *launches) {

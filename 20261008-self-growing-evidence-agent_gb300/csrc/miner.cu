@@ -397,8 +397,10 @@ void Miner::load_cooc() {
     if (d == 0 || d > 8192) return;
     DevBuf &out = w_.cooc;
     out.reserve((size_t)d * d * 4, h_->stream);
-    cooc_device(ds_.bitmaps.as<uint64_t>(), d, ds_.n_words, ds_.stride, out.as<uint32_t>(), 1, h_->stream, h_->n_sm,
-                nullptr, 0, &launches_);
+    for (int kind : {SGFIM_COOC_TC_F4, SGFIM_COOC_POPC})   // the popcount kernel when the layout does not suit
+        if (cooc_device(ds_.bitmaps.as<uint64_t>(), d, ds_.n_words, ds_.stride, out.as<uint32_t>(), kind, h_->stream,
+                        h_->n_sm, nullptr, 0, &launches_, h_->dev_err.as<uint32_t>()) == 0)
+            break;
     SG_CUDA_TRY(cudaMemcpyAsync(cooc_.data(), out.ptr, (size_t)d * d * 4, cudaMemcpyDeviceToHost, h_->stream));
     SG_CUDA_TRY(cudaStreamSynchronize(h_->stream));
 }
