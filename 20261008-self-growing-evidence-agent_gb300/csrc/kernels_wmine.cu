@@ -342,6 +342,7 @@ __device__ __forceinline__ uint32_t build_base(const WMineParams &p, uint64_t st
     const uint64_t m_first = ~0ull << (start & 63);
     const uint64_t m_last = n ? (~0ull >> (63 - ((start + n - 1) & 63))) : 0;
     uint32_t cn = 0;
+#pragma unroll 1
     for (uint64_t b = 0; b < nwd; b += 32) {
         const uint64_t i = b + lane;
         uint64_t bits = 0;
@@ -355,6 +356,7 @@ __device__ __forceinline__ uint32_t build_base(const WMineParams &p, uint64_t st
         }
         // pass 1: how many of this lane's transactions keep a tail item
         uint32_t mine = 0;
+#pragma unroll 1
         for (uint64_t x = bits; x; x &= x - 1) {
             const uint64_t pos = ((w0 + i) << 6) + (__ffsll((long long)x) - 1);
             mine += m_nz(m_and(m_load<MW>(p.hm + (pos & p.cap_mask) * MW), T));
@@ -368,6 +370,7 @@ __device__ __forceinline__ uint32_t build_base(const WMineParams &p, uint64_t st
         }
         uint64_t at = cn + incl - mine;
         // pass 2: write them
+#pragma unroll 1
         for (uint64_t x = bits; x; x &= x - 1) {
             const uint64_t pos = ((w0 + i) << 6) + (__ffsll((long long)x) - 1);
             const Mask<MW> m = m_and(m_load<MW>(p.hm + (pos & p.cap_mask) * MW), T);
@@ -382,96 +385,117 @@ __device__ __forceinline__ uint32_t build_base(const WMineParams &p, uint64_t st
     return cn > p.list_cap ? 0xffffffffu : cn;
 }
 
-// Position of item e among the items of T0: its row slot in the vertical layout.
-template <int MW> __device__ __forceinline__ uint32_t m_rank(const Mask<MW> &T0, uint32_t e) {
-    uint32_t r = 0;
-    const uint32_t wi = e >> 6;
+// 32 x 32 bit transpose over the warp: lane i ends with bit i of every lane's word.
+__device__ __forceinline__ uint32_t transpose32(uint32_t x, uint32_t lane) {
+    uint32_t y = __shfl_xor_sync(kFull, x, 16);
+    x = lane & 16 ? __byte_perm(x, y, 0x3276) : __byte_perm(x, y, 0x5410);
+    y = __shfl_xor_sync(kFull, x, 8);
+    x = lane & 8 ? __byte_perm(x, y, 0x3715) : __byte_perm(x, y, 0x6240);
+    const uint32_t m[3] = {0x0f0f0f0fu, 0x33333333u, 0x55555555u};
 #pragma unroll
-    for (int k = 0; k < MW; ++k) {
-        const uint64_t below = (uint32_t)k < wi ? ~0ull : ((uint32_t)k == wi ? ((1ull << (e & 63)) - 1) : 0ull);
-        r += __popcll(T0.w[k] & below);
+    for (int i = 0; i < 3; ++i) {
+        const int j = 4 >> i;
+        y = __shfl_xor_sync(kFull, x, j);
+        x = lane & j ? (x & ~m[i]) | ((y >> j) & m[i]) : (x & m[i]) | ((y & m[i]) << j);
     }
-    return r;
+    return x;
 }
 
-// Vertical rows of a database of n0 entries: bit i of word c of row slot s is
-// set when entry 32c+i holds the s-th item of T0 (entries are restricted to T0).
+// Vertical rows of a database of n0 entries, by item id: bit i of word c of row e
+// is set when entry 32c+i holds item e (rows of T0's items; vw a multiple of 4).
+// Four chunks of 32 entries at a time, so a row's words leave as one 16-byte store.
 template <int MW>
 __device__ __forceinline__ void build_rows(const uint64_t *lists, uint32_t n0, const Mask<MW> &T0, uint32_t *rows,
                                            uint32_t vw, uint32_t lane) {
     const uint32_t W = (n0 + 31) / 32;
-    for (uint32_t c = 0; c < W; ++c) {
-        const uint32_t i = c * 32 + lane;
-        const Mask<MW> m = i < n0 ? m_load<MW>(lists + (uint64_t)i * MW) : m_zero<MW>();
-        uint32_t mine = 0, slot = 0;
+#pragma unroll 1
+    for (uint32_t c = 0; c < W; c += 4) {
+        Mask<MW> m[4];
 #pragma unroll
-        for (int ww = 0; ww < MW; ++ww) {
-            const uint64_t mw_ = m.w[ww];
-            uint64_t x = T0.w[ww];
-            while (x) {
-                const uint32_t bit = __ffsll((long long)x) - 1;
-                x &= x - 1;
-                const uint32_t word = __ballot_sync(kFull, (mw_ >> bit) & 1ull);
-                if (lane == (slot & 31)) mine = word;
-                ++slot;
-                if ((slot & 31) == 0) rows[(uint64_t)(slot - 32 + lane) * vw + c] = mine;
-            }
+        for (int u = 0; u < 4; ++u) {
+            const uint32_t i = (c + u) * 32 + lane;
+            m[u] = i < n0 ? m_load<MW>(lists + (uint64_t)i * MW) : m_zero<MW>();
         }
-        if ((slot & 31) && lane < (slot & 31)) rows[(uint64_t)((slot & ~31u) + lane) * vw + c] = mine;
-    }
-    __syncwarp();
-}
-
-// c_e = popc(tid AND row(e)) for e in T (lane 0 writes cnt[e]).
-template <int MW>
-__device__ __forceinline__ void vcount(const uint32_t *tid, const uint32_t *rows, uint32_t vw, uint32_t W,
-                                       const Mask<MW> &T, const Mask<MW> &T0, uint32_t *cnt, uint32_t lane) {
-    constexpr uint32_t kReg = 4;   // tidsets of up to 128 words stay in registers across the items
-    uint32_t tr[kReg];
-    const bool small = W <= 32 * kReg;
 #pragma unroll
-    for (uint32_t k = 0; k < kReg; ++k) tr[k] = (small && lane + 32 * k < W) ? tid[lane + 32 * k] : 0u;
+        for (int b = 0; b < 2 * MW; ++b) {
+            const uint32_t want = (uint32_t)(T0.w[b >> 1] >> ((b & 1) * 32));
+            if (!want) continue;
+            uint32_t w[4];
 #pragma unroll
-    for (int ww = 0; ww < MW; ++ww) {
-        uint64_t x = T.w[ww];
-        while (x) {
-            const uint32_t e = ww * 64 + (__ffsll((long long)x) - 1);
-            x &= x - 1;
-            const uint32_t *row = rows + (uint64_t)m_rank(T0, e) * vw;
-            uint32_t acc = 0;
-            if (small) {
-#pragma unroll
-                for (uint32_t k = 0; k < kReg; ++k)
-                    if (lane + 32 * k < W) acc += __popc(tr[k] & row[lane + 32 * k]);
-            } else {
-                for (uint32_t w = lane; w < W; w += 32) acc += __popc(tid[w] & row[w]);
-            }
-            acc = __reduce_add_sync(kFull, acc);
-            if (lane == 0) cnt[e] = acc;
+            for (int u = 0; u < 4; ++u) w[u] = transpose32((uint32_t)(m[u].w[b >> 1] >> ((b & 1) * 32)), lane);
+            if ((want >> lane) & 1u)
+                *reinterpret_cast<uint4 *>(rows + (uint64_t)(b * 32 + lane) * vw + c) = make_uint4(w[0], w[1], w[2], w[3]);
         }
     }
     __syncwarp();
 }
 
-// |{entries of tid holding every item of F}|
-template <int MW>
-__device__ __forceinline__ uint32_t vcount_superset(const uint32_t *tid, const uint32_t *rows, uint32_t vw, uint32_t W,
-                                                    const Mask<MW> &F, const Mask<MW> &T0, uint32_t lane) {
-    uint32_t acc = 0;
-    for (uint32_t w = lane; w < W; w += 32) {
-        uint32_t v = tid[w];
+// Tidset words a lane keeps in registers (tidsets of up to 128 words).
+constexpr uint32_t kReg = 4;
+
+// cnt[i] = popc(tidset AND row(items[i])), four items at a time, a lane per word;
+// R: words per lane (0: the tidset is read from tid).  Two sums share a reduction
+// while the database has fewer than 65,536 entries.
+template <int R>
+__device__ __forceinline__ void count_tail(const uint32_t *rows, uint32_t vw, uint32_t W, const uint32_t (&tr)[kReg],
+                                           const uint32_t *tid, const uint8_t *items, uint32_t nt, bool two,
+                                           uint32_t *cnt, uint32_t lane) {
+#pragma unroll 1
+    for (uint32_t i = 0; i < nt; i += 4) {
+        const uint32_t *r[4];
+        uint32_t a[4] = {0, 0, 0, 0};
 #pragma unroll
-        for (int ww = 0; ww < MW; ++ww) {
-            uint64_t x = F.w[ww];
-            while (x && v) {
-                const uint32_t e = ww * 64 + (__ffsll((long long)x) - 1);
-                x &= x - 1;
-                v &= rows[(uint64_t)m_rank(T0, e) * vw + w];
+        for (int u = 0; u < 4; ++u) r[u] = rows + (uint32_t)items[min(i + u, nt - 1)] * vw;
+        if (R > 0) {
+#pragma unroll
+            for (int k = 0; k < R; ++k)
+                if (lane + 32 * k < W)
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) a[u] += __popc(tr[k] & r[u][lane + 32 * k]);
+        } else {
+#pragma unroll 2
+            for (uint32_t x = lane; x < W; x += 32) {
+                const uint32_t v = tid[x];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) a[u] += __popc(v & r[u][x]);
             }
         }
-        acc += __popc(v);
+        if (two) {
+            const uint32_t s = __reduce_add_sync(kFull, a[0] | a[1] << 16), t = __reduce_add_sync(kFull, a[2] | a[3] << 16);
+            a[0] = s & 0xffffu;
+            a[1] = s >> 16;
+            a[2] = t & 0xffffu;
+            a[3] = t >> 16;
+        } else {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) a[u] = __reduce_add_sync(kFull, a[u]);
+        }
+        if (lane == 0) *reinterpret_cast<uint4 *>(cnt + i) = make_uint4(a[0], a[1], a[2], a[3]);
     }
-    return __reduce_add_sync(kFull, acc);
+}
+
+// Support of the node's head with all k items, rarest first, or any number below
+// thr once it falls below.
+template <int R>
+__device__ __forceinline__ uint32_t count_all(const uint32_t *rows, uint32_t vw, uint32_t W, const uint32_t (&tr)[kReg],
+                                              const uint8_t *items, uint32_t k, uint32_t thr, uint32_t lane) {
+    uint32_t v[R], cf = 0;
+#pragma unroll
+    for (int x = 0; x < R; ++x) v[x] = tr[x];
+#pragma unroll 1
+    for (uint32_t i = 0; i < k; i += 2) {
+        const uint32_t *r0 = rows + (uint32_t)items[i] * vw, *r1 = rows + (uint32_t)items[min(i + 1, k - 1)] * vw;
+        uint32_t a = 0;
+#pragma unroll
+        for (int x = 0; x < R; ++x)
+            if (lane + 32 * x < W) {
+                v[x] &= r0[lane + 32 * x] & r1[lane + 32 * x];
+                a += __popc(v[x]);
+            }
+        cf = __reduce_add_sync(kFull, a);
+        if (cf < thr) break;
+    }
+    return cf;
 }
 
 }  // namespace
@@ -900,7 +924,7 @@ template <int MW> __global__ void __launch_bounds__(128) wtask_kernel(WMineParam
     }
 }
 
-// Resident CTAs per SM the register allocation is fitted to.  Measured on the
+// Resident CTAs per SM the register allocation is fitted to.  Measured with tails as masks on the
 // 4,096 service windows: 6 (80 registers, 3,648 warps) 337 ms, 7 (72 registers,
 // 4,176 warps, the workspace budget's limit) 338 ms with a longer makespan, 8
 // (64 registers, spills) 358 ms -- more resident warps do not shorten the search.
@@ -908,12 +932,27 @@ template <int MW> __global__ void __launch_bounds__(128) wtask_kernel(WMineParam
 #define SGFIM_WVTASK_MIN_BLOCKS 6
 #endif
 
+// A node's tail is a list in shared memory, ascending (support, id) in its parent.
+// Counting runs with a lane per tidset word, four items at a time; the frequent
+// items are packed, sorted by (support, id) (an item's place is the number of
+// smaller keys) and become the node's record and its children's tails.  FHUT ANDs
+// the rows rarest first and stops as soon as fewer than thr transactions are left.
+// Bound by instruction issue and by fetching them (tidsets of 16 to 2,048 words:
+// each item's count is a few loads and a reduction).  Item by item with 64-bit
+// masks the node cost 2,000 instructions, now 1,060, and the code is 68 KB instead
+// of 84.  45 windows of 512 to 65,536 transactions (floor 2%): 8.8 -> 6.5 ms, of
+// which the longest task is 6.1 ms; 768 windows: 69 -> 44 ms.
 template <int MW> __global__ void __launch_bounds__(128, SGFIM_WVTASK_MIN_BLOCKS) wvtask_kernel(WMineParams p) {
-    __shared__ uint32_t s_cnt[4][128];
+    constexpr uint32_t NI = 64 * MW;                        // items
+    __shared__ __align__(16) uint32_t s_cnt[4][NI];
+    __shared__ uint64_t s_key[4][NI];                       // (support, id) of the frequent items
+    __shared__ uint8_t s_tail[4][NI], s_sort[4][NI];        // a node's tail; its frequent part, sorted
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t wib = threadIdx.x >> 5;
     const uint64_t warp = (uint64_t)blockIdx.x * (blockDim.x >> 5) + wib;
+    uint8_t *tail = s_tail[wib], *sorted = s_sort[wib];
     uint32_t *cnt = s_cnt[wib];
+    uint64_t *keys = s_key[wib];
     uint64_t *lists = p.lists + warp * (uint64_t)p.list_cap * MW;
     uint32_t *lmfi = p.lmfi + warp * (uint64_t)p.lmfi_cap;
     uint64_t *pool = p.pool_m + warp * (uint64_t)p.pool_cap * MW;
@@ -922,7 +961,7 @@ template <int MW> __global__ void __launch_bounds__(128, SGFIM_WVTASK_MIN_BLOCKS
     const WRoot<MW> *roots = reinterpret_cast<const WRoot<MW> *>(p.roots);
     const uint32_t d = p.d;
     const uint32_t vw = p.v_words;
-    uint32_t *vrows = p.vbuf + warp * (uint64_t)(128 + kWDepth) * vw;   // row slot s: vrows + s * vw
+    uint32_t *vrows = p.vbuf + warp * (uint64_t)(128 + kWDepth) * vw;   // item e: vrows + e * vw
     uint32_t *vtid = vrows + (uint64_t)128 * vw;                        // level l: vtid + l * vw
 
     for (;;) {
@@ -943,30 +982,21 @@ template <int MW> __global__ void __launch_bounds__(128, SGFIM_WVTASK_MIN_BLOCKS
         uint32_t np = 0;
         uint64_t nodes = 0;
 
-        // the task's first node: the whole window, or child `child` of its root
-        bool ring0 = child == kWholeWindow;
-        Mask<MW> H = m_zero<MW>(), T = m_zero<MW>();
-        uint32_t sup = n, list_n = n;
-        bool done = false;   // a split child that is itself terminal: its one candidate
-        if (ring0) {
-            for (uint32_t e = 0; e < d; ++e) m_set(T, e);
-            list_n = build_base<MW>(p, start, n, m_zero<MW>(), T, lists, lane);
-            if (list_n == 0xffffffffu) status = 1;
+        // the task's first node: the whole window, or a child (grandchild) of its root
+        Mask<MW> H = m_zero<MW>(), T0 = m_zero<MW>(), req = m_zero<MW>();
+        uint32_t sup = n, list_n = n, nt = 0;
+        bool done = false;               // a split child that is itself terminal: its one candidate
+        const uint8_t *src = nullptr;    // where the first tail is listed (null: all items)
+        if (child == kWholeWindow) {
+            nt = d;
         } else if (sub == kWholeWindow) {
             const WRoot<MW> &R = roots[w];
-            const uint32_t k = R.k;
-            for (uint32_t q = child + 1 + lane; q < k; q += 32) m_set(T, R.f[q]);
-            T = warp_or(T);
             H = m_load<MW>(R.hp);
-            Mask<MW> req = m_zero<MW>();
             m_set(req, R.f[child]);
             m_set(H, R.f[child]);
             sup = R.c[child];
-            list_n = 0;
-            if (m_nz(T)) {
-                list_n = build_base<MW>(p, start, n, req, T, lists, lane);
-                if (list_n == 0xffffffffu) status = 1;
-            }
+            src = R.f + child + 1;
+            nt = R.k - child - 1;
         } else {
             const WRoot<MW> &S = reinterpret_cast<const WRoot<MW> *>(p.subs)[sub];
             if (S.overflow) {
@@ -978,32 +1008,47 @@ template <int MW> __global__ void __launch_bounds__(128, SGFIM_WVTASK_MIN_BLOCKS
                 nodes = 1;
                 done = true;
             } else {
-                const uint32_t k1 = S.k;
-                for (uint32_t q = gchild + 1 + lane; q < k1; q += 32) m_set(T, S.f[q]);
-                T = warp_or(T);
                 H = m_load<MW>(S.hp);
-                Mask<MW> req = m_zero<MW>();
                 m_set(req, roots[w].f[child]);
                 m_set(req, S.f[gchild]);
                 m_set(H, S.f[gchild]);
                 sup = S.c[gchild];
-                list_n = 0;
-                if (m_nz(T)) {
-                    list_n = build_base<MW>(p, start, n, req, T, lists, lane);
-                    if (list_n == 0xffffffffu) status = 1;
-                }
+                src = S.f + gchild + 1;
+                nt = S.k - gchild - 1;
             }
         }
-        // ---- the task's database as vertical rows over its entries (one row per item of T0)
-        const Mask<MW> T0 = T;
-        const uint32_t W = (list_n + 31) / 32;
+#pragma unroll 1
+        for (uint32_t i = lane; i < nt; i += 32) {
+            const uint32_t e = src ? src[i] : i;
+            tail[i] = (uint8_t)e;
+            m_set(T0, e);
+        }
+        T0 = warp_or(T0);
         if (status == 0 && !done) {
-            if (W > vw) {
+            list_n = 0;
+            if (nt) {
+                list_n = build_base<MW>(p, start, n, req, T0, lists, lane);
+                if (list_n == 0xffffffffu) status = 1;
+            }
+        }
+        // ---- the task's database as vertical rows over its entries
+        const uint32_t W = (list_n + 31) / 32;
+        const bool small = W <= 32 * kReg, two = list_n < 65536;
+        const uint32_t nk = (W + 31) / 32;   // words per lane
+        uint32_t tr[kReg] = {0, 0, 0, 0};   // the node's tidset, when small
+        if (status == 0 && !done) {
+            if (((W + 3) & ~3u) > vw) {
                 status = 1;
             } else {
                 build_rows<MW>(lists, list_n, T0, vrows, vw, lane);
-                for (uint32_t x = lane; x < W; x += 32)
-                    vtid[x] = (x + 1 < W || (list_n & 31) == 0) ? 0xffffffffu : ((1u << (list_n & 31)) - 1);
+#pragma unroll 1
+                for (uint32_t x = lane; x < W; x += 32) {
+                    const uint32_t v = (x + 1 < W || (list_n & 31) == 0) ? 0xffffffffu : ((1u << (list_n & 31)) - 1);
+                    vtid[x] = v;
+#pragma unroll
+                    for (uint32_t k = 0; k < kReg; ++k)
+                        if (x == lane + 32 * k) tr[k] = v;
+                }
                 __syncwarp();
             }
         }
@@ -1016,19 +1061,45 @@ template <int MW> __global__ void __launch_bounds__(128, SGFIM_WVTASK_MIN_BLOCKS
                 expand = false;
                 ++nodes;
                 const uint32_t *tid = vtid + (uint64_t)l * vw;
-                vcount<MW>(tid, vrows, vw, W, T, T0, cnt, lane);
-                Mask<MW> P, F;
-                classify<MW>(T, cnt, d, thr, sup, lane, P, F);
-                Mask<MW> Hp, Q;
-                uint32_t k = 0;
-#pragma unroll
-                for (int i = 0; i < MW; ++i) {
-                    Hp.w[i] = H.w[i] | P.w[i];
-                    Q.w[i] = Hp.w[i] | F.w[i];
-                    k += __popcll(F.w[i]);
+                // ---- supports of the tail's items
+                if (nk <= 1) count_tail<1>(vrows, vw, W, tr, tid, tail, nt, two, cnt, lane);
+                else if (nk <= 2) count_tail<2>(vrows, vw, W, tr, tid, tail, nt, two, cnt, lane);
+                else if (small) count_tail<4>(vrows, vw, W, tr, tid, tail, nt, two, cnt, lane);
+                else count_tail<0>(vrows, vw, W, tr, tid, tail, nt, two, cnt, lane);
+                __syncwarp();
+                // ---- PEP items P (they join H) and the frequent tail F
+                Mask<MW> Pl = m_zero<MW>(), Fl = m_zero<MW>();
+                uint32_t k = 0, any_p = 0;
+#pragma unroll 1
+                for (uint32_t b = 0; b < nt; b += 32) {
+                    const bool in = b + lane < nt;
+                    const uint32_t e = in ? tail[b + lane] : 0, c = in ? cnt[b + lane] : 0;
+                    const bool isp = in && c >= thr && c == sup, isf = in && c >= thr && c < sup;
+                    const uint32_t bal = __ballot_sync(kFull, isf);
+                    any_p |= __ballot_sync(kFull, isp);
+                    if (isp) m_set(Pl, e);
+                    if (isf) {
+                        m_set(Fl, e);
+                        keys[k + __popc(bal & ((1u << lane) - 1))] = (uint64_t)c << 8 | e;
+                    }
+                    k += __popc(bal);
                 }
+                Mask<MW> Hp = H, Q;
+                if (any_p) {
+                    Pl = warp_or(Pl);
+#pragma unroll
+                    for (int i = 0; i < MW; ++i) Hp.w[i] |= Pl.w[i];
+                }
+                Q = Hp;
+                if (k) {
+                    Fl = warp_or(Fl);
+#pragma unroll
+                    for (int i = 0; i < MW; ++i) Q.w[i] |= Fl.w[i];
+                }
+                __syncwarp();
                 // ---- is H u P u F inside a known MFI?  (local list; nothing was found since entry)
                 bool hit = false;
+#pragma unroll 1
                 for (uint32_t b = 0; b < lm_n && !hit; b += 32 * kU) {
                     uint32_t idx[kU];
 #pragma unroll
@@ -1054,8 +1125,39 @@ template <int MW> __global__ void __launch_bounds__(128, SGFIM_WVTASK_MIN_BLOCKS
                     __syncwarp();
                     continue;
                 }
+                // ---- F by (support, id): an item's place is the number of smaller keys
+                WLevel<MW> &A = LV[l];
+#pragma unroll 1
+                for (uint32_t b = 0; b < k; b += 32) {
+                    const uint64_t mine = b + lane < k ? keys[b + lane] : ~0ull;
+                    uint32_t rank = 0;
+#pragma unroll 2
+                    for (uint32_t i = 0; i < k; ++i) rank += keys[i] < mine;
+                    if (b + lane < k) {
+                        sorted[rank] = (uint8_t)mine;
+                        A.f[rank] = (uint8_t)mine;
+                        A.c[rank] = (uint32_t)(mine >> 8);
+                    }
+                }
+                __syncwarp();
                 // ---- FHUT: support of H u P u F
-                const uint32_t cf = vcount_superset<MW>(tid, vrows, vw, W, F, T0, lane);
+                uint32_t cf = 0;
+                if (nk <= 1) {
+                    cf = count_all<1>(vrows, vw, W, tr, sorted, k, thr, lane);
+                } else if (nk <= 2) {
+                    cf = count_all<2>(vrows, vw, W, tr, sorted, k, thr, lane);
+                } else if (small) {
+                    cf = count_all<4>(vrows, vw, W, tr, sorted, k, thr, lane);
+                } else {
+#pragma unroll 1
+                    for (uint32_t x = lane; x < W; x += 32) {
+                        uint32_t v = tid[x];
+#pragma unroll 1
+                        for (uint32_t i = 0; i < k && v; ++i) v &= vrows[sorted[i] * vw + x];
+                        cf += __popc(v);
+                    }
+                    cf = __reduce_add_sync(kFull, cf);
+                }
                 if (cf >= thr) {
                     if (np >= p.pool_cap) { status = 1; break; }
                     if (lane < MW) pool[(uint64_t)np * MW + lane] = m_word(Q, lane);
@@ -1066,9 +1168,7 @@ template <int MW> __global__ void __launch_bounds__(128, SGFIM_WVTASK_MIN_BLOCKS
                     __syncwarp();
                     continue;
                 }
-                // ---- record the node: frequent tail sorted by (support, id)
-                WLevel<MW> &A = LV[l];
-                sort_tail<MW>(F, cnt, lane, A.f, A.c);
+                // ---- record the node
                 if (lane < MW) A.hp[lane] = m_word(Hp, lane);
                 if (lane == 0) {
                     A.lm_off = lm_off;
@@ -1091,24 +1191,36 @@ template <int MW> __global__ void __launch_bounds__(128, SGFIM_WVTASK_MIN_BLOCKS
             if (lane == 0) A.j = j + 1;
             const uint32_t e = A.f[j];
             const uint32_t csup = A.c[j];
-            Mask<MW> Tc = m_zero<MW>();
-            for (uint32_t q = j + 1 + lane; q < k; q += 32) m_set(Tc, A.f[q]);
-            Tc = warp_or(Tc);
             Mask<MW> Hc = m_load<MW>(A.hp);
             m_set(Hc, e);
             {
                 // child tidset = parent tidset AND row(e)
                 const uint32_t *ptid = vtid + (uint64_t)l * vw;
                 uint32_t *ctid = vtid + (uint64_t)(l + 1) * vw;
-                const uint32_t *row = vrows + (uint64_t)m_rank(T0, e) * vw;
-                if (l + 1 < kWDepth)
-                    for (uint32_t x = lane; x < W; x += 32) ctid[x] = ptid[x] & row[x];
+                const uint32_t *row = vrows + e * vw;
+                if (l + 1 < kWDepth) {
+                    if (small) {
+#pragma unroll
+                        for (uint32_t x = 0; x < kReg; ++x)
+                            if (lane + 32 * x < W) {
+                                tr[x] = ptid[lane + 32 * x] & row[lane + 32 * x];
+                                ctid[lane + 32 * x] = tr[x];
+                            }
+                    } else {
+#pragma unroll 1
+                        for (uint32_t x = lane; x < W; x += 32) ctid[x] = ptid[x] & row[x];
+                    }
+                }
             }
+            nt = k - j - 1;
+#pragma unroll 1
+            for (uint32_t i = lane; i < nt; i += 32) tail[i] = A.f[j + 1 + i];
             // child local-MFI list: members containing the child's head
             const uint32_t c_lm = A.lm_off + A.lm_n;
             const uint32_t p_lm_off = A.lm_off, p_lm_n = A.lm_n, p_entry = A.entry;
             const uint32_t n_src = p_lm_n + (np - p_entry);
             uint32_t ln = 0;
+#pragma unroll 1
             for (uint32_t b = 0; b < n_src; b += 32 * kU) {
                 uint32_t idx[kU];
                 bool keep[kU];
@@ -1136,7 +1248,6 @@ template <int MW> __global__ void __launch_bounds__(128, SGFIM_WVTASK_MIN_BLOCKS
             __syncwarp();
             ++l;
             H = Hc;
-            T = Tc;
             sup = csup;
             lm_off = c_lm;
             lm_n = ln;
@@ -1153,7 +1264,9 @@ template <int MW> __global__ void __launch_bounds__(128, SGFIM_WVTASK_MIN_BLOCKS
                 status = 2;
             } else {
                 __syncwarp();
+#pragma unroll 1
                 for (uint32_t i = lane; i < np * MW; i += 32) p.out_m[off * MW + i] = pool[i];
+#pragma unroll 1
                 for (uint32_t i = lane; i < np; i += 32) p.out_s[off + i] = pool_s[i];
             }
         }

@@ -378,7 +378,7 @@ int sgfim_ring_mine_windows(sgfim_ring *r, sgfim_handle *h, const uint64_t *star
             const uint64_t list_cap = std::min<uint64_t>(
                 std::max<uint64_t>(8192, (vertical ? 1 : 2) * max_len + 1024), 1ull << 30);
             const uint64_t lmfi_cap = 1u << 16, pool_cap = 1u << 16;
-            const uint64_t v_words = vertical ? (max_len + 31) / 32 + 1 : 0;
+            const uint64_t v_words = vertical ? ((max_len + 31) / 32 + 1 + 3) & ~3ull : 0;   // whole 16-byte pieces
             const size_t v_bytes = (size_t)(128 + wmine_depth()) * v_words * 4;
             const size_t per_warp =
                 list_cap * mw * 8 + lmfi_cap * 4 + pool_cap * (mw * 8 + 4) + wmine_level_bytes(mw) + v_bytes;

@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(256) to_columns_kernel(const double *__restric
 // to its digit.  Ranks with the same prefix share a histogram.
 //
 // Bound: HBM/L2, one read of the columns per pass and group of prefixes, and
-// shared-memory atomics.  1,000,000 rows x 21 sensors, 12 ranks: 0.65 ms for the
+// shared-memory atomics.  1,000,000 rows x 21 sensors, 13 ranks: 0.65 ms for the
 // six passes against 7.3 ms for one CTA per (sensor, rank) and eight passes;
 // the transpose 68 us (143 us when every lane stored to its own column).
 constexpr int kDigitBits = 11;
