@@ -123,14 +123,12 @@ struct Staged {
 // table and its per-window results.
 struct WindowWorkspace {
     DevBuf lists, lmfi, pool_m, pool_s, levels, out_m, out_s, ctrl, table, res, sub, tasks, vbuf;
-    HostBuf h_table, h_res, h_out;
+    HostBuf h_table, h_res, h_out, h_sub[2];
     void release() {
         for (DevBuf *b : {&lists, &lmfi, &pool_m, &pool_s, &levels, &out_m, &out_s, &ctrl, &table, &res, &sub, &tasks,
                           &vbuf})
             b->release();
-        h_table.release();
-        h_res.release();
-        h_out.release();
+        for (HostBuf *b : {&h_table, &h_res, &h_out, &h_sub[0], &h_sub[1]}) b->release();
     }
 };
 

@@ -158,10 +158,9 @@ int cooc_tc_device(const uint64_t *bitmaps, uint32_t d, uint64_t n_words, uint64
                    cudaStream_t st, int n_sm, uint32_t *dev_err, uint64_t *launches);
 size_t cooc_scratch_bytes(uint32_t d, uint64_t n_words, int kind);
 
-// Batched window miner (kernels_wmine.cu).  A task is a whole window
-// (child == kWholeWindow) or one subtree of a split window's root (child =
-// index into the root's sorted frequent tail; wroot_kernel fills the root
-// records first).  Per-warp workspaces are warp-major: lists list_cap x MW
+// Batched window miner (kernels_wmine.cu).  A task is a whole window or one
+// child's subtree of an expanded node: the root of a split window (wroot_kernel
+// fills the root records first) or a node below it (wsub_kernel).  Per-warp workspaces are warp-major: lists list_cap x MW
 // words, lmfi lmfi_cap, pool pool_cap x MW words + pool_cap supports, levels
 // wmine_level_bytes(MW).  task_status: 0 done, 1 workspace overflow (mine the
 // window elsewhere), 2 output arena full (retry the task).
@@ -178,18 +177,26 @@ struct WMineParams {
     void *roots = nullptr;              // per window, wmine_root_bytes(MW) each
     const uint32_t *split_win = nullptr;
     uint32_t n_split = 0;
-    void *subs = nullptr;               // split root children, wmine_root_bytes(MW) each
+    // expanded nodes below the roots (wmine_root_bytes(MW) each): launch_wsub expands child
+    // sub_child[i] of record sub_parent[i] of sub_parents (the roots by window, or subs) into
+    // subs[sub_out + i]; sub_next: its work counter (zero)
+    void *subs = nullptr;
+    const void *sub_parents = nullptr;
     const uint32_t *sub_win = nullptr;
+    const uint32_t *sub_parent = nullptr;
     const uint32_t *sub_child = nullptr;
-    uint32_t n_sub = 0;
+    uint32_t *sub_next = nullptr;
+    uint32_t n_sub = 0, sub_out = 0;
+    // per task: its window; the record it starts from (index into subs, kWholeWindow = the
+    // window's root) and the child (kWholeWindow = the record's own candidate, or with no record
+    // the whole window); how many children from that one on (more than one: wvtask_kernel only)
     const uint32_t *task_win = nullptr;
+    const uint32_t *task_rec = nullptr;
     const uint32_t *task_child = nullptr;
-    const uint32_t *task_sub = nullptr;     // null or per task: split-child record, kWholeWindow = none
-    const uint32_t *task_gchild = nullptr;  // per task with a record: grandchild index, kWholeWindow = the
-                                            // record's own candidate (a terminal child)
+    const uint32_t *task_n_child = nullptr;
     const uint32_t *task_order = nullptr;
     uint32_t n_tasks = 0;
-    uint32_t *next = nullptr;           // [0] task counter, [1] root counter, [2] split-child counter
+    uint32_t *next = nullptr;           // [0] task counter, [1] root counter
     uint64_t *lists = nullptr;
     uint32_t list_cap = 0;
     uint32_t *lmfi = nullptr;
@@ -249,7 +256,7 @@ struct WGatherParams {
 };
 size_t wmine_level_bytes(int mw);
 size_t wmine_root_bytes(int mw);
-// blocks of 128 threads (4 warps; wfilter: 256 or 1,024 threads)
+// blocks of 128 threads (4 warps; wroot: 256; wfilter: 256 or 1,024 threads)
 void launch_wroot(const WMineParams &p, int mw, unsigned blocks, cudaStream_t st);
 void launch_wsub(const WMineParams &p, int mw, unsigned blocks, cudaStream_t st);
 void launch_wtask(const WMineParams &p, int mw, unsigned blocks, cudaStream_t st);

@@ -6,15 +6,14 @@
 // window's transactions at the window's floor, which these kernels reproduce.
 //
 // Representation.  Items are the ring's dense ids 0..d-1 (d <= 64*MW); an
-// itemset is an MW-word mask.  A task's base database holds one MW-word entry
-// per window transaction that contains the task's required items and still
-// holds a tail item, restricted to the tail (build_base: the transactions are
-// found through the ring's vertical rows, their item masks read from the
-// ring's horizontal masks).  wvtask_kernel (the default) turns the base into
-// vertical rows, one bit per entry per item, and keeps one tidset per search
-// level: counts are AND-popcounts of the level's tidset with the item rows.
-// wtask_kernel (SGFIM_F_WINDOWS_HORIZONTAL) instead stacks each level's
-// projected database as entries.
+// itemset is an MW-word mask.  A task's base database is the window's
+// transactions that contain the task's required items, found through the ring's
+// vertical rows; their item masks are read from the ring's horizontal masks.
+// wvtask_kernel (the default) turns them into vertical rows, one bit per entry
+// per item, and keeps one tidset per search level: counts are AND-popcounts of
+// the level's tidset with the item rows.  wtask_kernel
+// (SGFIM_F_WINDOWS_HORIZONTAL) instead stacks each level's projected database as
+// entries, restricted to the level's tail.
 //
 // Search.  Depth-first over the set-enumeration tree, one node at a time per
 // warp, children in ascending (support, id) order -- the order under which a
@@ -35,8 +34,8 @@
 // searches the whole tree and its pool is the exact MFI set.  Longer windows
 // are split at the root: wroot_kernel counts the root and sorts its frequent
 // tail f_0..f_{k-1}; task (w, j) searches child j's subtree alone.  The
-// costliest children are split once more (wsub_kernel expands child j the same
-// way; task (w, j, g) searches its child g).  Tasks share no pool, so a
+// costliest children are expanded the same way (wsub_kernel) and their children
+// become the tasks, the costliest of these once more.  Tasks share no pool, so a
 // candidate of one subtree may sit inside a candidate of an earlier subtree
 // in depth-first order (never of a later one, by the argument above);
 // wfilter_kernel removes exactly those with a vertical bitmap of the window's
@@ -136,27 +135,30 @@ template <int MW> struct alignas(16) WLevel {
     uint32_t lm_off, lm_n;  // local-MFI list (pool indices)
     uint32_t entry;         // pool size when the node was entered
     uint32_t k, j;          // frequent tail size, next child
+    uint32_t end;           // children to search: k, or a task's part of them
     uint8_t f[128];         // frequent tail, ascending (support, id)
     uint32_t c[128];        // supports of f
 };
 
-// Root of a split window (wroot_kernel), or a root child that is split again
-// (wsub_kernel); read by wtask_kernel.
+// An expanded node of a split window: its root (wroot_kernel), or a child of an
+// expanded node that is split again (wsub_kernel).  Its children are tasks, or
+// expanded in turn.
 template <int MW> struct alignas(16) WRoot {
-    uint64_t hp[MW];        // root head after PEP (items in every transaction)
-    uint64_t cand[MW];      // the window's only MFI when the root is terminal
+    uint64_t hp[MW];        // head after PEP (items in every transaction of the node)
+    uint64_t cand[MW];      // the node's only MFI when it is terminal
     uint32_t cand_sup;
-    uint32_t has_cand;      // 1: the MFI set is {cand}; 0: the tasks (k of them) hold it
+    uint32_t has_cand;      // 1: the subtree's MFIs are {cand}; 0: the children (k of them) hold them
     uint32_t k;
-    uint32_t overflow;      // subtree records: the node's database did not fit (mine the window elsewhere)
+    uint32_t pad;
     uint8_t f[128];
     uint32_t c[128];
+    uint64_t req[MW];       // the items that were chosen on the way here: the node's transactions hold them
 };
 
 // the host reads these fields of the root records (ring.cu)
 static_assert(offsetof(WRoot<2>, cand) == 16 && offsetof(WRoot<2>, cand_sup) == 32 &&
                   offsetof(WRoot<2>, has_cand) == 36 && offsetof(WRoot<2>, k) == 40 &&
-                  offsetof(WRoot<2>, overflow) == 44 && offsetof(WRoot<2>, f) == 48 && offsetof(WRoot<2>, c) == 176,
+                  offsetof(WRoot<2>, f) == 48 && offsetof(WRoot<2>, c) == 176,
               "root record layout read by sgfim_ring_mine_windows");
 
 __device__ __forceinline__ uint64_t globaltimer_ns() {
@@ -317,74 +319,6 @@ __device__ __forceinline__ uint32_t build_child(bool ring, const WMineParams &p,
 }
 
 
-// Base database of a task, found through the ring's vertical rows: the
-// window's transactions holding every item of req (at most two items; none =
-// every transaction), each as its item mask restricted to T, dropped when
-// empty, in transaction order, written at lists[0 ..).  Returns the count, or
-// 0xffffffff when it does not fit.
-template <int MW>
-__device__ __forceinline__ uint32_t build_base(const WMineParams &p, uint64_t start, uint32_t n, const Mask<MW> &req,
-                                               const Mask<MW> &T, uint64_t *lists, uint32_t lane) {
-    uint32_t r0 = 0xffffffffu, r1 = 0xffffffffu;
-#pragma unroll
-    for (int ww = 0; ww < MW; ++ww) {
-        uint64_t x = req.w[ww];
-        while (x) {
-            const uint32_t e = ww * 64 + (__ffsll((long long)x) - 1);
-            x &= x - 1;
-            if (r0 == 0xffffffffu) r0 = e;
-            else r1 = e;
-        }
-    }
-    const uint64_t cwm = p.ring_words - 1;
-    const uint64_t w0 = start >> 6;
-    const uint64_t nwd = n ? ((start + n - 1) >> 6) - w0 + 1 : 0;
-    const uint64_t m_first = ~0ull << (start & 63);
-    const uint64_t m_last = n ? (~0ull >> (63 - ((start + n - 1) & 63))) : 0;
-    uint32_t cn = 0;
-#pragma unroll 1
-    for (uint64_t b = 0; b < nwd; b += 32) {
-        const uint64_t i = b + lane;
-        uint64_t bits = 0;
-        if (i < nwd) {
-            bits = ~0ull;
-            if (i == 0) bits &= m_first;
-            if (i + 1 == nwd) bits &= m_last;
-            const uint64_t wq = (w0 + i) & cwm;
-            if (r0 != 0xffffffffu) bits &= p.ring_rows[(uint64_t)r0 * p.ring_words + wq];
-            if (r1 != 0xffffffffu) bits &= p.ring_rows[(uint64_t)r1 * p.ring_words + wq];
-        }
-        // pass 1: how many of this lane's transactions keep a tail item
-        uint32_t mine = 0;
-#pragma unroll 1
-        for (uint64_t x = bits; x; x &= x - 1) {
-            const uint64_t pos = ((w0 + i) << 6) + (__ffsll((long long)x) - 1);
-            mine += m_nz(m_and(m_load<MW>(p.hm + (pos & p.cap_mask) * MW), T));
-        }
-        // exclusive prefix over the lanes keeps transaction order
-        uint32_t incl = mine;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t v = __shfl_up_sync(kFull, incl, o);
-            if (lane >= (uint32_t)o) incl += v;
-        }
-        uint64_t at = cn + incl - mine;
-        // pass 2: write them
-#pragma unroll 1
-        for (uint64_t x = bits; x; x &= x - 1) {
-            const uint64_t pos = ((w0 + i) << 6) + (__ffsll((long long)x) - 1);
-            const Mask<MW> m = m_and(m_load<MW>(p.hm + (pos & p.cap_mask) * MW), T);
-            if (m_nz(m)) {
-                if (at < p.list_cap) m_store(lists + at * MW, m);
-                ++at;
-            }
-        }
-        cn += __shfl_sync(kFull, incl, 31);
-    }
-    __syncwarp();
-    return cn > p.list_cap ? 0xffffffffu : cn;
-}
-
 // 32 x 32 bit transpose over the warp: lane i ends with bit i of every lane's word.
 __device__ __forceinline__ uint32_t transpose32(uint32_t x, uint32_t lane) {
     uint32_t y = __shfl_xor_sync(kFull, x, 16);
@@ -399,35 +333,6 @@ __device__ __forceinline__ uint32_t transpose32(uint32_t x, uint32_t lane) {
         x = lane & j ? (x & ~m[i]) | ((y >> j) & m[i]) : (x & m[i]) | ((y & m[i]) << j);
     }
     return x;
-}
-
-// Vertical rows of a database of n0 entries, by item id: bit i of word c of row e
-// is set when entry 32c+i holds item e (rows of T0's items; vw a multiple of 4).
-// Four chunks of 32 entries at a time, so a row's words leave as one 16-byte store.
-template <int MW>
-__device__ __forceinline__ void build_rows(const uint64_t *lists, uint32_t n0, const Mask<MW> &T0, uint32_t *rows,
-                                           uint32_t vw, uint32_t lane) {
-    const uint32_t W = (n0 + 31) / 32;
-#pragma unroll 1
-    for (uint32_t c = 0; c < W; c += 4) {
-        Mask<MW> m[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const uint32_t i = (c + u) * 32 + lane;
-            m[u] = i < n0 ? m_load<MW>(lists + (uint64_t)i * MW) : m_zero<MW>();
-        }
-#pragma unroll
-        for (int b = 0; b < 2 * MW; ++b) {
-            const uint32_t want = (uint32_t)(T0.w[b >> 1] >> ((b & 1) * 32));
-            if (!want) continue;
-            uint32_t w[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) w[u] = transpose32((uint32_t)(m[u].w[b >> 1] >> ((b & 1) * 32)), lane);
-            if ((want >> lane) & 1u)
-                *reinterpret_cast<uint4 *>(rows + (uint64_t)(b * 32 + lane) * vw + c) = make_uint4(w[0], w[1], w[2], w[3]);
-        }
-    }
-    __syncwarp();
 }
 
 // Tidset words a lane keeps in registers (tidsets of up to 128 words).
@@ -500,176 +405,196 @@ __device__ __forceinline__ uint32_t count_all(const uint32_t *rows, uint32_t vw,
 
 }  // namespace
 
-// ------------------------------------------------------------------ roots
-// Root counts from the ring's vertical rows: item e's support in the window
-// is the popcount of its row over the window's bit range (the ring keeps
-// one row per item, 64 transactions per word).
-template <int MW> __global__ void __launch_bounds__(128) wroot_kernel(WMineParams p) {
-    __shared__ uint32_t s_cnt[4][128];
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t wib = threadIdx.x >> 5;
-    uint32_t *cnt = s_cnt[wib];
+// ------------------------------------------------------------------ expanded nodes
+// Supports come from the ring's vertical rows: the node's transactions are the
+// window's bit range ANDed with the rows of the items chosen so far (one row per
+// item, 64 transactions per word), and an item's support is the popcount of that
+// with its row.  A node's words are taken 128 at a time, four per lane.
+
+namespace {
+
+// The window's words of a node, four per lane from word b on: its bits in words
+// b + lane + 32 u of the window.
+template <int MW> struct NodeWords {
+    uint64_t w0, nwd, m_first, m_last, cwm;
+    const uint64_t *rows;
+    uint64_t ring_words;
+    __device__ NodeWords(const WMineParams &p, uint64_t start, uint32_t n) {
+        // unwrapped words w0 .., masked at both ends; ring words: a power of two
+        w0 = start >> 6;
+        nwd = n ? ((start + n - 1) >> 6) - w0 + 1 : 0;
+        m_first = ~0ull << (start & 63);
+        m_last = n ? (~0ull >> (63 - ((start + n - 1) & 63))) : 0;
+        cwm = p.ring_words - 1;
+        rows = p.ring_rows;
+        ring_words = p.ring_words;
+    }
+    __device__ __forceinline__ uint64_t word(uint32_t e, uint64_t i) const {
+        return rows[(uint64_t)e * ring_words + ((w0 + i) & cwm)];
+    }
+    __device__ __forceinline__ void load(uint64_t b, const Mask<MW> &req, uint32_t lane, uint64_t (&v)[4]) const {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const uint64_t i = b + lane + 32 * u;
+            v[u] = 0;
+            if (i < nwd) {
+                v[u] = ~0ull;
+                if (i == 0) v[u] &= m_first;
+                if (i + 1 == nwd) v[u] &= m_last;
+            }
+        }
+#pragma unroll
+        for (int ww = 0; ww < MW; ++ww)
+            for (uint64_t x = req.w[ww]; x; x &= x - 1) {
+                const uint32_t e = ww * 64 + (__ffsll((long long)x) - 1);
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (v[u]) v[u] &= word(e, b + lane + 32 * u);
+            }
+    }
+};
+
+// Finishes a node from its items' supports cnt[e], e in T: PEP, the frequent tail,
+// FHUT over the node's words, and the record (one warp).
+template <int MW>
+__device__ __forceinline__ void finish_node(const WMineParams &p, const NodeWords<MW> &nw, const Mask<MW> &H,
+                                            const Mask<MW> &T, const Mask<MW> &req, uint32_t sup, uint32_t thr,
+                                            const uint32_t *cnt, uint32_t lane, WRoot<MW> &S) {
+    Mask<MW> P, F;
+    classify<MW>(T, cnt, p.d, thr, sup, lane, P, F);
+    Mask<MW> Hp, cand;
+    uint32_t k = 0;
+#pragma unroll
+    for (int i = 0; i < MW; ++i) {
+        Hp.w[i] = H.w[i] | P.w[i];
+        cand.w[i] = Hp.w[i];
+        k += __popcll(F.w[i]);
+    }
+    uint32_t has = 0, csup = 0;
+    if (k == 0) {
+        has = m_nz(Hp) ? 1u : 0u;   // (a root without any item has no candidate)
+        csup = sup;
+    } else {
+        // FHUT: transactions holding every item of F
+        sort_tail<MW>(F, cnt, lane, S.f, S.c);
+        __syncwarp();
+        uint32_t acc = 0;
+        for (uint64_t b = 0; b < nw.nwd; b += 128) {
+            uint64_t v[4];
+            nw.load(b, req, lane, v);
+            for (uint32_t j = 0; j < k; ++j) {   // rarest first
+                const uint32_t e = S.f[j];
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (v[u]) v[u] &= nw.word(e, b + lane + 32 * u);
+                if (!__any_sync(kFull, (v[0] | v[1] | v[2] | v[3]) != 0)) break;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) acc += __popcll(v[u]);
+        }
+        const uint32_t cf = __reduce_add_sync(kFull, acc);
+        if (cf >= thr) {
+            has = 1;
+            csup = cf;
+#pragma unroll
+            for (int i = 0; i < MW; ++i) cand.w[i] |= F.w[i];
+        }
+    }
+    if (lane < MW) {
+        S.hp[lane] = m_word(Hp, lane);
+        S.cand[lane] = m_word(cand, lane);
+        S.req[lane] = m_word(req, lane);
+    }
+    if (lane == 0) {
+        S.cand_sup = csup;
+        S.has_cand = has;
+        S.k = has ? 0 : k;
+        S.pad = 0;
+    }
+    __syncwarp();
+}
+
+// acc[item] over the node's words for the items of T given by its bits: every
+// warp of `warps` takes its share of the items.
+template <int MW>
+__device__ __forceinline__ void count_node(const NodeWords<MW> &nw, const Mask<MW> &T, const Mask<MW> &req,
+                                           uint32_t first, uint32_t step, uint32_t *cnt, uint32_t lane) {
+    for (uint64_t b = 0; b < nw.nwd || b == 0; b += 128) {
+        uint64_t v[4];
+        nw.load(b, req, lane, v);
+        uint32_t at = 0;
+#pragma unroll
+        for (int ww = 0; ww < MW; ++ww)
+            for (uint64_t x = T.w[ww]; x; x &= x - 1, ++at) {
+                if (at % step != first) continue;
+                const uint32_t e = ww * 64 + (__ffsll((long long)x) - 1);
+                uint32_t acc = 0;
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (v[u]) acc += __popcll(v[u] & nw.word(e, b + lane + 32 * u));
+                acc = __reduce_add_sync(kFull, acc);
+                if (lane == 0) cnt[e] = (b ? cnt[e] : 0u) + acc;
+            }
+    }
+    __syncwarp();
+}
+
+}  // namespace
+
+// Roots of split windows: a CTA of 8 warps per window, the items shared out (a
+// warp per window left a batch of 45 windows on 45 warps: 0.55 ms, now 0.13).
+constexpr int kRootThreads = 256;
+template <int MW> __global__ void __launch_bounds__(kRootThreads) wroot_kernel(WMineParams p) {
+    __shared__ uint32_t cnt[128];
+    __shared__ uint32_t s_wi;
+    const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     WRoot<MW> *roots = reinterpret_cast<WRoot<MW> *>(p.roots);
-    const uint64_t cwm = p.ring_words - 1;   // ring words: a power of two
     for (;;) {
-        uint32_t wi = 0;
-        if (lane == 0) wi = atomicAdd(p.next + 1, 1u);
-        wi = __shfl_sync(kFull, wi, 0);
+        __syncthreads();
+        if (threadIdx.x == 0) s_wi = atomicAdd(p.next + 1, 1u);
+        __syncthreads();
+        const uint32_t wi = s_wi;
         if (wi >= p.n_split) break;
         const uint32_t w = p.split_win[wi];
-        const uint64_t start = p.starts[w];
         const uint32_t n = p.lens[w];
-        const uint32_t thr = p.thrs[w] ? p.thrs[w] : 1;
-        // window bits: unwrapped words w0 .. w1, masked at both ends
-        const uint64_t w0 = start >> 6, w1 = n ? (start + n - 1) >> 6 : w0;
-        const uint64_t nwd = n ? w1 - w0 + 1 : 0;
-        const uint64_t m_first = ~0ull << (start & 63);
-        const uint64_t m_last = n ? (~0ull >> (63 - ((start + n - 1) & 63))) : 0;
-        auto word_mask = [&](uint64_t i) {
-            uint64_t m = ~0ull;
-            if (i == 0) m &= m_first;
-            if (i + 1 == nwd) m &= m_last;
-            return m;
-        };
+        const NodeWords<MW> nw(p, p.starts[w], n);
         Mask<MW> T = m_zero<MW>();
         for (uint32_t e = 0; e < p.d; ++e) m_set(T, e);
-        for (uint32_t e = 0; e < p.d; ++e) {
-            const uint64_t *row = p.ring_rows + (uint64_t)e * p.ring_words;
-            uint32_t acc = 0;
-            for (uint64_t i = lane; i < nwd; i += 32) acc += __popcll(row[(w0 + i) & cwm] & word_mask(i));
-            acc = __reduce_add_sync(kFull, acc);
-            if (lane == 0) cnt[e] = acc;
-        }
-        __syncwarp();
-        Mask<MW> P, F;
-        classify<MW>(T, cnt, p.d, thr, n, lane, P, F);
-        uint32_t k = 0;
-#pragma unroll
-        for (int i = 0; i < MW; ++i) k += __popcll(F.w[i]);
-        WRoot<MW> &R = roots[w];
-        uint32_t has = 0, csup = 0;
-        Mask<MW> cand = P;   // root head after PEP (H = {} at the root)
-        if (k == 0) {
-            has = m_nz(P) ? 1u : 0u;
-            csup = n;
-        } else {
-            // FHUT: transactions holding every item of F
-            uint32_t acc = 0;
-            for (uint64_t i = lane; i < nwd; i += 32) {
-                uint64_t v = word_mask(i);
-#pragma unroll
-                for (int ww = 0; ww < MW; ++ww) {
-                    uint64_t x = F.w[ww];
-                    while (x && v) {
-                        const uint32_t e = ww * 64 + (__ffsll((long long)x) - 1);
-                        x &= x - 1;
-                        v &= p.ring_rows[(uint64_t)e * p.ring_words + ((w0 + i) & cwm)];
-                    }
-                }
-                acc += __popcll(v);
-            }
-            const uint32_t cf = __reduce_add_sync(kFull, acc);
-            if (cf >= thr) {
-                has = 1;
-                csup = cf;
-#pragma unroll
-                for (int i = 0; i < MW; ++i) cand.w[i] |= F.w[i];
-            }
-        }
-        if (!has && k) sort_tail<MW>(F, cnt, lane, R.f, R.c);
-        if (lane < MW) {
-            R.hp[lane] = m_word(P, lane);
-            R.cand[lane] = m_word(cand, lane);
-        }
-        if (lane == 0) {
-            R.cand_sup = csup;
-            R.has_cand = has;
-            R.k = has ? 0 : k;
-            R.overflow = 0;
-        }
-        __syncwarp();
+        count_node<MW>(nw, T, m_zero<MW>(), wib, kRootThreads / 32, cnt, lane);
+        __syncthreads();
+        if (wib == 0)
+            finish_node<MW>(p, nw, m_zero<MW>(), T, m_zero<MW>(), n, p.thrs[w] ? p.thrs[w] : 1, cnt, lane, roots[w]);
     }
 }
 
-// ------------------------------------------------------------------ split root children
-// Child j of a split window's root, expanded like a root: its database is
-// built from the ring (transactions holding f_j, restricted to f_{j+1..}),
-// then counts, PEP, FHUT and the sorted frequent tail go to its record.
+// Children of expanded nodes that are expanded themselves: child sub_child[i] of
+// record sub_parent[i] of `parents` (roots by window, or earlier records), a warp
+// each, into subs[sub_out + i].  (Counted over the children's listed databases they
+// took 2.0 ms in a batch of 45 windows, 0.25 ms this way.)
 template <int MW> __global__ void __launch_bounds__(128) wsub_kernel(WMineParams p) {
     __shared__ uint32_t s_cnt[4][128];
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t wib = threadIdx.x >> 5;
-    const uint64_t warp = (uint64_t)blockIdx.x * (blockDim.x >> 5) + wib;
     uint32_t *cnt = s_cnt[wib];
-    uint64_t *lists = p.lists + warp * (uint64_t)p.list_cap * MW;
-    const WRoot<MW> *roots = reinterpret_cast<const WRoot<MW> *>(p.roots);
+    const WRoot<MW> *parents = reinterpret_cast<const WRoot<MW> *>(p.sub_parents);
     WRoot<MW> *subs = reinterpret_cast<WRoot<MW> *>(p.subs);
     for (;;) {
         uint32_t si = 0;
-        if (lane == 0) si = atomicAdd(p.next + 2, 1u);
+        if (lane == 0) si = atomicAdd(p.sub_next, 1u);
         si = __shfl_sync(kFull, si, 0);
         if (si >= p.n_sub) break;
         const uint32_t w = p.sub_win[si], j = p.sub_child[si];
-        const uint64_t start = p.starts[w];
-        const uint32_t n = p.lens[w];
-        const uint32_t thr = p.thrs[w] ? p.thrs[w] : 1;
-        const WRoot<MW> &R = roots[w];
+        const WRoot<MW> &R = parents[p.sub_parent[si]];
         const uint32_t k = R.k;
-        Mask<MW> T = m_zero<MW>(), req = m_zero<MW>();
+        Mask<MW> T = m_zero<MW>();
         for (uint32_t q = j + 1 + lane; q < k; q += 32) m_set(T, R.f[q]);
         T = warp_or(T);
-        const uint32_t e = R.f[j];
-        m_set(req, e);
-        Mask<MW> H = m_load<MW>(R.hp);
-        m_set(H, e);
-        const uint32_t sup = R.c[j];
-        WRoot<MW> &S = subs[si];
-        uint32_t n1 = 0, overflow = 0;
-        if (m_nz(T)) {
-            // the child's database through the ring's row of item e: only the window's
-            // transactions holding e have their item masks read
-            n1 = build_base<MW>(p, start, n, req, T, lists, lane);
-            if (n1 == 0xffffffffu) {
-                overflow = 1;
-                n1 = 0;
-            }
-        }
-        count_items<MW>(false, p, start, lists, 0, n1, T, cnt, lane);
-        Mask<MW> P, F;
-        classify<MW>(T, cnt, p.d, thr, sup, lane, P, F);
-        uint32_t k1 = 0;
-        Mask<MW> Hp, cand;
-#pragma unroll
-        for (int i = 0; i < MW; ++i) {
-            Hp.w[i] = H.w[i] | P.w[i];
-            cand.w[i] = Hp.w[i];
-            k1 += __popcll(F.w[i]);
-        }
-        uint32_t has = 0, csup = 0;
-        if (k1 == 0) {
-            has = 1;   // Hp holds f_j
-            csup = sup;
-        } else {
-            const uint32_t cf = count_superset<MW>(false, p, start, lists, 0, n1, F, lane);
-            if (cf >= thr) {
-                has = 1;
-                csup = cf;
-#pragma unroll
-                for (int i = 0; i < MW; ++i) cand.w[i] |= F.w[i];
-            }
-        }
-        if (!has) sort_tail<MW>(F, cnt, lane, S.f, S.c);
-        if (lane < MW) {
-            S.hp[lane] = m_word(Hp, lane);
-            S.cand[lane] = m_word(cand, lane);
-        }
-        if (lane == 0) {
-            S.cand_sup = csup;
-            S.has_cand = has;
-            S.k = has ? 0 : k1;
-            S.overflow = overflow;
-        }
-        __syncwarp();
+        Mask<MW> H = m_load<MW>(R.hp), req = m_load<MW>(R.req);
+        m_set(H, R.f[j]);
+        m_set(req, R.f[j]);
+        const NodeWords<MW> nw(p, p.starts[w], p.lens[w]);
+        count_node<MW>(nw, T, req, 0, 1, cnt, lane);
+        finish_node<MW>(p, nw, H, T, req, R.c[j], p.thrs[w] ? p.thrs[w] : 1, cnt, lane, subs[p.sub_out + si]);
     }
 }
 
@@ -697,8 +622,7 @@ template <int MW> __global__ void __launch_bounds__(128) wtask_kernel(WMineParam
         const uint32_t t = p.task_order[ti];
         const uint32_t w = p.task_win[t];
         const uint32_t child = p.task_child[t];
-        const uint32_t sub = p.task_sub ? p.task_sub[t] : kWholeWindow;
-        const uint32_t gchild = p.task_gchild ? p.task_gchild[t] : kWholeWindow;
+        const uint32_t rec = p.task_rec[t];
         const uint64_t start = p.starts[w];
         const uint32_t n = p.lens[w];
         const uint32_t thr = p.thrs[w] ? p.thrs[w] : 1;
@@ -706,48 +630,29 @@ template <int MW> __global__ void __launch_bounds__(128) wtask_kernel(WMineParam
         uint32_t np = 0;
         uint64_t nodes = 0;
 
-        // the task's first node: the whole window, or child `child` of its root
-        bool ring0 = child == kWholeWindow;
+        // the task's first node: the whole window, or a child of an expanded node
+        const bool ring0 = rec == kWholeWindow && child == kWholeWindow;
         Mask<MW> H = m_zero<MW>(), T = m_zero<MW>();
         uint32_t sup = n, list_n = n;
-        bool done = false;   // a split child that is itself terminal: its one candidate
+        bool done = false;   // an expanded node that is itself terminal: its one candidate
         if (ring0) {
             for (uint32_t e = 0; e < d; ++e) m_set(T, e);
-        } else if (sub == kWholeWindow) {
-            const WRoot<MW> &R = roots[w];
-            const uint32_t k = R.k;
-            for (uint32_t q = child + 1 + lane; q < k; q += 32) m_set(T, R.f[q]);
-            T = warp_or(T);
-            H = m_load<MW>(R.hp);
-            Mask<MW> req = m_zero<MW>();
-            m_set(req, R.f[child]);
-            m_set(H, R.f[child]);
-            sup = R.c[child];
-            list_n = 0;
-            if (m_nz(T)) {
-                list_n = build_child<MW>(true, p, start, lists, 0, n, req, T, 0, lane);
-                if (list_n == 0xffffffffu) status = 1;
-            }
         } else {
-            const WRoot<MW> &S = reinterpret_cast<const WRoot<MW> *>(p.subs)[sub];
-            if (S.overflow) {
-                status = 1;
-            } else if (gchild == kWholeWindow) {
-                if (lane < MW) pool[lane] = S.cand[lane];
-                if (lane == 0) pool_s[0] = S.cand_sup;
+            const WRoot<MW> &R = rec == kWholeWindow ? roots[w] : reinterpret_cast<const WRoot<MW> *>(p.subs)[rec];
+            if (child == kWholeWindow) {
+                if (lane < MW) pool[lane] = R.cand[lane];
+                if (lane == 0) pool_s[0] = R.cand_sup;
                 np = 1;
                 nodes = 1;
                 done = true;
             } else {
-                const uint32_t k1 = S.k;
-                for (uint32_t q = gchild + 1 + lane; q < k1; q += 32) m_set(T, S.f[q]);
+                for (uint32_t q = child + 1 + lane; q < R.k; q += 32) m_set(T, R.f[q]);
                 T = warp_or(T);
-                H = m_load<MW>(S.hp);
-                Mask<MW> req = m_zero<MW>();
-                m_set(req, roots[w].f[child]);
-                m_set(req, S.f[gchild]);
-                m_set(H, S.f[gchild]);
-                sup = S.c[gchild];
+                H = m_load<MW>(R.hp);
+                Mask<MW> req = m_load<MW>(R.req);
+                m_set(req, R.f[child]);
+                m_set(H, R.f[child]);
+                sup = R.c[child];
                 list_n = 0;
                 if (m_nz(T)) {
                     list_n = build_child<MW>(true, p, start, lists, 0, n, req, T, 0, lane);
@@ -924,6 +829,84 @@ template <int MW> __global__ void __launch_bounds__(128) wtask_kernel(WMineParam
     }
 }
 
+namespace {
+
+// Base database of a task: the window's transactions holding every item of req,
+// found through the ring's vertical rows; their places, counted from the
+// transaction the window's first word starts with, at at[0 ..), in no particular
+// order.  Returns how many (at[] has room for the window's length).
+template <int MW>
+__device__ __forceinline__ uint32_t list_base(const NodeWords<MW> &nw, const Mask<MW> &req, uint32_t *at,
+                                              uint32_t lane) {
+    uint32_t cn = 0;
+#pragma unroll 1
+    for (uint64_t b = 0; b < nw.nwd; b += 128) {
+        uint64_t v[4];
+        nw.load(b, req, lane, v);
+        uint32_t mine = 0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) mine += __popcll(v[u]);
+        uint32_t incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t x = __shfl_up_sync(kFull, incl, o);
+            if (lane >= (uint32_t)o) incl += x;
+        }
+        uint32_t to = cn + incl - mine;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const uint32_t at0 = (uint32_t)(b + lane + 32 * u) * 64;
+#pragma unroll 1
+            for (uint64_t x = v[u]; x; x &= x - 1) at[to++] = at0 + (__ffsll((long long)x) - 1);
+        }
+        cn += __shfl_sync(kFull, incl, 31);
+    }
+    __syncwarp();
+    return cn;
+}
+
+// Vertical rows of a database of n0 transactions, by item id: bit i of word c of
+// row e is set when entry 32c+i holds item e (rows of T0's items; vw a multiple of
+// 4).  Four chunks of 32 entries at a time, so a row's words leave as one 16-byte
+// store; the next four chunks' masks are on their way meanwhile.  (Each lane
+// fetching the masks of its own words one by one, twice, took 90 to 330 us a task
+// in a batch, most of the time of the tasks that search a handful of nodes; now 30 to 100 us.)
+template <int MW>
+__device__ __forceinline__ void build_rows(const WMineParams &p, const NodeWords<MW> &nw, const uint32_t *at,
+                                           uint32_t n0, const Mask<MW> &T0, uint32_t *rows, uint32_t vw,
+                                           uint32_t lane) {
+    const uint32_t W = (n0 + 31) / 32;
+    Mask<MW> next[4];
+    auto fetch = [&](uint32_t c) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const uint32_t i = (c + u) * 32 + lane;
+            next[u] = i < n0 ? m_load<MW>(p.hm + (((nw.w0 << 6) + at[i]) & p.cap_mask) * MW) : m_zero<MW>();
+        }
+    };
+    fetch(0);
+#pragma unroll 1
+    for (uint32_t c = 0; c < W; c += 4) {
+        Mask<MW> m[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) m[u] = next[u];
+        if (c + 4 < W) fetch(c + 4);
+#pragma unroll
+        for (int b = 0; b < 2 * MW; ++b) {
+            const uint32_t want = (uint32_t)(T0.w[b >> 1] >> ((b & 1) * 32));
+            if (!want) continue;
+            uint32_t w[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) w[u] = transpose32((uint32_t)(m[u].w[b >> 1] >> ((b & 1) * 32)), lane);
+            if ((want >> lane) & 1u)
+                *reinterpret_cast<uint4 *>(rows + (uint64_t)(b * 32 + lane) * vw + c) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+    }
+    __syncwarp();
+}
+
+}  // namespace
+
 // Resident CTAs per SM the register allocation is fitted to.  Measured with tails as masks on the
 // 4,096 service windows: 6 (80 registers, 3,648 warps) 337 ms, 7 (72 registers,
 // 4,176 warps, the workspace budget's limit) 338 ms with a longer makespan, 8
@@ -940,8 +923,11 @@ template <int MW> __global__ void __launch_bounds__(128) wtask_kernel(WMineParam
 // Bound by instruction issue and by fetching them (tidsets of 16 to 2,048 words:
 // each item's count is a few loads and a reduction).  Item by item with 64-bit
 // masks the node cost 2,000 instructions, now 1,060, and the code is 68 KB instead
-// of 84.  45 windows of 512 to 65,536 transactions (floor 2%): 8.8 -> 6.5 ms, of
-// which the longest task is 6.1 ms; 768 windows: 69 -> 44 ms.
+// of 84.  45 windows of 512 to 65,536 transactions (floor 2%): 8.8 -> 6.5 ms;
+// 768 windows: 69 -> 44 ms.  A child whose head and tail lie in a known MFI ends its
+// parent's loop (2.15 -> 1.50 million nodes for 0.99 million MFIs; 37.1 -> 25.6
+// million for 17.1), and a task may search several children of an expanded node:
+// 6.5 -> 5.8 ms (the longest task; 2.4 ms a warp on average), 44 -> 36 ms.
 template <int MW> __global__ void __launch_bounds__(128, SGFIM_WVTASK_MIN_BLOCKS) wvtask_kernel(WMineParams p) {
     constexpr uint32_t NI = 64 * MW;                        // items
     __shared__ __align__(16) uint32_t s_cnt[4][NI];
@@ -953,7 +939,7 @@ template <int MW> __global__ void __launch_bounds__(128, SGFIM_WVTASK_MIN_BLOCKS
     uint8_t *tail = s_tail[wib], *sorted = s_sort[wib];
     uint32_t *cnt = s_cnt[wib];
     uint64_t *keys = s_key[wib];
-    uint64_t *lists = p.lists + warp * (uint64_t)p.list_cap * MW;
+    uint32_t *at = reinterpret_cast<uint32_t *>(p.lists) + warp * (uint64_t)p.list_cap;
     uint32_t *lmfi = p.lmfi + warp * (uint64_t)p.lmfi_cap;
     uint64_t *pool = p.pool_m + warp * (uint64_t)p.pool_cap * MW;
     uint32_t *pool_s = p.pool_s + warp * (uint64_t)p.pool_cap;
@@ -973,8 +959,8 @@ template <int MW> __global__ void __launch_bounds__(128, SGFIM_WVTASK_MIN_BLOCKS
         const uint32_t t = p.task_order[ti];
         const uint32_t w = p.task_win[t];
         const uint32_t child = p.task_child[t];
-        const uint32_t sub = p.task_sub ? p.task_sub[t] : kWholeWindow;
-        const uint32_t gchild = p.task_gchild ? p.task_gchild[t] : kWholeWindow;
+        const uint32_t rec = p.task_rec[t];
+        const uint32_t n_child = p.task_n_child[t];
         const uint64_t start = p.starts[w];
         const uint32_t n = p.lens[w];
         const uint32_t thr = p.thrs[w] ? p.thrs[w] : 1;
@@ -982,39 +968,48 @@ template <int MW> __global__ void __launch_bounds__(128, SGFIM_WVTASK_MIN_BLOCKS
         uint32_t np = 0;
         uint64_t nodes = 0;
 
-        // the task's first node: the whole window, or a child (grandchild) of its root
+        // the task's first node: the whole window, a child of an expanded node, or (n_child > 1)
+        // an expanded node of whose children this task searches n_child
+        const bool part = n_child > 1;
         Mask<MW> H = m_zero<MW>(), T0 = m_zero<MW>(), req = m_zero<MW>();
         uint32_t sup = n, list_n = n, nt = 0;
-        bool done = false;               // a split child that is itself terminal: its one candidate
+        bool done = false;               // an expanded node that is itself terminal: its one candidate
         const uint8_t *src = nullptr;    // where the first tail is listed (null: all items)
-        if (child == kWholeWindow) {
+        if (rec == kWholeWindow && child == kWholeWindow) {
             nt = d;
-        } else if (sub == kWholeWindow) {
-            const WRoot<MW> &R = roots[w];
-            H = m_load<MW>(R.hp);
-            m_set(req, R.f[child]);
-            m_set(H, R.f[child]);
-            sup = R.c[child];
-            src = R.f + child + 1;
-            nt = R.k - child - 1;
         } else {
-            const WRoot<MW> &S = reinterpret_cast<const WRoot<MW> *>(p.subs)[sub];
-            if (S.overflow) {
-                status = 1;
-            } else if (gchild == kWholeWindow) {
-                if (lane < MW) pool[lane] = S.cand[lane];
-                if (lane == 0) pool_s[0] = S.cand_sup;
+            const WRoot<MW> &R = rec == kWholeWindow ? roots[w] : reinterpret_cast<const WRoot<MW> *>(p.subs)[rec];
+            if (child == kWholeWindow) {
+                if (lane < MW) pool[lane] = R.cand[lane];
+                if (lane == 0) pool_s[0] = R.cand_sup;
                 np = 1;
                 nodes = 1;
                 done = true;
             } else {
-                H = m_load<MW>(S.hp);
-                m_set(req, roots[w].f[child]);
-                m_set(req, S.f[gchild]);
-                m_set(H, S.f[gchild]);
-                sup = S.c[gchild];
-                src = S.f + gchild + 1;
-                nt = S.k - gchild - 1;
+                H = m_load<MW>(R.hp);
+                req = m_load<MW>(R.req);
+                src = R.f + child;
+                nt = R.k - child;
+                if (part) {   // the node is in the record: level 0, children from `child` on
+                    WLevel<MW> &A = LV[0];
+                    if (lane < MW) A.hp[lane] = R.hp[lane];
+                    for (uint32_t i = lane; i < nt; i += 32) {
+                        A.f[i] = src[i];
+                        A.c[i] = R.c[child + i];
+                    }
+                    if (lane == 0) {
+                        A.lm_off = A.lm_n = A.entry = 0;
+                        A.k = nt;
+                        A.end = n_child;
+                        A.j = 0;
+                    }
+                } else {
+                    m_set(req, R.f[child]);
+                    m_set(H, R.f[child]);
+                    sup = R.c[child];
+                    ++src;
+                    --nt;
+                }
             }
         }
 #pragma unroll 1
@@ -1024,11 +1019,12 @@ template <int MW> __global__ void __launch_bounds__(128, SGFIM_WVTASK_MIN_BLOCKS
             m_set(T0, e);
         }
         T0 = warp_or(T0);
-        if (status == 0 && !done) {
+        const NodeWords<MW> nw(p, start, n);
+        if (!done) {
             list_n = 0;
             if (nt) {
-                list_n = build_base<MW>(p, start, n, req, T0, lists, lane);
-                if (list_n == 0xffffffffu) status = 1;
+                if (n > p.list_cap) status = 1;
+                else list_n = list_base<MW>(nw, req, at, lane);
             }
         }
         // ---- the task's database as vertical rows over its entries
@@ -1040,7 +1036,7 @@ template <int MW> __global__ void __launch_bounds__(128, SGFIM_WVTASK_MIN_BLOCKS
             if (((W + 3) & ~3u) > vw) {
                 status = 1;
             } else {
-                build_rows<MW>(lists, list_n, T0, vrows, vw, lane);
+                build_rows<MW>(p, nw, at, list_n, T0, vrows, vw, lane);
 #pragma unroll 1
                 for (uint32_t x = lane; x < W; x += 32) {
                     const uint32_t v = (x + 1 < W || (list_n & 31) == 0) ? 0xffffffffu : ((1u << (list_n & 31)) - 1);
@@ -1054,7 +1050,7 @@ template <int MW> __global__ void __launch_bounds__(128, SGFIM_WVTASK_MIN_BLOCKS
         }
         int l = 0;
         uint32_t lm_off = 0, lm_n = 0, entry = 0;
-        bool expand = true;
+        bool expand = !part;
 
         while (status == 0 && !done) {
             if (expand) {
@@ -1174,7 +1170,7 @@ template <int MW> __global__ void __launch_bounds__(128, SGFIM_WVTASK_MIN_BLOCKS
                     A.lm_off = lm_off;
                     A.lm_n = lm_n;
                     A.entry = entry;
-                    A.k = k;
+                    A.k = A.end = k;
                     A.j = 0;
                 }
                 __syncwarp();
@@ -1182,7 +1178,7 @@ template <int MW> __global__ void __launch_bounds__(128, SGFIM_WVTASK_MIN_BLOCKS
             // ---- next child of level l, or up
             WLevel<MW> &A = LV[l];
             const uint32_t j = A.j, k = A.k;
-            if (j >= k) {
+            if (j >= A.end) {
                 if (l == 0) break;
                 --l;
                 continue;
@@ -1193,29 +1189,21 @@ template <int MW> __global__ void __launch_bounds__(128, SGFIM_WVTASK_MIN_BLOCKS
             const uint32_t csup = A.c[j];
             Mask<MW> Hc = m_load<MW>(A.hp);
             m_set(Hc, e);
-            {
-                // child tidset = parent tidset AND row(e)
-                const uint32_t *ptid = vtid + (uint64_t)l * vw;
-                uint32_t *ctid = vtid + (uint64_t)(l + 1) * vw;
-                const uint32_t *row = vrows + e * vw;
-                if (l + 1 < kWDepth) {
-                    if (small) {
-#pragma unroll
-                        for (uint32_t x = 0; x < kReg; ++x)
-                            if (lane + 32 * x < W) {
-                                tr[x] = ptid[lane + 32 * x] & row[lane + 32 * x];
-                                ctid[lane + 32 * x] = tr[x];
-                            }
-                    } else {
-#pragma unroll 1
-                        for (uint32_t x = lane; x < W; x += 32) ctid[x] = ptid[x] & row[x];
-                    }
-                }
-            }
             nt = k - j - 1;
+            Mask<MW> all = m_zero<MW>();   // the child's head and its whole tail
 #pragma unroll 1
-            for (uint32_t i = lane; i < nt; i += 32) tail[i] = A.f[j + 1 + i];
-            // child local-MFI list: members containing the child's head
+            for (uint32_t i = lane; i < nt; i += 32) {
+                const uint32_t f = A.f[j + 1 + i];
+                tail[i] = (uint8_t)f;
+                m_set(all, f);
+            }
+            if (nt) all = warp_or(all);
+#pragma unroll
+            for (int i = 0; i < MW; ++i) all.w[i] |= Hc.w[i];
+            // child local-MFI list: members containing the child's head.  One that contains its
+            // tail too leaves nothing new below this child, nor below any later one: their heads
+            // and tails are subsets of this one's.
+            bool known = false;
             const uint32_t c_lm = A.lm_off + A.lm_n;
             const uint32_t p_lm_off = A.lm_off, p_lm_n = A.lm_n, p_entry = A.entry;
             const uint32_t n_src = p_lm_n + (np - p_entry);
@@ -1233,7 +1221,11 @@ template <int MW> __global__ void __launch_bounds__(128, SGFIM_WVTASK_MIN_BLOCKS
                 }
 #pragma unroll
                 for (int u = 0; u < kU; ++u)
-                    if (b + u * 32 + lane < n_src) keep[u] = m_sub(Hc, m_load<MW>(pool + (uint64_t)idx[u] * MW));
+                    if (b + u * 32 + lane < n_src) {
+                        const Mask<MW> m = m_load<MW>(pool + (uint64_t)idx[u] * MW);
+                        keep[u] = m_sub(Hc, m);
+                        known |= m_sub(all, m);
+                    }
                 // the child's list goes after the parent's: writes never touch indices still to be read
 #pragma unroll
                 for (int u = 0; u < kU; ++u) {
@@ -1243,8 +1235,40 @@ template <int MW> __global__ void __launch_bounds__(128, SGFIM_WVTASK_MIN_BLOCKS
                     ln += __popc(bal);
                 }
             }
+            if (__any_sync(kFull, known)) {
+                if (l == 0) break;
+                --l;
+                __syncwarp();
+                continue;
+            }
+            if (nt == 0) {   // the last child, alone: a candidate
+                ++nodes;
+                if (np >= p.pool_cap) { status = 1; break; }
+                if (lane < MW) pool[(uint64_t)np * MW + lane] = m_word(Hc, lane);
+                if (lane == 0) pool_s[np] = csup;
+                ++np;
+                __syncwarp();
+                continue;
+            }
             if ((uint64_t)c_lm + ln > p.lmfi_cap) { status = 1; break; }
             if (l + 1 >= kWDepth) { status = 1; break; }
+            {
+                // child tidset = parent tidset AND row(e)
+                const uint32_t *ptid = vtid + (uint64_t)l * vw;
+                uint32_t *ctid = vtid + (uint64_t)(l + 1) * vw;
+                const uint32_t *row = vrows + e * vw;
+                if (small) {
+#pragma unroll
+                    for (uint32_t x = 0; x < kReg; ++x)
+                        if (lane + 32 * x < W) {
+                            tr[x] = ptid[lane + 32 * x] & row[lane + 32 * x];
+                            ctid[lane + 32 * x] = tr[x];
+                        }
+                } else {
+#pragma unroll 1
+                    for (uint32_t x = lane; x < W; x += 32) ctid[x] = ptid[x] & row[x];
+                }
+            }
             __syncwarp();
             ++l;
             H = Hc;
@@ -1423,7 +1447,7 @@ size_t wmine_root_bytes(int mw) { return mw == 2 ? sizeof(WRoot<2>) : 0; }
 
 void launch_wroot(const WMineParams &p, int mw, unsigned blocks, cudaStream_t st) {
     if (mw != 2) throw CudaError(cudaErrorInvalidValue, "batched window miner supports 2 mask words", __FILE__, __LINE__);
-    wroot_kernel<2><<<blocks, 128, 0, st>>>(p);
+    wroot_kernel<2><<<blocks, kRootThreads, 0, st>>>(p);
     SG_CUDA_TRY(cudaGetLastError());
 }
 void launch_wsub(const WMineParams &p, int mw, unsigned blocks, cudaStream_t st) {

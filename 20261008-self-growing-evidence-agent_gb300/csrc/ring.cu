@@ -372,24 +372,25 @@ int sgfim_ring_mine_windows(sgfim_ring *r, sgfim_handle *h, const uint64_t *star
                 max_len = std::max(max_len, lens[w]);
                 if (lens[w] >= kSplitMin) split.push_back((uint32_t)w);
             }
-            // the vertical search keeps only the task's base database as entries; the horizontal
-            // one stacks every level's database
+            // the vertical search lists the task's transactions (4 bytes each); the horizontal one
+            // stacks every level's database as masks
             const bool vertical = !(h->flags & SGFIM_F_WINDOWS_HORIZONTAL);
             const uint64_t list_cap = std::min<uint64_t>(
-                std::max<uint64_t>(8192, (vertical ? 1 : 2) * max_len + 1024), 1ull << 30);
+                std::max<uint64_t>(8192, (vertical ? 1 : 2) * max_len + 1024) & ~3ull, 1ull << 30);
+            const size_t list_b = vertical ? 4 : mw * 8;
             const uint64_t lmfi_cap = 1u << 16, pool_cap = 1u << 16;
             const uint64_t v_words = vertical ? ((max_len + 31) / 32 + 1 + 3) & ~3ull : 0;   // whole 16-byte pieces
             const size_t v_bytes = (size_t)(128 + wmine_depth()) * v_words * 4;
             const size_t per_warp =
-                list_cap * mw * 8 + lmfi_cap * 4 + pool_cap * (mw * 8 + 4) + wmine_level_bytes(mw) + v_bytes;
+                list_cap * list_b + lmfi_cap * 4 + pool_cap * (mw * 8 + 4) + wmine_level_bytes(mw) + v_bytes;
             uint64_t warps = (uint64_t)h->n_sm * 4 * (uint64_t)wtask_blocks_per_sm(vertical);
             warps = std::min<uint64_t>(warps, std::max<uint64_t>(4, (h->hbm_budget / 2) / per_warp));
             warps = std::max<uint64_t>(4, warps & ~3ull);
             const size_t cand_bytes = mw * 8 + 4 + 1;
             const uint64_t out_cap = std::max<uint64_t>(
-                1u << 20, std::min<uint64_t>(n_windows * 65536, (h->hbm_budget / 4) / cand_bytes));
+                1u << 20, std::min<uint64_t>(n_windows << 17, (h->hbm_budget / 4) / cand_bytes));
             const size_t root_b = wmine_root_bytes(mw);
-            ws.lists.reserve(warps * list_cap * mw * 8, st);
+            ws.lists.reserve(warps * list_cap * list_b, st);
             ws.lmfi.reserve(warps * lmfi_cap * 4, st);
             ws.pool_m.reserve(warps * pool_cap * mw * 8, st);
             ws.pool_s.reserve(warps * pool_cap * 4, st);
@@ -459,8 +460,8 @@ int sgfim_ring_mine_windows(sgfim_ring *r, sgfim_handle *h, const uint64_t *star
             p.out_m = ws.out_m.as<uint64_t>();
             p.out_s = ws.out_s.as<uint32_t>();
             p.out_cap = out_cap;
-            // record fields read here (WRoot<2>: hp[2], cand[2], cand_sup, has_cand, k, overflow, f[128], c[128])
-            const size_t o_cand = 16, o_csup = 32, o_has = 36, o_k = 40, o_ovf = 44, o_f = 48, o_c = 176;
+            // record fields read here (WRoot<2>: hp[2], cand[2], cand_sup, has_cand, k, pad, f[128], c[128])
+            const size_t o_cand = 16, o_csup = 32, o_has = 36, o_k = 40, o_c = 176;
             auto u32_at = [](const unsigned char *rec, size_t off) {
                 uint32_t v;
                 memcpy(&v, rec + off, 4);
@@ -470,7 +471,7 @@ int sgfim_ring_mine_windows(sgfim_ring *r, sgfim_handle *h, const uint64_t *star
             std::vector<unsigned char> roots_h;
             if (!split.empty()) {
                 SG_CUDA_TRY(cudaEventRecord(k0, st));
-                launch_wroot(p, (int)mw, (unsigned)std::min<uint64_t>((split.size() + 3) / 4, (uint64_t)h->n_sm * 8),
+                launch_wroot(p, (int)mw, (unsigned)std::min<uint64_t>(split.size(), (uint64_t)h->n_sm * 8),
                              st);
                 SG_CUDA_TRY(cudaEventRecord(k1, st));
                 ++launches;
@@ -481,59 +482,120 @@ int sgfim_ring_mine_windows(sgfim_ring *r, sgfim_handle *h, const uint64_t *star
                 kernel_ms += timed_ms();
             }
             auto root_at = [&](uint64_t w) { return roots_h.data() + (size_t)w * root_b; };
-            // cost estimate of a subtree: its database size plus a fixed per-node share, per tail item
-            auto child_cost = [](uint32_t sup, uint32_t tail) { return ((double)sup + 512.0) * (double)tail; };
+            // Cost estimates in us, fitted to the task times of batches of 45 and 768 windows (mean nodes
+            // by tail and by the support as a multiple of the floor, r: 1.4 at r = 1.2, 21 at 2.5, 50 at
+            // 3.5, 220 at 5, 450 at 7.5 and above, whatever the window's length).  A node takes 2.2 us
+            // and 0.8 us per 1,000 transactions of its task, building a task's database 20 us and more.
+            auto est_nodes = [](uint32_t sup, uint32_t tail, uint32_t thr) {
+                const double q = (double)sup / (double)thr;
+                return 1.0 + std::min(1.2 * q * q * q, 10.0 * (double)tail);
+            };
+            auto node_us = [](uint32_t n_txn) { return 2.2 + 0.0008 * (double)n_txn; };
+            auto build_us = [](uint32_t n_txn, uint32_t n_window) {
+                return 20.0 + 0.006 * (double)n_txn + 0.0004 * (double)n_window;
+            };
+            auto child_cost = [&](uint32_t sup, uint32_t tail, uint32_t thr) {
+                return est_nodes(sup, tail, thr) * node_us(sup);
+            };
+            auto window_cost = [&](uint64_t w) { return child_cost((uint32_t)lens[w], r->d, t_thr[w]); };
             std::vector<uint8_t> is_split(n_windows, 0), bad(n_windows, 0);
             for (uint32_t w : split) is_split[w] = 1;
-            // ---- 2. the costliest root children are split again (their own expansion in wsub_kernel)
+            // ---- 2. the costliest children are expanded in turn (wsub_kernel), level by level
             double total_cost = 0.0;
             for (uint64_t w = 0; w < n_windows; ++w) {
                 if (!is_split[w]) {
-                    total_cost += 1300.0 * (double)lens[w];
+                    total_cost += window_cost(w);
                     continue;
                 }
                 const unsigned char *R = root_at(w);
                 const uint32_t k = u32_at(R, o_has) ? 0 : u32_at(R, o_k);
-                for (uint32_t j = 0; j < k; ++j) total_cost += child_cost(u32_at(R, o_c + 4 * j), k - j);
+                for (uint32_t j = 0; j < k; ++j) total_cost += child_cost(u32_at(R, o_c + 4 * j), k - j, t_thr[w]);
             }
-            const double split_above = total_cost / (double)(warps * 2);
-            std::vector<uint32_t> sub_win, sub_child;
-            std::vector<uint32_t> sub_of_first(n_windows, 0);   // first sub index of each split window
-            for (uint32_t w : split) {
-                sub_of_first[w] = (uint32_t)sub_win.size();
-                const unsigned char *R = root_at(w);
-                if (u32_at(R, o_has)) continue;
-                const uint32_t k = u32_at(R, o_k);
-                for (uint32_t j = 0; j + 2 < k; ++j)
-                    if (child_cost(u32_at(R, o_c + 4 * j), k - j) > split_above) {
-                        sub_win.push_back(w);
-                        sub_child.push_back(j);
+            // Levels below the roots (a task's base database is found with three rows at most).  Subtrees
+            // that share no pool repeat candidates, at floors of a few transactions most of them (4,096
+            // transactions at floor 1: 0.2 million with one level, 0.9 with two): a second level only up
+            // to 32 times the floor, and not in the horizontal search, which cannot put neighbours into
+            // one task.
+            const int kLevels = vertical ? 2 : 1;
+            // A node is expanded when it is estimated above a warp's share.  Batch of 45 windows, tasks
+            // (12,000 / 24,000 / 51,000) at 2, 1 and 1/4 of it: 10.9 / 10.4 / 11.8 ms a call (task
+            // kernel 6.5 / 5.8 / 5.0; building more databases and the host's lists cost the rest).
+            const double split_above = total_cost / (double)warps;
+            std::vector<uint32_t> sub_win, sub_parent, sub_child;   // the records of all levels
+            // first record expanded from a node's children (children ascending): by window, by record
+            std::vector<uint32_t> first_of_root(n_windows, 0), first_of_sub;
+            uint32_t lvl_lo = 0;   // first record of the level above
+            uint32_t lvl2 = 0xffffffffu;   // first record of the second level
+            auto sub_at = [&](uint32_t i) {
+                return i < lvl2 ? ws.h_sub[0].as<unsigned char>() + (size_t)i * root_b
+                                : ws.h_sub[1].as<unsigned char>() + (size_t)(i - lvl2) * root_b;
+            };
+            for (int lvl = 0; lvl < kLevels; ++lvl) {
+                const uint32_t out0 = (uint32_t)sub_win.size();
+                auto expand_children = [&](uint32_t w, uint32_t parent, const unsigned char *R) {
+                    if (u32_at(R, o_has)) return;
+                    const uint32_t k = u32_at(R, o_k);
+                    for (uint32_t j = 0; j + 2 < k; ++j)
+                        if ((lvl == 0 || u32_at(R, o_c + 4 * j) <= 32ull * t_thr[w]) &&
+                            child_cost(u32_at(R, o_c + 4 * j), k - j, t_thr[w]) > split_above) {
+                            sub_win.push_back(w);
+                            sub_parent.push_back(parent);
+                            sub_child.push_back(j);
+                        }
+                };
+                if (lvl == 0) {
+                    for (uint32_t w : split) {
+                        first_of_root[w] = (uint32_t)sub_win.size();
+                        expand_children(w, w, root_at(w));
                     }
-            }
-            std::vector<unsigned char> subs_h;
-            if (!sub_win.empty()) {
-                const size_t ns = sub_win.size();
-                ws.sub.reserve(ns * root_b + ns * 8 + 256, st);
-                uint32_t *d_sw = reinterpret_cast<uint32_t *>(ws.sub.as<char>() + ((ns * root_b + 255) & ~(size_t)255));
-                std::vector<uint32_t> sw(sub_win);
-                sw.insert(sw.end(), sub_child.begin(), sub_child.end());
-                SG_CUDA_TRY(cudaMemcpyAsync(d_sw, sw.data(), sw.size() * 4, cudaMemcpyHostToDevice, st));
+                } else {
+                    for (uint32_t i = lvl_lo; i < out0; ++i) {
+                        first_of_sub[i] = (uint32_t)sub_win.size();
+                        expand_children(sub_win[i], i, sub_at(i));
+                    }
+                }
+                const size_t all = sub_win.size(), ns = all - out0;
+                first_of_sub.resize(all, (uint32_t)all);
+                if (ns == 0) break;
+                // records, then this level's lists
+                const size_t rec_b = (all * root_b + 255) & ~(size_t)255;
+                if (ws.sub.bytes < rec_b + 3 * ns * 4) {   // keep the level above
+                    DevBuf bigger;
+                    bigger.reserve(rec_b * 4 + 3 * ns * 4, st);
+                    if (out0)
+                        SG_CUDA_TRY(cudaMemcpyAsync(bigger.ptr, ws.sub.ptr, out0 * root_b, cudaMemcpyDeviceToDevice, st));
+                    h->sync();
+                    ws.sub.release();
+                    ws.sub = bigger;
+                }
+                uint32_t *d_list = reinterpret_cast<uint32_t *>(ws.sub.as<char>() + rec_b);
+                std::vector<uint32_t> list(sub_win.begin() + out0, sub_win.end());
+                list.insert(list.end(), sub_parent.begin() + out0, sub_parent.end());
+                list.insert(list.end(), sub_child.begin() + out0, sub_child.end());
+                SG_CUDA_TRY(cudaMemcpyAsync(d_list, list.data(), list.size() * 4, cudaMemcpyHostToDevice, st));
                 p.subs = ws.sub.ptr;
-                p.sub_win = d_sw;
-                p.sub_child = d_sw + ns;
+                p.sub_parents = lvl == 0 ? ws.res.ptr : ws.sub.ptr;
+                p.sub_win = d_list;
+                p.sub_parent = d_list + ns;
+                p.sub_child = d_list + 2 * ns;
+                p.sub_next = ws.ctrl.as<uint32_t>() + 2 + lvl;
                 p.n_sub = (uint32_t)ns;
+                p.sub_out = out0;
                 SG_CUDA_TRY(cudaEventRecord(k0, st));
-                launch_wsub(p, (int)mw, (unsigned)(std::min<uint64_t>(warps, (ns + 3) & ~3ull) / 4), st);
+                launch_wsub(p, (int)mw, (unsigned)(std::min<uint64_t>((uint64_t)h->n_sm * 64, (ns + 3) & ~3ull) / 4), st);
                 SG_CUDA_TRY(cudaEventRecord(k1, st));
                 ++launches;
                 ++h->launches;
-                subs_h.resize(ns * root_b);
-                SG_CUDA_TRY(cudaMemcpyAsync(subs_h.data(), ws.sub.ptr, ns * root_b, cudaMemcpyDeviceToHost, st));
+                ws.h_sub[lvl].reserve(ns * root_b);
+                if (lvl == 1) lvl2 = out0;
+                SG_CUDA_TRY(cudaMemcpyAsync(ws.h_sub[lvl].ptr, ws.sub.as<char>() + out0 * root_b, ns * root_b,
+                                            cudaMemcpyDeviceToHost, st));
                 h->sync();
                 kernel_ms += timed_ms();
+                lvl_lo = out0;
             }
             // ---- 3. tasks in depth-first order within each window
-            std::vector<uint32_t> t_win, t_child, t_sub, t_gchild;
+            std::vector<uint32_t> t_win, t_child, t_rec, t_n_child;
             std::vector<double> t_cost;
             {
                 size_t est = n_windows;
@@ -541,23 +603,71 @@ int sgfim_ring_mine_windows(sgfim_ring *r, sgfim_handle *h, const uint64_t *star
                     const unsigned char *R = root_at(w);
                     if (!u32_at(R, o_has)) est += u32_at(R, o_k);
                 }
-                for (size_t i = 0; i < sub_win.size(); ++i) est += u32_at(subs_h.data() + i * root_b, o_k);
+                for (size_t i = 0; i < sub_win.size(); ++i) est += u32_at(sub_at((uint32_t)i), o_k);
                 t_win.reserve(est);
                 t_child.reserve(est);
-                t_sub.reserve(est);
-                t_gchild.reserve(est);
+                t_rec.reserve(est);
+                t_n_child.reserve(est);
                 t_cost.reserve(est);
             }
-            auto add_task = [&](uint32_t w, uint32_t c, uint32_t sb, uint32_t g, double cost) {
+            auto add_task = [&](uint32_t w, uint32_t rec, uint32_t c, double cost, uint32_t n_child = 1) {
                 t_win.push_back(w);
+                t_rec.push_back(rec);
                 t_child.push_back(c);
-                t_sub.push_back(sb);
-                t_gchild.push_back(g);
+                t_n_child.push_back(n_child);
                 t_cost.push_back(cost);
+            };
+            // The children of an expanded node: tasks, or where a child is expanded itself its children.
+            // A task of its own costs a child the building of its database, but its nodes then run over
+            // its transactions alone; neighbours with few nodes share a task over their parent's.
+            auto add_children = [&](auto &self, uint32_t w, uint32_t rec, const unsigned char *R, uint32_t psup,
+                                    uint32_t si) -> void {
+                const uint32_t k = u32_at(R, o_k), n = (uint32_t)lens[w];
+                const uint32_t parent = rec == kWholeWindow ? w : rec;
+                uint32_t run = 0;        // neighbours before child j that would share a task
+                double run_shared = 0.0, run_alone = 0.0;
+                auto end_run = [&](uint32_t j) {
+                    const double shared = run_shared + build_us(psup, n);
+                    if (run > 1 && shared <= run_alone) {
+                        add_task(w, rec, j - run, shared, run);
+                    } else {
+                        for (uint32_t i = j - run; i < j; ++i) {
+                            const uint32_t sup = u32_at(R, o_c + 4 * i);
+                            add_task(w, rec, i, child_cost(sup, k - i, t_thr[w]) + build_us(sup, n));
+                        }
+                    }
+                    run = 0;
+                    run_shared = run_alone = 0.0;
+                };
+                for (uint32_t j = 0; j < k; ++j) {
+                    const bool expanded = si < sub_win.size() && sub_win[si] == w && sub_parent[si] == parent &&
+                                          sub_child[si] == j;
+                    const uint32_t sup = u32_at(R, o_c + 4 * j);
+                    if (!expanded) {
+                        const double alone = child_cost(sup, k - j, t_thr[w]) + build_us(sup, n);
+                        const double shared = est_nodes(sup, k - j, t_thr[w]) * node_us(psup);
+                        if (!vertical || shared > alone) {
+                            end_run(j);
+                            add_task(w, rec, j, alone);
+                            continue;
+                        }
+                        if (run_shared + shared > split_above) end_run(j);
+                        ++run;
+                        run_shared += shared;
+                        run_alone += alone;
+                        continue;
+                    }
+                    end_run(j);
+                    const unsigned char *S = sub_at(si);
+                    if (u32_at(S, o_has)) add_task(w, si, kWholeWindow, 1.0);
+                    else self(self, w, si, S, sup, first_of_sub[si]);
+                    ++si;
+                }
+                end_run(k);
             };
             for (uint64_t w = 0; w < n_windows; ++w) {
                 if (!is_split[w]) {
-                    add_task((uint32_t)w, kWholeWindow, kWholeWindow, kWholeWindow, 1300.0 * (double)lens[w]);
+                    add_task((uint32_t)w, kWholeWindow, kWholeWindow, window_cost(w));
                     continue;
                 }
                 const unsigned char *R = root_at(w);
@@ -570,27 +680,8 @@ int sgfim_ring_mine_windows(sgfim_ring *r, sgfim_handle *h, const uint64_t *star
                     root_cand_sup.push_back(u32_at(R, o_csup));
                     continue;
                 }
-                const uint32_t k = u32_at(R, o_k);
-                uint32_t si = sub_of_first[w];
-                for (uint32_t j = 0; j < k; ++j) {
-                    if (si < sub_win.size() && sub_win[si] == w && sub_child[si] == j) {
-                        const unsigned char *S = subs_h.data() + (size_t)si * root_b;
-                        if (u32_at(S, o_ovf)) {
-                            bad[w] = 1;
-                        } else if (u32_at(S, o_has)) {
-                            add_task((uint32_t)w, j, si, kWholeWindow, 1.0);
-                        } else {
-                            const uint32_t k1 = u32_at(S, o_k);
-                            for (uint32_t g = 0; g < k1; ++g)
-                                add_task((uint32_t)w, j, si, g, child_cost(u32_at(S, o_c + 4 * g), k1 - g));
-                        }
-                        ++si;
-                    } else {
-                        add_task((uint32_t)w, j, kWholeWindow, kWholeWindow, child_cost(u32_at(R, o_c + 4 * j), k - j));
-                    }
-                }
+                add_children(add_children, (uint32_t)w, kWholeWindow, R, (uint32_t)lens[w], first_of_root[w]);
             }
-            (void)o_f;
             const uint64_t nt = t_win.size();
             n_tasks_total = nt;
             std::vector<uint32_t> order(nt);
@@ -609,15 +700,15 @@ int sgfim_ring_mine_windows(sgfim_ring *r, sgfim_handle *h, const uint64_t *star
                 for (int b = 0; b < 128; ++b) cnt[b + 1] += cnt[b];
                 for (uint64_t i = 0; i < nt; ++i) order[cnt[bucket[i]]++] = (uint32_t)i;
             }
-            // task arrays: win | child | sub | gchild | order | cnt | kept | status (u32) | off | nodes (u64)
+            // task arrays: win | rec | child | n_child | order | cnt | kept | status (u32) | off | nodes | ns (u64)
             const size_t nt1 = std::max<uint64_t>(nt, 1);
             const size_t u32_bytes = (8 * 4 * nt1 + 15) & ~(size_t)15;
             ws.tasks.reserve(u32_bytes + 3 * 8 * nt1, st);
             uint32_t *dt_win = ws.tasks.as<uint32_t>();
-            uint32_t *dt_child = dt_win + nt1;
-            uint32_t *dt_sub = dt_child + nt1;
-            uint32_t *dt_gchild = dt_sub + nt1;
-            uint32_t *dt_order = dt_gchild + nt1;
+            uint32_t *dt_rec = dt_win + nt1;
+            uint32_t *dt_child = dt_rec + nt1;
+            uint32_t *dt_n_child = dt_child + nt1;
+            uint32_t *dt_order = dt_n_child + nt1;
             uint32_t *dt_cnt = dt_order + nt1;
             uint32_t *dt_kept = dt_cnt + nt1;
             int32_t *dt_status = reinterpret_cast<int32_t *>(dt_kept + nt1);
@@ -630,15 +721,15 @@ int sgfim_ring_mine_windows(sgfim_ring *r, sgfim_handle *h, const uint64_t *star
                 ws.h_res.reserve(5 * nt1 * 4);
                 uint32_t *hw = ws.h_res.as<uint32_t>();
                 memcpy(hw, t_win.data(), nt * 4);
-                memcpy(hw + nt1, t_child.data(), nt * 4);
-                memcpy(hw + 2 * nt1, t_sub.data(), nt * 4);
-                memcpy(hw + 3 * nt1, t_gchild.data(), nt * 4);
+                memcpy(hw + nt1, t_rec.data(), nt * 4);
+                memcpy(hw + 2 * nt1, t_child.data(), nt * 4);
+                memcpy(hw + 3 * nt1, t_n_child.data(), nt * 4);
                 memcpy(hw + 4 * nt1, order.data(), nt * 4);
                 SG_CUDA_TRY(cudaMemcpyAsync(dt_win, hw, 5 * nt1 * 4, cudaMemcpyHostToDevice, st));
                 p.task_win = dt_win;
+                p.task_rec = dt_rec;
                 p.task_child = dt_child;
-                p.task_sub = dt_sub;
-                p.task_gchild = dt_gchild;
+                p.task_n_child = dt_n_child;
                 p.task_order = dt_order;
                 p.n_tasks = (uint32_t)nt;
                 p.task_off = dt_off;
