@@ -238,10 +238,11 @@ struct WFilterParams {
     uint32_t *task_kept = nullptr;      // in: task_cnt; out: kept
     const uint64_t *out_m = nullptr;
     uint8_t *keep = nullptr;            // per arena slot (in: 1)
-    uint64_t *scratch = nullptr;        // per CTA scratch_words words
-    uint64_t scratch_words = 0;
-    int32_t *win_status = nullptr;      // per split window: 1 = scratch too small
-    uint32_t *next = nullptr;
+    uint64_t *scratch = nullptr;        // the windows' bitmaps: d rows of ceil(total / 64) words each
+    const uint64_t *win_row0 = nullptr; // first word of each window's bitmap
+    uint32_t *win_stats = nullptr;      // per window and item: candidates, ~first word, last word (in: zero)
+    const uint32_t *win_unit0 = nullptr;   // first unit (wfilter_unit() candidates) of each window
+    uint32_t n_units = 0;
 };
 struct WGatherParams {
     uint64_t n_tasks = 0;
@@ -256,11 +257,12 @@ struct WGatherParams {
 };
 size_t wmine_level_bytes(int mw);
 size_t wmine_root_bytes(int mw);
-// blocks of 128 threads (4 warps; wroot: 256; wfilter: 256 or 1,024 threads)
+// blocks of 128 threads (4 warps; wroot and wfilter: 256)
 void launch_wroot(const WMineParams &p, int mw, unsigned blocks, cudaStream_t st);
 void launch_wsub(const WMineParams &p, int mw, unsigned blocks, cudaStream_t st);
 void launch_wtask(const WMineParams &p, int mw, unsigned blocks, cudaStream_t st);
-void launch_wfilter(const WFilterParams &p, int mw, unsigned blocks, unsigned threads, cudaStream_t st);
+void launch_wfilter(const WFilterParams &p, int mw, unsigned blocks, cudaStream_t st);
+int wfilter_unit();
 void launch_wgather(const WGatherParams &p, int mw, unsigned blocks, cudaStream_t st);
 
 }  // namespace sg

@@ -36,13 +36,6 @@ struct sgfim_ring {
     std::string err;
 };
 
-// CTAs per SM of the cross-subtree filter (each holds one window's candidate
-// rows in its own scratch).  On the 4,096 service windows, largest first: 2 per
-// SM 59 ms, 4 per SM 46.5 ms, 8 per SM 45.4 ms.
-#ifndef SGFIM_WFILTER_CTAS_PER_SM
-#define SGFIM_WFILTER_CTAS_PER_SM 8
-#endif
-constexpr uint64_t kFilterCtasPerSm = SGFIM_WFILTER_CTAS_PER_SM;
 // results up to this size leave the device through a pinned staging buffer
 constexpr size_t kStageOutMax = 64ull << 20;
 
@@ -807,59 +800,76 @@ int sgfim_ring_mine_windows(sgfim_ring *r, sgfim_handle *h, const uint64_t *star
                     d_keep = keep;
                     SG_CUDA_TRY(cudaMemsetAsync(keep, 1, used, st));
                     SG_CUDA_TRY(cudaMemcpyAsync(dt_kept, dt_cnt, nt * 4, cudaMemcpyDeviceToDevice, st));
-                    const uint64_t W = (max_m + 63) / 64;
-                    const uint64_t scratch_words = std::max<uint64_t>(W * r->d, 64);
-                    const uint64_t ctas = std::min<uint64_t>(
-                        fwin.size(), std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)h->n_sm * kFilterCtasPerSm,
-                                                                              (h->hbm_budget / 8) / (scratch_words * 8))));
-                    // tables: first u64 | total u64 | task0 u32 | task_of u32 | status i32, then the scratch
-                    const size_t tab =
-                        ((first.size() + wtotal.size()) * 8 + (task0.size() + task_of.size() + fwin.size()) * 4 + 255) &
-                        ~(size_t)255;
-                    ws.lists.reserve(tab + ctas * scratch_words * 8, st);
-                    char *fb = ws.lists.as<char>();
-                    uint64_t *d_first = reinterpret_cast<uint64_t *>(fb);
-                    uint64_t *d_total = d_first + first.size();
-                    uint32_t *d_task0 = reinterpret_cast<uint32_t *>(d_total + wtotal.size());
-                    uint32_t *d_task_of = d_task0 + task0.size();
-                    int32_t *d_wstat = reinterpret_cast<int32_t *>(d_task_of + task_of.size());
+                    // rounds of as many windows as the bitmaps' share of the budget holds
+                    std::vector<uint64_t> row0(fwin.size());
+                    std::vector<uint32_t> unit0(fwin.size()), round0;
+                    const uint64_t round_words =
+                        std::max<uint64_t>((max_m + 63) / 64 * r->d, (h->hbm_budget / 8) / 8);
+                    uint64_t words_used = 0, units = 0, scratch_words = 0;
+                    std::vector<uint32_t> round_units;
+                    for (size_t i = 0; i < fwin.size(); ++i) {
+                        const uint64_t need = (wtotal[i] + 63) / 64 * r->d;
+                        if (i == 0 || words_used + need > round_words) {
+                            if (i) round_units.push_back((uint32_t)units);
+                            round0.push_back((uint32_t)i);
+                            words_used = units = 0;
+                        }
+                        row0[i] = words_used;
+                        unit0[i] = (uint32_t)units;
+                        words_used += need;
+                        units += (wtotal[i] + wfilter_unit() - 1) / wfilter_unit();
+                        scratch_words = std::max(scratch_words, words_used);
+                    }
+                    round_units.push_back((uint32_t)units);
+                    round0.push_back((uint32_t)fwin.size());
+                    // tables: first | total | row0 u64, task0 | task_of | unit0 | stats u32, then the bitmaps
                     std::vector<uint64_t> t64(first);
                     t64.insert(t64.end(), wtotal.begin(), wtotal.end());
+                    t64.insert(t64.end(), row0.begin(), row0.end());
                     std::vector<uint32_t> t32(task0);
                     t32.insert(t32.end(), task_of.begin(), task_of.end());
+                    t32.insert(t32.end(), unit0.begin(), unit0.end());
+                    const size_t stats_b = fwin.size() * 3 * 64 * mw * 4;
+                    const size_t tab = (t64.size() * 8 + t32.size() * 4 + stats_b + 255) & ~(size_t)255;
+                    ws.lists.reserve(tab + std::max<uint64_t>(scratch_words, 1) * 8, st);
+                    char *fb = ws.lists.as<char>();
+                    uint64_t *d_first = reinterpret_cast<uint64_t *>(fb);
+                    uint64_t *d_total = d_first + first.size(), *d_row0 = d_total + wtotal.size();
+                    uint32_t *d_task0 = reinterpret_cast<uint32_t *>(d_row0 + row0.size());
+                    uint32_t *d_task_of = d_task0 + task0.size(), *d_unit0 = d_task_of + task_of.size();
+                    uint32_t *d_stats = d_unit0 + unit0.size();
                     SG_CUDA_TRY(cudaMemcpyAsync(d_first, t64.data(), t64.size() * 8, cudaMemcpyHostToDevice, st));
                     SG_CUDA_TRY(cudaMemcpyAsync(d_task0, t32.data(), t32.size() * 4, cudaMemcpyHostToDevice, st));
-                    SG_CUDA_TRY(cudaMemsetAsync(d_wstat, 0, fwin.size() * 4, st));
-                    WFilterParams fp;
-                    fp.d = r->d;
-                    fp.n_win = (uint32_t)fwin.size();
-                    fp.win_task0 = d_task0;
-                    fp.task_of = d_task_of;
-                    fp.task_first = d_first;
-                    fp.win_total = d_total;
-                    fp.task_off = dt_off;
-                    fp.task_cnt = dt_cnt;
-                    fp.task_kept = dt_kept;
-                    fp.out_m = p.out_m;
-                    fp.keep = keep;
-                    fp.scratch = reinterpret_cast<uint64_t *>(fb + tab);
-                    fp.scratch_words = scratch_words;
-                    fp.win_status = d_wstat;
-                    fp.next = ws.ctrl.as<uint32_t>() + 8;
+                    SG_CUDA_TRY(cudaMemsetAsync(d_stats, 0, stats_b, st));
                     SG_CUDA_TRY(cudaEventRecord(k0, st));
-                    // few windows (a service batch): 1,024 threads per window's CTA, so the
-                    // largest window's candidates are scanned four times as wide
-                    launch_wfilter(fp, (int)mw, (unsigned)ctas, fwin.size() <= (size_t)h->n_sm * 2 ? 1024u : 256u, st);
+                    for (size_t ro = 0; ro + 1 < round0.size(); ++ro) {
+                        const uint32_t i0 = round0[ro];
+                        if (round_units[ro] == 0) continue;
+                        WFilterParams fp;
+                        fp.d = r->d;
+                        fp.n_win = round0[ro + 1] - i0;
+                        fp.win_task0 = d_task0 + i0;
+                        fp.task_of = d_task_of;
+                        fp.task_first = d_first;
+                        fp.win_total = d_total + i0;
+                        fp.task_off = dt_off;
+                        fp.task_cnt = dt_cnt;
+                        fp.task_kept = dt_kept;
+                        fp.out_m = p.out_m;
+                        fp.keep = keep;
+                        fp.scratch = reinterpret_cast<uint64_t *>(fb + tab);
+                        fp.win_row0 = d_row0 + i0;
+                        fp.win_stats = d_stats + (size_t)i0 * 3 * 64 * mw;
+                        fp.win_unit0 = d_unit0 + i0;
+                        fp.n_units = round_units[ro];
+                        launch_wfilter(fp, (int)mw, std::min(round_units[ro], (unsigned)h->n_sm * 8u), st);
+                        launches += 2;
+                        h->launches += 2;
+                    }
                     SG_CUDA_TRY(cudaEventRecord(k1, st));
-                    ++launches;
-                    ++h->launches;
-                    std::vector<int32_t> wstat(fwin.size());
                     SG_CUDA_TRY(cudaMemcpyAsync(kept.data(), dt_kept, nt * 4, cudaMemcpyDeviceToHost, st));
-                    SG_CUDA_TRY(cudaMemcpyAsync(wstat.data(), d_wstat, fwin.size() * 4, cudaMemcpyDeviceToHost, st));
                     h->sync();
                     kernel_ms += timed_ms();
-                    for (size_t i = 0; i < fwin.size(); ++i)
-                        if (wstat[i]) bad[fwin[i]] = 1;
                 }
                 t_win_of.assign(t_win.begin(), t_win.end());
                 for (uint64_t t = 0; t < nt; ++t)
