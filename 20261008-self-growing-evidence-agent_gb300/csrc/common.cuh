@@ -163,4 +163,20 @@ __device__ __forceinline__ uint32_t warp_sum(uint32_t v) {
     return v;
 }
 
+// 32 x 32 bit transpose over the warp: lane i ends with bit i of every lane's word.
+__device__ __forceinline__ uint32_t transpose32(uint32_t x, uint32_t lane) {
+    uint32_t y = __shfl_xor_sync(0xffffffffu, x, 16);
+    x = lane & 16 ? __byte_perm(x, y, 0x3276) : __byte_perm(x, y, 0x5410);
+    y = __shfl_xor_sync(0xffffffffu, x, 8);
+    x = lane & 8 ? __byte_perm(x, y, 0x3715) : __byte_perm(x, y, 0x6240);
+    const uint32_t m[3] = {0x0f0f0f0fu, 0x33333333u, 0x55555555u};
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const int j = 4 >> i;
+        y = __shfl_xor_sync(0xffffffffu, x, j);
+        x = lane & j ? (x & ~m[i]) | ((y >> j) & m[i]) : (x & m[i]) | ((y & m[i]) << j);
+    }
+    return x;
+}
+
 }  // namespace sg

@@ -118,6 +118,42 @@ struct Staged {
     }
 };
 
+// Several host arrays to the device in one copy: begin(room for all), add() each, send().
+struct StagedPack {
+    Staged buf;
+    size_t used = 0;
+    template <class T> static size_t room(size_t n) { return (n * sizeof(T) + 15) & ~(size_t)15; }
+    void begin(size_t bytes, cudaStream_t st) {
+        if (buf.pending) {
+            cudaError_t e = cudaEventSynchronize(buf.ev);
+            if (e != cudaSuccess) throw CudaError(e, "cudaEventSynchronize", __FILE__, __LINE__);
+            buf.pending = false;
+        }
+        buf.host.reserve(bytes ? bytes : 16);
+        buf.dev.reserve(bytes ? bytes : 16, st);
+        used = 0;
+    }
+    template <class T> const T *add(const T *src, size_t n) {
+        const size_t at = used;
+        if (n) memcpy(buf.host.as<char>() + at, src, n * sizeof(T));
+        used = at + room<T>(n);
+        return reinterpret_cast<const T *>(buf.dev.as<char>() + at);
+    }
+    void send(cudaStream_t st) {
+        if (used == 0) return;
+        cudaError_t e = cudaMemcpyAsync(buf.dev.ptr, buf.host.ptr, used, cudaMemcpyHostToDevice, st);
+        if (e != cudaSuccess) throw CudaError(e, "cudaMemcpyAsync", __FILE__, __LINE__);
+        if (!buf.ev) {
+            e = cudaEventCreateWithFlags(&buf.ev, cudaEventDisableTiming);
+            if (e != cudaSuccess) throw CudaError(e, "cudaEventCreateWithFlags", __FILE__, __LINE__);
+        }
+        e = cudaEventRecord(buf.ev, st);
+        if (e != cudaSuccess) throw CudaError(e, "cudaEventRecord", __FILE__, __LINE__);
+        buf.pending = true;
+    }
+    void release() { buf.release(); }
+};
+
 // Buffers of the batched window miner (sgfim_ring_mine_windows), kept by the
 // handle across calls: per-warp workspaces, the output arena, the window
 // table and its per-window results.
@@ -136,17 +172,17 @@ struct WindowWorkspace {
 // that repeated mining (anytime stages, window services) allocates nothing
 // once warm.
 struct MinerWorkspace {
-    DevBuf arena, pool, q_out, score, cooc, t_out, pdb, pofs, pmask, spool;
-    HostBuf hq_out, hscore, ht_out;
-    Staged q_ptr, q_items, q_slot, c_ptr, c_items, c_ps, c_cs, p_ptr, p_items, feat, w0, t_ptr, t_items, t_slot,
-        p_items_list, s_ptr, s_items, s_cols;
+    DevBuf arena, pool, q_out[2], score, cooc, t_out, pdb, pofs, plist, spool;
+    HostBuf hq_out[2], hscore, ht_out;
+    StagedPack queries[2], counts, masks, append, sappend;
+    Staged feat, p_items_list[16];
     void release() {
-        arena.release(); pool.release(); q_out.release(); score.release(); cooc.release(); t_out.release();
-        pdb.release(); pofs.release(); pmask.release(); spool.release();
-        hq_out.release(); hscore.release(); ht_out.release();
-        for (Staged *s : {&q_ptr, &q_items, &q_slot, &c_ptr, &c_items, &c_ps, &c_cs, &p_ptr, &p_items, &feat, &w0,
-                          &t_ptr, &t_items, &t_slot, &p_items_list, &s_ptr, &s_items, &s_cols})
-            s->release();
+        for (DevBuf *b : {&arena, &pool, &q_out[0], &q_out[1], &score, &cooc, &t_out, &pdb, &pofs, &plist, &spool})
+            b->release();
+        for (HostBuf *b : {&hq_out[0], &hq_out[1], &hscore, &ht_out}) b->release();
+        for (StagedPack *s : {&queries[0], &queries[1], &counts, &masks, &append, &sappend}) s->release();
+        feat.release();
+        for (Staged &s : p_items_list) s.release();
     }
 };
 

@@ -8,6 +8,8 @@
 namespace sg {
 
 constexpr uint32_t kNoSlot = 0xffffffffu;
+// in QueryBatch::mask_slot, with a slot: the query's first row belongs to the mask
+constexpr uint32_t kLeadRow = 0x80000000u;
 
 // Counting modes of the streaming query kernel.  QUERY_ANY stops at the first
 // set bit (result 0 / non-zero); QUERY_ANY2 stops once two bits are counted
@@ -34,6 +36,9 @@ struct QueryBatch {
     uint32_t *out = nullptr;
     uint64_t empty_value = 0;       // result of an empty query without mask
     int mode = QUERY_COUNT;
+    // optional: set bits of each query's mask (AND its first row with kLeadRow); a count below thr may then come out as anything below thr
+    const uint32_t *mask_sup = nullptr;
+    uint32_t thr = 0;
 };
 
 // Launchers (all asynchronous on `st`).
@@ -49,8 +54,8 @@ void launch_queries(const QueryBatch &qb, cudaStream_t st, int n_sm);
 // Counts of every (node, tail item) of a wave whose nodes hold a mask slot:
 // out[j] = popc(arena[slot[i]] AND rows[items[j]]) for tail_ptr[i] <= j < tail_ptr[i+1].
 void launch_tail_counts(const uint64_t *rows, uint64_t row_stride, uint64_t n_words, const uint64_t *arena,
-                        uint64_t arena_stride, const uint32_t *slot, const uint64_t *tail_ptr, uint32_t n_nodes,
-                        uint64_t n_entries, const uint32_t *items, uint32_t *out, cudaStream_t st, int n_sm);
+                        uint64_t arena_stride, const uint32_t *slot, const uint32_t *piv, const uint64_t *tail_ptr,
+                        uint32_t n_nodes, uint64_t n_entries, const uint32_t *items, uint32_t *out, cudaStream_t st, int n_sm);
 
 // Batched candidate supports (config "support-1m" path).  Packs CSR candidates
 // into 16-byte records when every item fits 16 bits and k <= 8, runs the
@@ -125,12 +130,15 @@ size_t staged_smem_bytes(uint32_t d, uint32_t cands_per_cta);
 void launch_wait_probe(uint32_t *err, cudaStream_t st);
 
 // Projected database of one item (the miner's root subtrees): out row e (for
-// every e in items, out_words <= out_stride words, all d rows zeroed first)
+// every e in items; out_words even, <= out_stride; zero past the packed bits)
 // holds the bits of row e at the transactions of row root_row, packed in order.
-// Scratch: ofs n_words x 4 B, masks 6 x n_words x 8 B.
-void launch_projection(const uint64_t *rows, uint64_t stride, uint64_t n_words, uint32_t root_row,
-                       const uint32_t *items, uint32_t n_items, uint32_t *ofs, uint64_t *masks, uint64_t *out,
-                       uint64_t out_stride, uint64_t out_words, uint32_t d, cudaStream_t st, int n_sm);
+// Other rows are left as they are.  n_set: the root row's set bits.  Scratch: sums
+// projection_chunks(n_words) x 4 B, list n_set x 4 B when projection_listed().
+void launch_projection(const uint64_t *rows, uint64_t stride, uint64_t n_words, uint32_t root_row, uint64_t n_set,
+                       const uint32_t *items, uint32_t n_items, uint32_t *sums, uint32_t *list, uint64_t *out,
+                       uint64_t out_stride, uint64_t out_words, cudaStream_t st);
+bool projection_listed(uint64_t n_set, uint64_t n_words);
+uint64_t projection_chunks(uint64_t n_words);   // words of sums;
 
 // Miner helpers.
 // mask(child c) = (parent_slot[c] != kNoSlot ? arena[parent_slot[c]] : ones) & AND rows(items[ptr[c]..ptr[c+1]))

@@ -166,93 +166,234 @@ void launch_row_popc(const uint64_t *rows, uint64_t stride, uint64_t n_words, ui
 }
 
 // ---------------------------------------------------------------- streaming queries
-// One warp per query; each lane streams 16-byte words of the mask and of the
-// query's rows with non-coherent 128-bit loads, ANDs them and popcounts.
-__global__ void __launch_bounds__(256) query_kernel(QueryBatch qb) {
+// A warp owns one segment of one query's words: a step covers 256 words, two rows
+// at a time (eight 16-byte loads in flight per lane), rows are read only where the
+// AND of the mask and the rows before them still has a bit, and the row numbers
+// travel in the lanes.  Few queries are cut into segments that fill the chip, whose
+// counts add up in `out`.  A count below qb.thr may be reported as anything below
+// it: a segment stops once its words miss more of the mask's mask_sup transactions
+// than mask_sup - thr (the search tree's FHUT queries mostly do, and soon).  These
+// queries wait for loads, not bandwidth: one 16-byte load per lane in flight, a
+// warp per query took 113 ms of a 2,000,000-transaction search, now 24 ms.
+constexpr uint32_t kQueryU = 4;
+constexpr uint32_t kQueryStep = 64 * kQueryU;   // words a warp covers per step
+
+constexpr uint32_t kQueryWarps = 96;            // per SM, four times what is resident: short tails
+
+static uint32_t query_segments(uint64_t n_units, uint64_t n_words, int n_sm) {
+    const uint64_t most = std::max<uint64_t>(1, (n_words + kQueryStep - 1) / kQueryStep);
+    return (uint32_t)std::min<uint64_t>(most, std::max<uint64_t>(1, (uint64_t)n_sm * kQueryWarps / std::max<uint64_t>(n_units, 1)));
+}
+
+__global__ void __launch_bounds__(256, 3) query_kernel(QueryBatch qb, uint32_t n_seg, uint64_t seg_words) {
+    constexpr unsigned kAll = 0xffffffffu;
     const uint32_t lane = threadIdx.x & 31;
-    const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
     const uint64_t n_warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t q = warp; q < qb.n_q; q += n_warps) {
-        const uint64_t a = qb.q_ptr[q], b = qb.q_ptr[q + 1];
+    const uint64_t total = qb.n_q * n_seg;
+    for (uint64_t unit = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; unit < total; unit += n_warps) {
+        const uint64_t q = n_seg == 1 ? unit : unit / n_seg, seg = unit - q * n_seg;
+        const uint64_t a = qb.q_ptr[q], k = qb.q_ptr[q + 1] - a;
         const uint64_t *mask = nullptr;
+        bool lead = false;   // the first row belongs to the mask
         if (qb.mask_slot) {
             const uint32_t s = qb.mask_slot[q];
-            if (s != kNoSlot) mask = qb.arena + (uint64_t)s * qb.arena_stride;
-        }
-        if (a == b && mask == nullptr) {
-            if (lane == 0) qb.out[q] = (uint32_t)qb.empty_value;
-            continue;
-        }
-        bool bad = false;
-        for (uint64_t i = a + lane; i < b; i += 32) bad |= qb.q_items[i] >= qb.d;
-        if (__any_sync(0xffffffffu, bad)) {
-            if (lane == 0) qb.out[q] = 0;
-            continue;
+            if (s != kNoSlot) mask = qb.arena + (uint64_t)(s & ~kLeadRow) * qb.arena_stride;
+            lead = s != kNoSlot && (s & kLeadRow);
         }
         uint32_t acc = 0;
-        const uint64_t w_first = qb.q_w0 ? (qb.q_w0[q] & ~1ull) : 0;
-        for (uint64_t base = w_first; base < qb.n_words; base += 64) {
-            const uint64_t w = base + 2 * lane;
-            if (w < qb.n_words) {
-                uint4 v = mask ? ld_nc_v4(mask + w) : make_uint4(~0u, ~0u, ~0u, ~0u);
-                for (uint64_t i = a; i < b; ++i) {
-                    // once the AND is empty the remaining rows cannot add a bit
-                    if ((v.x | v.y | v.z | v.w) == 0) break;
-                    v = and4(v, ld_nc_v4(qb.rows + (uint64_t)qb.q_items[i] * qb.row_stride + w));
+        if (k == 0 && mask == nullptr) {
+            acc = seg == 0 ? (uint32_t)qb.empty_value : 0u;
+        } else {
+            // the first 32 rows travel in the lanes
+            const uint32_t mine = lane < k ? qb.q_items[a + lane] : 0u;
+            bool bad = mine >= qb.d && lane < k;
+            for (uint64_t i = 32 + lane; i < k; i += 32) bad |= qb.q_items[a + i] >= qb.d;
+            if (!__any_sync(kAll, bad)) {
+                const uint64_t w_first = qb.q_w0 ? (qb.q_w0[q] & ~1ull) : 0;
+                const uint64_t w0 = max(w_first, seg * seg_words), w1 = min(qb.n_words, (seg + 1) * seg_words);
+                const bool bounded = mask && qb.mask_sup;
+                const uint32_t sup = bounded ? qb.mask_sup[q] : 0;
+                const uint32_t slack = bounded && sup > qb.thr ? sup - qb.thr : 0;
+                uint32_t part = 0, missed = 0;   // per lane
+                for (uint64_t base = w0; base < w1; base += kQueryStep) {
+                    const uint64_t at = base + 2 * lane;
+                    uint4 v[kQueryU];
+#pragma unroll
+                    for (uint32_t u = 0; u < kQueryU; ++u) {
+                        v[u] = make_uint4(0, 0, 0, 0);
+                        if (at + 64 * u < w1) v[u] = mask ? ld_nc_v4(mask + at + 64 * u) : make_uint4(~0u, ~0u, ~0u, ~0u);
+                    }
+                    if (lead) {
+                        const uint64_t *row = qb.rows + (uint64_t)__shfl_sync(kAll, mine, 0) * qb.row_stride + at;
+#pragma unroll
+                        for (uint32_t u = 0; u < kQueryU; ++u)
+                            if (at + 64 * u < w1) v[u] = and4(v[u], ld_nc_v4(row + 64 * u));
+                    }
+                    if (bounded)
+#pragma unroll
+                        for (uint32_t u = 0; u < kQueryU; ++u) missed += popc4(v[u]);
+                    bool left = true;   // some lane's AND still has a bit
+                    for (uint64_t i = lead; i < k; i += 2) {
+                        const uint64_t i2 = i + 1 < k ? i + 1 : i;   // an odd count ANDs its last row twice
+                        const uint32_t x = i < 32 ? __shfl_sync(kAll, mine, (int)i) : qb.q_items[a + i];
+                        const uint32_t y = i2 < 32 ? __shfl_sync(kAll, mine, (int)i2) : qb.q_items[a + i2];
+                        const uint64_t *rx = qb.rows + (uint64_t)x * qb.row_stride + at;
+                        const uint64_t *ry = qb.rows + (uint64_t)y * qb.row_stride + at;
+                        uint4 r[kQueryU], o[kQueryU];
+                        bool any = false;
+#pragma unroll
+                        for (uint32_t u = 0; u < kQueryU; ++u) {
+                            const bool live = (v[u].x | v[u].y | v[u].z | v[u].w) != 0;
+                            r[u] = o[u] = make_uint4(0, 0, 0, 0);
+                            if (live) {
+                                r[u] = ld_nc_v4(rx + 64 * u);
+                                o[u] = ld_nc_v4(ry + 64 * u);
+                            }
+                            any |= live;
+                        }
+#pragma unroll
+                        for (uint32_t u = 0; u < kQueryU; ++u) v[u] = and4(v[u], and4(r[u], o[u]));
+                        left = __any_sync(kAll, any);
+                        if (!left) break;
+                    }
+                    uint32_t got = 0;
+                    if (left)
+#pragma unroll
+                        for (uint32_t u = 0; u < kQueryU; ++u) got += popc4(v[u]);
+                    part += got;
+                    if (bounded) {
+                        missed -= got;
+                        if (__reduce_add_sync(kAll, missed) > slack) break;
+                    }
+                    if (qb.mode == QUERY_ANY && __any_sync(kAll, part != 0)) break;
+                    if (qb.mode == QUERY_ANY2 && __reduce_add_sync(kAll, part) >= 2) break;
                 }
-                acc += popc4(v);
+                acc = warp_sum(part);
             }
-            if (qb.mode == QUERY_ANY && __any_sync(0xffffffffu, acc != 0)) break;
-            if (qb.mode == QUERY_ANY2 && __reduce_add_sync(0xffffffffu, acc) >= 2) break;
         }
-        acc = warp_sum(acc);
-        if (lane == 0) qb.out[q] = acc;
+        if (lane == 0) {
+            if (n_seg == 1) qb.out[q] = acc;
+            else if (acc) atomicAdd(&qb.out[q], acc);
+        }
     }
 }
 
 // Tail counts of a wave's nodes: entry j of the concatenated tails belongs to
 // node i (tail_ptr[i] <= j < tail_ptr[i+1]); out[j] = popc(mask(slot[i]) AND
-// row(items[j])).  One warp per entry, the node found by binary search, so
-// the host builds one record per node instead of one query per tail item.
-__global__ void __launch_bounds__(256) tail_count_kernel(const uint64_t *__restrict__ rows, uint64_t row_stride,
+// row(piv[i]) AND row(items[j])); piv[i] may be kNoSlot (the mask is the node's own;
+// else it is its parent's).  A warp takes four entries at a time (the node found 32 places at
+// a time), so a node's mask is read once for up to four of its items, ten 16-byte
+// loads in flight per lane.  The population counts bound it (16 lanes a clock per
+// SM): eight words pass through carry-save adders (R. W. Harley's method; H. S.
+// Warren, Hacker's Delight, 2nd ed., section 5-1) into one count of eights.  Few
+// entries are cut into segments like the queries.  (A warp per entry, a count per
+// word: 28 ms of a 2,000,000-transaction search with
+// a mask per child, whose making took 22 ms more; now 28 and 5.)
+__device__ __forceinline__ void csa(uint32_t &high, uint32_t &low, uint32_t x, uint32_t y) {
+    const uint32_t u = low ^ x;
+    high = (low & x) | (u & y);
+    low = u ^ y;
+}
+constexpr uint32_t kTailI = 4, kTailU = 2;   // entries, 16-byte pieces of each in flight
+
+__global__ void __launch_bounds__(256, 3) tail_count_kernel(const uint64_t *__restrict__ rows, uint64_t row_stride,
                                                         uint64_t n_words, const uint64_t *__restrict__ arena,
                                                         uint64_t arena_stride, const uint32_t *__restrict__ slot,
+                                                        const uint32_t *__restrict__ piv,
                                                         const uint64_t *__restrict__ tail_ptr, uint32_t n_nodes,
-                                                        const uint32_t *__restrict__ items, uint32_t *__restrict__ out) {
+                                                        const uint32_t *__restrict__ items, uint32_t *__restrict__ out,
+                                                        uint32_t n_seg, uint64_t seg_words, uint32_t search_step) {
+    constexpr unsigned kAll = 0xffffffffu;
     const uint32_t lane = threadIdx.x & 31;
-    const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
     const uint64_t n_warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    const uint64_t total = tail_ptr[n_nodes];
-    for (uint64_t j = warp; j < total; j += n_warps) {
-        uint32_t lo = 0, hi = n_nodes - 1;
-        while (lo < hi) {
-            const uint32_t mid = (lo + hi + 1) >> 1;
-            if (tail_ptr[mid] <= j) lo = mid;
-            else hi = mid - 1;
+    const uint64_t n_entries = tail_ptr[n_nodes];
+    const uint64_t total = (n_entries + kTailI - 1) / kTailI * n_seg;
+    for (uint64_t unit = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; unit < total; unit += n_warps) {
+        const uint64_t g = n_seg == 1 ? unit : unit / n_seg, seg = unit - g * n_seg;
+        uint64_t j = g * kTailI;
+        const uint64_t j_end = min(n_entries, j + kTailI);
+        const uint64_t w0 = seg * seg_words, w1 = min(n_words, w0 + seg_words);
+        // the node of entry j: 32 places at a time
+        uint32_t lo = 0;
+        for (uint32_t step = search_step;; step >>= 5) {
+            const uint64_t at = (uint64_t)lo + (uint64_t)lane * step;
+            const unsigned le = __ballot_sync(kAll, at < n_nodes && tail_ptr[at] <= j);
+            lo += (31 - __clz(le)) * step;   // lane 0's place always holds
+            if (step == 1) break;
         }
-        const uint64_t *mask = arena + (uint64_t)slot[lo] * arena_stride;
-        const uint64_t *row = rows + (uint64_t)items[j] * row_stride;
-        uint32_t acc = 0;
-        for (uint64_t w = 2 * lane; w < n_words; w += 64) acc += popc4(and4(ld_nc_v4(mask + w), ld_nc_v4(row + w)));
-        acc = warp_sum(acc);
-        if (lane == 0) out[j] = acc;
+        while (j < j_end) {   // runs of one node's entries
+            while (tail_ptr[lo + 1] <= j) ++lo;
+            const uint32_t n = (uint32_t)(min(j_end, tail_ptr[lo + 1]) - j);
+            const uint64_t *mask = arena + (uint64_t)slot[lo] * arena_stride;
+            const uint64_t *lead = piv[lo] != kNoSlot ? rows + (uint64_t)piv[lo] * row_stride : mask;
+            const uint64_t *r[kTailI];
+#pragma unroll
+            for (uint32_t i = 0; i < kTailI; ++i) r[i] = rows + (uint64_t)items[j + min(i, n - 1)] * row_stride;
+            uint32_t ones[kTailI] = {0, 0, 0, 0}, twos[kTailI] = {0, 0, 0, 0}, fours[kTailI] = {0, 0, 0, 0};
+            uint32_t eights[kTailI] = {0, 0, 0, 0};
+            for (uint64_t base = w0; base < w1; base += 64 * kTailU) {
+                uint4 m[kTailU], v[kTailI][kTailU];
+#pragma unroll
+                for (uint32_t u = 0; u < kTailU; ++u) {
+                    const uint64_t w = base + 64 * u + 2 * lane;
+                    const bool in = w < w1;
+                    m[u] = in ? and4(ld_nc_v4(mask + w), ld_nc_v4(lead + w)) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+                    for (uint32_t i = 0; i < kTailI; ++i)
+                        v[i][u] = in && i < n ? ld_nc_v4(r[i] + w) : make_uint4(0, 0, 0, 0);
+                }
+#pragma unroll
+                for (uint32_t i = 0; i < kTailI; ++i) {
+                    if (i >= n) break;
+                    const uint4 x = and4(m[0], v[i][0]), y = and4(m[1], v[i][1]);
+                    uint32_t t0, t1, f0, f1, e;
+                    csa(t0, ones[i], x.x, x.y);
+                    csa(t1, ones[i], x.z, x.w);
+                    csa(f0, twos[i], t0, t1);
+                    csa(t0, ones[i], y.x, y.y);
+                    csa(t1, ones[i], y.z, y.w);
+                    csa(f1, twos[i], t0, t1);
+                    csa(e, fours[i], f0, f1);
+                    eights[i] += __popc(e);
+                }
+            }
+#pragma unroll
+            for (uint32_t i = 0; i < kTailI; ++i) {
+                const uint32_t c = warp_sum(8 * eights[i] + 4 * __popc(fours[i]) + 2 * __popc(twos[i]) + __popc(ones[i]));
+                if (lane == 0 && i < n) {
+                    if (n_seg == 1) out[j + i] = c;
+                    else if (c) atomicAdd(&out[j + i], c);
+                }
+            }
+            j += n;
+        }
     }
 }
 
 void launch_tail_counts(const uint64_t *rows, uint64_t row_stride, uint64_t n_words, const uint64_t *arena,
-                        uint64_t arena_stride, const uint32_t *slot, const uint64_t *tail_ptr, uint32_t n_nodes,
-                        uint64_t n_entries, const uint32_t *items, uint32_t *out, cudaStream_t st, int n_sm) {
+                        uint64_t arena_stride, const uint32_t *slot, const uint32_t *piv, const uint64_t *tail_ptr,
+                        uint32_t n_nodes, uint64_t n_entries, const uint32_t *items, uint32_t *out, cudaStream_t st, int n_sm) {
     if (n_nodes == 0 || n_entries == 0) return;
-    const uint64_t blocks = std::min<uint64_t>((n_entries + 7) / 8, (uint64_t)n_sm * 64);
-    tail_count_kernel<<<(unsigned)blocks, 256, 0, st>>>(rows, row_stride, n_words, arena, arena_stride, slot, tail_ptr,
-                                                        n_nodes, items, out);
+    const uint64_t groups = (n_entries + kTailI - 1) / kTailI;
+    const uint32_t n_seg = query_segments(groups, n_words, n_sm);
+    const uint64_t seg_words = ((n_words + n_seg - 1) / n_seg + kQueryStep - 1) / kQueryStep * kQueryStep;
+    if (n_seg > 1) SG_CUDA_TRY(cudaMemsetAsync(out, 0, n_entries * 4, st));
+    uint32_t search_step = 1;   // 32 steps of it cover the nodes
+    while ((uint64_t)search_step * 32 < n_nodes) search_step *= 32;
+    const uint64_t blocks = std::min<uint64_t>((groups * n_seg + 7) / 8, (uint64_t)n_sm * 64);
+    tail_count_kernel<<<(unsigned)blocks, 256, 0, st>>>(rows, row_stride, n_words, arena, arena_stride, slot, piv,
+                                                        tail_ptr, n_nodes, items, out, n_seg, seg_words, search_step);
     SG_CUDA_TRY(cudaGetLastError());
 }
 
 void launch_queries(const QueryBatch &qb, cudaStream_t st, int n_sm) {
     if (qb.n_q == 0) return;
-    const uint64_t blocks = std::min<uint64_t>((qb.n_q + 7) / 8, (uint64_t)n_sm * 64);
-    query_kernel<<<(unsigned)blocks, 256, 0, st>>>(qb);
+    const uint32_t n_seg = query_segments(qb.n_q, qb.n_words, n_sm);
+    const uint64_t seg_words =
+        std::max<uint64_t>(1, ((qb.n_words + n_seg - 1) / n_seg + kQueryStep - 1) / kQueryStep) * kQueryStep;
+    if (n_seg > 1) SG_CUDA_TRY(cudaMemsetAsync(qb.out, 0, qb.n_q * 4, st));
+    const uint64_t blocks = std::min<uint64_t>((qb.n_q * n_seg + 7) / 8, (uint64_t)n_sm * 64);
+    query_kernel<<<(unsigned)blocks, 256, 0, st>>>(qb, n_seg, seg_words);
     SG_CUDA_TRY(cudaGetLastError());
 }
 
@@ -1096,40 +1237,96 @@ void launch_wait_probe(uint32_t *err, cudaStream_t st) {
 }
 
 // ---------------------------------------------------------------- projected databases
-// Exclusive prefix popcounts of a row's words (one CTA): ofs[w] = set bits of
-// words 0 .. w-1, the position of word w's first transaction in the projection.
-__global__ void __launch_bounds__(1024) row_prefix_kernel(const uint64_t *__restrict__ row, uint64_t n_words,
-                                                          uint32_t *__restrict__ ofs) {
-    __shared__ uint32_t part[1024];
-    const uint32_t t = threadIdx.x;
-    const uint64_t per = (n_words + 1023) / 1024;
-    const uint64_t w0 = min(n_words, (uint64_t)t * per), w1 = min(n_words, w0 + per);
-    uint32_t s = 0;
-    for (uint64_t w = w0; w < w1; ++w) s += popc64(row[w]);
-    part[t] = s;
-    __syncthreads();
-    for (uint32_t o = 1; o < 1024; o <<= 1) {   // inclusive scan
-        const uint32_t v = t >= o ? part[t - o] : 0u;
-        __syncthreads();
-        part[t] += v;
-        __syncthreads();
+// A row restricted to the transactions of a root row, packed in their order.  A
+// block takes 256 words of the root: where its transactions start is the sum of the
+// blocks' popcounts before it (projection_sums_kernel), where its words' start a
+// scan.  The move masks of the compress of a root word, after H. S. Warren,
+// Hacker's Delight, 2nd ed., section 7-4 (six steps, step i shifting the bits under
+// mask i right by 2^i), depend on the root alone: they stay in registers while the
+// block goes through its items, eight at a time, packing into shared memory; whole
+// output words leave as plain stores, the two it shares with its neighbours by an
+// atomic on the cleared row.  (A launch of one CTA for the starts, masks kept in
+// memory and read again for each item, and an L2 atomic per input word took 18 + 3
+// + 31 us a root (31,250 words, 320 items on average), 74 ms with the clearing in a
+// 2,000,000-transaction search of 633 roots and their candidate pools; this way 57,
+// with the listed form below for sparse roots 47.)
+constexpr int kProjWords = 256;    // root words per block
+constexpr int kProjItems = 8;      // items packed between two barriers
+constexpr int kProjGroup = 32;     // items per block
+
+// blocks [0, n_chunks): sums[b] = set bits of the root's words [256 b, 256 (b+1));
+// the blocks after them clear one item's output row each
+__global__ void __launch_bounds__(kProjWords) projection_sums_kernel(const uint64_t *__restrict__ root, uint64_t n_words,
+                                                                    uint32_t n_chunks, uint32_t *__restrict__ sums,
+                                                                    const uint32_t *__restrict__ items,
+                                                                    uint64_t *__restrict__ out, uint64_t out_stride,
+                                                                    uint64_t out_words) {
+    if (blockIdx.x >= n_chunks) {
+        uint64_t *row = out + (uint64_t)items[blockIdx.x - n_chunks] * out_stride;
+        for (uint64_t w = 2 * threadIdx.x; w < out_words; w += 2 * kProjWords)
+            *reinterpret_cast<ulonglong2 *>(row + w) = make_ulonglong2(0, 0);
+        return;
     }
-    uint32_t run = part[t] - s;
-    for (uint64_t w = w0; w < w1; ++w) {
-        ofs[w] = run;
-        run += popc64(row[w]);
+    __shared__ uint32_t part[kProjWords / 32];
+    const uint64_t w = (uint64_t)blockIdx.x * kProjWords + threadIdx.x;
+    const uint32_t c = __reduce_add_sync(0xffffffffu, w < n_words ? (uint32_t)popc64(root[w]) : 0u);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = c;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t t = 0;
+        for (uint32_t i = 0; i < kProjWords / 32; ++i) t += part[i];
+        sums[blockIdx.x] = t;
     }
 }
 
-// The move masks of the compress (generalized extract) of each root word m,
-// after H. S. Warren, Hacker's Delight, 2nd ed., section 7-4: six steps, step i
-// shifting the bits in masks[i] right by 2^i, pack the bits of x under m to the
-// low end in order.  The masks depend on m alone, so they are computed once per
-// root and used for every projected row (masks[i * n_words + w]).
-__global__ void root_masks_kernel(const uint64_t *__restrict__ root, uint64_t n_words, uint64_t *__restrict__ masks) {
-    for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < n_words; w += (uint64_t)gridDim.x * blockDim.x) {
-        uint64_t m = root[w];
-        uint64_t mk = ~m << 1;   // ones at positions whose lower neighbour is a zero of m
+// Where a chunk's set bits start in the packed row (base: the chunks before), where
+// this thread's word starts in the chunk, and the chunk's total.
+__device__ __forceinline__ void chunk_positions(uint32_t c, const uint32_t *sums, uint32_t chunk, uint32_t t,
+                                                uint32_t lane, uint32_t wid, uint32_t *s_part, uint32_t *s_base,
+                                                uint32_t &base, uint32_t &mine, uint32_t &tot) {
+    uint32_t incl = c, before = 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= (uint32_t)o) incl += x;
+    }
+    for (uint32_t b = t; b < chunk; b += kProjWords) before += sums[b];
+    before = __reduce_add_sync(0xffffffffu, before);
+    if (lane == 31) s_part[wid] = incl;
+    if (lane == 0) s_base[wid] = before;
+    __syncthreads();
+    base = tot = 0;
+    mine = incl - c;
+#pragma unroll
+    for (uint32_t i = 0; i < kProjWords / 32; ++i) {
+        base += s_base[i];
+        if (i < wid) mine += s_part[i];
+        tot += s_part[i];
+    }
+}
+
+__global__ void __launch_bounds__(kProjWords) project_rows_kernel(const uint64_t *__restrict__ rows, uint64_t stride,
+                                                                 uint64_t n_words, const uint64_t *__restrict__ root,
+                                                                 const uint32_t *__restrict__ sums,
+                                                                 const uint32_t *__restrict__ items, uint32_t n_items,
+                                                                 unsigned long long *__restrict__ out,
+                                                                 uint64_t out_stride) {
+    constexpr uint32_t kBuf = kProjWords + 1;   // output words a block touches at most
+    __shared__ unsigned long long buf[kProjItems][kBuf + 1];
+    __shared__ uint32_t s_part[kProjWords / 32], s_base[kProjWords / 32];
+    const uint32_t t = threadIdx.x, lane = t & 31, wid = t >> 5;
+    const uint64_t w = (uint64_t)blockIdx.x * kProjWords + t;
+    const uint64_t m = w < n_words ? root[w] : 0;
+    const uint32_t c = popc64(m);
+    uint32_t base, mine, tot;
+    chunk_positions(c, sums, blockIdx.x, t, lane, wid, s_part, s_base, base, mine, tot);
+    if (tot == 0) return;
+    const uint32_t first = base >> 6, n_out = ((base + tot - 1) >> 6) - first + 1;
+    const uint32_t pos = base + mine - (first << 6);   // of the word's first bit, in the block's buffer
+    const bool own_first = (base & 63) == 0, own_last = ((base + tot) & 63) == 0;
+    uint64_t mv[6];
+    {
+        uint64_t x = m, mk = ~m << 1;   // ones at positions whose lower neighbour is a zero of m
 #pragma unroll
         for (int i = 0; i < 6; ++i) {
             uint64_t mp = mk ^ (mk << 1);   // parallel suffix (prefix xor towards the high end)
@@ -1138,85 +1335,190 @@ __global__ void root_masks_kernel(const uint64_t *__restrict__ root, uint64_t n_
             mp ^= mp << 8;
             mp ^= mp << 16;
             mp ^= mp << 32;
-            const uint64_t mv = mp & m;     // bits that move by 2^i in this step
-            m = (m ^ mv) | (mv >> (1 << i));
+            mv[i] = mp & x;                 // bits that move by 2^i in this step
+            x = (x ^ mv[i]) | (mv[i] >> (1 << i));
             mk &= ~mp;
-            masks[(uint64_t)i * n_words + w] = mv;
         }
     }
-}
-
-// Row items[blockIdx.y] of the projection: the bits of that bitmap row at the set
-// positions of `root`, packed in transaction order (out rows zeroed beforehand).
-__global__ void project_rows_kernel(const uint64_t *__restrict__ rows, uint64_t stride, uint64_t n_words,
-                                    const uint64_t *__restrict__ root, const uint32_t *__restrict__ ofs,
-                                    const uint64_t *__restrict__ masks, const uint32_t *__restrict__ items,
-                                    unsigned long long *__restrict__ out, uint64_t out_stride) {
-    const uint32_t e = items[blockIdx.y];
-    const uint64_t *src = rows + (uint64_t)e * stride;
-    unsigned long long *dst = out + (uint64_t)e * out_stride;
-    for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < n_words; w += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t m = root[w];
-        if (!m) continue;
-        uint64_t p = src[w] & m;
-        if (!p) continue;
+    const uint32_t g0 = blockIdx.y * kProjGroup, g1 = min(n_items, g0 + kProjGroup);
+    for (uint32_t g = g0; g < g1; g += kProjItems) {
+        const uint32_t n = min((uint32_t)kProjItems, g1 - g);
+        uint64_t x[kProjItems];
 #pragma unroll
-        for (int i = 0; i < 6; ++i) {
-            const uint64_t t = p & masks[(uint64_t)i * n_words + w];
-            p = (p ^ t) | (t >> (1 << i));
+        for (uint32_t i = 0; i < kProjItems; ++i)
+            x[i] = i < n && m ? rows[(uint64_t)items[g + i] * stride + w] & m : 0;
+#pragma unroll
+        for (uint32_t i = 0; i < kProjItems; ++i)
+            for (uint32_t k = t; k <= n_out; k += kProjWords) buf[i][k] = 0;
+        __syncthreads();
+#pragma unroll
+        for (uint32_t i = 0; i < kProjItems; ++i) {
+            uint64_t v = x[i];
+            if (v == 0) continue;
+#pragma unroll
+            for (int k = 0; k < 6; ++k) v = (v & ~mv[k]) | ((v & mv[k]) >> (1 << k));
+            const uint32_t lo = (uint32_t)v, hi = (uint32_t)(v >> 32), sh = pos & 31;
+            uint32_t *to = reinterpret_cast<uint32_t *>(buf[i]) + (pos >> 5);
+            const uint32_t a = lo << sh, b = __funnelshift_l(lo, hi, sh), e = __funnelshift_l(hi, 0u, sh);
+            if (a) atomicOr(to, a);
+            if (b) atomicOr(to + 1, b);
+            if (e) atomicOr(to + 2, e);
         }
-        const uint32_t nb = popc64(m);
-        const uint32_t o = ofs[w], sh = o & 63;
-        atomicOr(dst + (o >> 6), (unsigned long long)(p << sh));
-        if (sh && sh + nb > 64) atomicOr(dst + (o >> 6) + 1, (unsigned long long)(p >> (64 - sh)));
+        __syncthreads();
+        for (uint32_t i = 0; i < n; ++i) {
+            unsigned long long *dst = out + (uint64_t)items[g + i] * out_stride + first;
+            for (uint32_t k = t; k < n_out; k += kProjWords) {
+                const unsigned long long v = buf[i][k];
+                if ((k > 0 || own_first) && (k + 1 < n_out || own_last)) dst[k] = v;
+                else if (v) atomicOr(dst + k, v);
+            }
+        }
+        __syncthreads();
     }
 }
 
-void launch_projection(const uint64_t *rows, uint64_t stride, uint64_t n_words, uint32_t root_row,
-                       const uint32_t *items, uint32_t n_items, uint32_t *ofs, uint64_t *masks, uint64_t *out,
-                       uint64_t out_stride, uint64_t out_words, uint32_t d, cudaStream_t st, int n_sm) {
-    SG_CUDA_TRY(cudaMemset2DAsync(out, out_stride * 8, 0, out_words * 8, d, st));
-    if (n_items == 0 || n_words == 0) return;
+// A sparse root's transactions are listed instead, and a warp packs 1,024 of them
+// per item: each lane fetches the bits at 32 of its positions into one word and the
+// warp transposes the words (180 instructions per 1,024 output bits, against about
+// 70 for every 32 words of the whole row above).
+constexpr int kListItems = 8;      // items per warp
+
+__global__ void __launch_bounds__(kProjWords) projection_list_kernel(const uint64_t *__restrict__ root, uint64_t n_words,
+                                                                    const uint32_t *__restrict__ sums,
+                                                                    uint32_t *__restrict__ list, uint32_t n_list) {
+    __shared__ uint32_t s_part[kProjWords / 32], s_base[kProjWords / 32];
+    const uint32_t t = threadIdx.x, lane = t & 31, wid = t >> 5;
+    const uint64_t w = (uint64_t)blockIdx.x * kProjWords + t;
+    uint32_t base, at, tot;
+    uint64_t m = w < n_words ? root[w] : 0;
+    chunk_positions(popc64(m), sums, blockIdx.x, t, lane, wid, s_part, s_base, base, at, tot);
+    at += base;
+    for (; m; m &= m - 1, ++at)
+        if (at < n_list) list[at] = (uint32_t)(w * 64) + (__ffsll((long long)m) - 1);
+}
+
+__global__ void __launch_bounds__(256) project_listed_kernel(const uint64_t *__restrict__ rows, uint64_t stride,
+                                                             uint64_t n_words, const uint32_t *__restrict__ list,
+                                                             uint32_t n_list,
+                                                             const uint32_t *__restrict__ items, uint32_t n_items,
+                                                             uint64_t *__restrict__ out, uint64_t out_stride,
+                                                             uint64_t out_words) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t unit = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);   // 1,024 output bits
+    if (unit * 16 >= out_words) return;
+    const uint32_t first = (uint32_t)(unit * 1024);
+    const uint32_t g1 = min(n_items, (blockIdx.y + 1) * kListItems);
+    if (unit * 1024 >= n_list) {   // past the packed bits: zeros
+        for (uint32_t g = blockIdx.y * kListItems; g < g1; ++g)
+            if (unit * 32 + lane < 2 * out_words)
+                reinterpret_cast<uint32_t *>(out + (uint64_t)items[g] * out_stride)[unit * 32 + lane] = 0;
+        return;
+    }
+    uint32_t pos[32];
+#pragma unroll
+    for (uint32_t i = 0; i < 32; ++i) {
+        const uint64_t at = (uint64_t)first + i * 32 + lane;
+        pos[i] = at < n_list ? list[at] : 0xffffffffu;
+        if ((pos[i] >> 6) >= n_words) pos[i] = 0xffffffffu;
+    }
+#pragma unroll 1
+    for (uint32_t g = blockIdx.y * kListItems; g < g1; ++g) {
+        const uint32_t e = items[g];
+        const uint32_t *src = reinterpret_cast<const uint32_t *>(rows + (uint64_t)e * stride);
+        uint32_t bits = 0;   // bit i: of position pos[i]
+#pragma unroll
+        for (uint32_t i0 = 0; i0 < 32; i0 += 16) {
+            uint32_t v[16];
+#pragma unroll
+            for (uint32_t i = 0; i < 16; ++i) v[i] = pos[i0 + i] != 0xffffffffu ? __ldg(src + (pos[i0 + i] >> 5)) : 0u;
+#pragma unroll
+            for (uint32_t i = 0; i < 16; ++i) bits = __funnelshift_r(bits, __funnelshift_r(v[i], 0u, pos[i0 + i]), 1);
+        }
+        const uint32_t word = transpose32(bits, lane);
+        const uint64_t to = unit * 32 + lane;
+        if (to < 2 * out_words) reinterpret_cast<uint32_t *>(out + (uint64_t)e * out_stride)[to] = word;
+    }
+}
+
+uint64_t projection_chunks(uint64_t n_words) { return (n_words + kProjWords - 1) / kProjWords; }
+// By instructions the two meet at about 12 set bits a word.
+bool projection_listed(uint64_t n_set, uint64_t n_words) { return n_set <= 10 * n_words; }
+
+void launch_projection(const uint64_t *rows, uint64_t stride, uint64_t n_words, uint32_t root_row, uint64_t n_set,
+                       const uint32_t *items, uint32_t n_items, uint32_t *sums, uint32_t *list, uint64_t *out,
+                       uint64_t out_stride, uint64_t out_words, cudaStream_t st) {
+    if (n_items == 0 || out_words == 0) return;
     const uint64_t *root = rows + (uint64_t)root_row * stride;
-    row_prefix_kernel<<<1, 1024, 0, st>>>(root, n_words, ofs);
-    SG_CUDA_TRY(cudaGetLastError());
-    root_masks_kernel<<<(unsigned)std::min<uint64_t>((n_words + 255) / 256, (uint64_t)n_sm * 8), 256, 0, st>>>(
-        root, n_words, masks);
-    SG_CUDA_TRY(cudaGetLastError());
-    const unsigned bx = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((n_words + 255) / 256,
-                                                                            (uint64_t)n_sm * 16 / std::max(1u, n_items) + 1));
-    project_rows_kernel<<<dim3(bx, n_items), 256, 0, st>>>(rows, stride, n_words, root, ofs, masks, items,
-                                                           reinterpret_cast<unsigned long long *>(out), out_stride);
+    const uint32_t chunks = (uint32_t)projection_chunks(n_words);
+    const bool listed = projection_listed(n_set, n_words);
+    const uint32_t clear = listed ? 0 : n_items;   // the listed kernel writes whole rows
+    if (chunks + clear) {
+        projection_sums_kernel<<<chunks + clear, kProjWords, 0, st>>>(root, n_words, chunks, sums, items, out,
+                                                                      out_stride, out_words);
+        SG_CUDA_TRY(cudaGetLastError());
+    }
+    if (listed) {
+        if (chunks) {
+            projection_list_kernel<<<chunks, kProjWords, 0, st>>>(root, n_words, sums, list, (uint32_t)n_set);
+            SG_CUDA_TRY(cudaGetLastError());
+        }
+        const uint64_t units = (out_words + 15) / 16;
+        project_listed_kernel<<<dim3((unsigned)((units + 7) / 8), (n_items + kListItems - 1) / kListItems), 256, 0, st>>>(
+            rows, stride, n_words, list, (uint32_t)n_set, items, n_items, out, out_stride, out_words);
+    } else if (chunks) {
+        project_rows_kernel<<<dim3(chunks, (n_items + kProjGroup - 1) / kProjGroup), kProjWords, 0, st>>>(
+            rows, stride, n_words, root, sums, items, n_items, reinterpret_cast<unsigned long long *>(out), out_stride);
+    }
     SG_CUDA_TRY(cudaGetLastError());
 }
 
 // ---------------------------------------------------------------- miner helpers
-__global__ void child_mask_kernel(uint64_t *__restrict__ arena, uint64_t astride, uint64_t n_words,
-                                  const uint64_t *__restrict__ rows, uint64_t rstride, const uint64_t *__restrict__ ptr,
-                                  const uint32_t *__restrict__ items, const uint32_t *__restrict__ parent_slot,
-                                  const uint32_t *__restrict__ child_slot, uint32_t n) {
-    const uint64_t n_vec = n_words / 2;
-    const uint64_t total = (uint64_t)n * n_vec;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t c = (uint32_t)(i / n_vec);
-        const uint64_t v = i - (uint64_t)c * n_vec;
+// Masks of new nodes: mask(child) = mask(parent) AND the listed rows.  A warp takes
+// 256 words of one child, four 16-byte pieces per lane in flight.  (One 16-byte
+// piece per thread behind a 64-bit division: 22 ms of a 2,000,000-transaction
+// search, 11 this way, and 5 with masks for expanding nodes alone.)
+__global__ void __launch_bounds__(256) child_mask_kernel(uint64_t *__restrict__ arena, uint64_t astride, uint64_t n_words,
+                                                        const uint64_t *__restrict__ rows, uint64_t rstride,
+                                                        const uint64_t *__restrict__ ptr,
+                                                        const uint32_t *__restrict__ items,
+                                                        const uint32_t *__restrict__ parent_slot,
+                                                        const uint32_t *__restrict__ child_slot, uint32_t n,
+                                                        uint32_t n_steps) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t n_warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    const uint64_t total = (uint64_t)n * n_steps;
+    for (uint64_t i = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; i < total; i += n_warps) {
+        const uint32_t c = (uint32_t)(i / n_steps);
+        const uint64_t w = (i - (uint64_t)c * n_steps) * kQueryStep + 2 * lane;
         const uint32_t ps = parent_slot[c];
-        uint4 r = make_uint4(~0u, ~0u, ~0u, ~0u);
-        if (ps != kNoSlot) r = *reinterpret_cast<const uint4 *>(arena + (uint64_t)ps * astride + 2 * v);
-        for (uint64_t j = ptr[c]; j < ptr[c + 1]; ++j) r = and4(r, ld_nc_v4(rows + (uint64_t)items[j] * rstride + 2 * v));
-        *reinterpret_cast<uint4 *>(arena + (uint64_t)child_slot[c] * astride + 2 * v) = r;
+        const uint64_t a = ptr[c], b = ptr[c + 1];
+        const uint64_t *from = ps != kNoSlot ? arena + (uint64_t)ps * astride + w : nullptr;
+        uint64_t *to = arena + (uint64_t)child_slot[c] * astride + w;
+        uint4 r[kQueryU];
+#pragma unroll
+        for (uint32_t u = 0; u < kQueryU; ++u)
+            r[u] = from && w + 64 * u < n_words ? *reinterpret_cast<const uint4 *>(from + 64 * u)
+                                                : make_uint4(~0u, ~0u, ~0u, ~0u);
+        for (uint64_t j = a; j < b; ++j) {
+            const uint64_t *row = rows + (uint64_t)items[j] * rstride + w;
+#pragma unroll
+            for (uint32_t u = 0; u < kQueryU; ++u)
+                if (w + 64 * u < n_words) r[u] = and4(r[u], ld_nc_v4(row + 64 * u));
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < kQueryU; ++u)
+            if (w + 64 * u < n_words) *reinterpret_cast<uint4 *>(to + 64 * u) = r[u];
     }
 }
 
 void launch_child_masks(uint64_t *arena, uint64_t arena_stride, uint64_t n_words, const uint64_t *rows,
                         uint64_t row_stride, const uint64_t *ptr, const uint32_t *items, const uint32_t *parent_slot,
                         const uint32_t *child_slot, uint32_t n, cudaStream_t st, int n_sm) {
-    if (n == 0) return;
-    const uint64_t total = (uint64_t)n * (n_words / 2);
-    const unsigned blocks = (unsigned)std::min<uint64_t>((total + 255) / 256, (uint64_t)n_sm * 32);
+    if (n == 0 || n_words == 0) return;
+    const uint32_t n_steps = (uint32_t)((n_words + kQueryStep - 1) / kQueryStep);
+    const unsigned blocks = (unsigned)std::min<uint64_t>(((uint64_t)n * n_steps + 7) / 8, (uint64_t)n_sm * 32);
     child_mask_kernel<<<blocks, 256, 0, st>>>(arena, arena_stride, n_words, rows, row_stride, ptr, items, parent_slot,
-                                              child_slot, n);
+                                              child_slot, n, n_steps);
     SG_CUDA_TRY(cudaGetLastError());
 }
 

@@ -65,14 +65,19 @@ namespace {
 using Clock = std::chrono::steady_clock;
 constexpr uint32_t kNoNode = 0xffffffffu;
 constexpr uint32_t kNoProj = 0xffffffffu;
-constexpr uint32_t kProjSlots = 8;
+constexpr uint32_t kNoItem = 0xffffffffu;
+constexpr uint32_t kProjSlots = 16;   // MinerWorkspace::p_items_list has one list per slot
+constexpr uint32_t kWaveRoots = 8;    // root subtrees of a wave; the other slots take the next ones meanwhile
 constexpr uint32_t kDim = SGFIM_TRACE_DIM;
 
 struct MNode {
     std::vector<uint32_t> head;  // dense ids
     std::vector<uint32_t> tail;  // dense ids, in the order's sequence
     uint32_t sup = 0;
-    uint32_t slot = kNoSlot;     // tidset mask slot; kNoSlot = AND of head rows
+    // tidset mask: slot's (its own) or, with a pivot, slot's (its parent's) AND the pivot's row;
+    // kNoSlot = AND of head rows
+    uint32_t slot = kNoSlot;
+    uint32_t piv = kNoItem;
     uint32_t id = 0;             // search-tree node id
     uint32_t proj = kNoProj;     // root item whose projected database the node's masks live in
 };
@@ -108,11 +113,8 @@ template <class F> void parallel_ranges(uint64_t n, F &&fn) {
 class Miner {
   public:
     Miner(sgfim_handle *h, const sgfim_mine_params &p)
-        : h_(h), ds_(h->ds), p_(p), w_(h->mws), arena_(w_.arena), pool_(w_.pool), q_ptr_(w_.q_ptr),
-          q_items_(w_.q_items), q_slot_(w_.q_slot), c_ptr_(w_.c_ptr), c_items_(w_.c_items), c_ps_(w_.c_ps),
-          c_cs_(w_.c_cs), p_ptr_(w_.p_ptr), p_items_(w_.p_items), feat_(w_.feat), w0_(w_.w0), q_out_(w_.q_out),
-          score_(w_.score), hq_out_(w_.hq_out), hscore_(w_.hscore) {}
-    // (tail-count staging lives in w_: t_ptr, t_items, t_slot, t_out, ht_out)
+        : h_(h), ds_(h->ds), p_(p), w_(h->mws), arena_(w_.arena), pool_(w_.pool), feat_(w_.feat),
+          score_(w_.score), hscore_(w_.hscore) {}
 
     int run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *user, sgfim_result **out);
 
@@ -127,6 +129,7 @@ class Miner {
     DevBuf &arena_;
     uint64_t slot_words_ = 0;
     std::vector<uint32_t> free_slots_;
+    std::vector<uint32_t> slot_refs_;    // nodes that use a slot
     // the bitmap view the wave's queries read: the whole database, or the
     // buffer of resident projections (rows translated per node by prow)
     const uint64_t *vrows_ = nullptr;
@@ -191,9 +194,9 @@ class Miner {
     bool need_feat_ = false;
     std::vector<uint32_t> cooc_;
     // staging (workspace)
-    Staged &q_ptr_, &q_items_, &q_slot_, &c_ptr_, &c_items_, &c_ps_, &c_cs_, &p_ptr_, &p_items_, &feat_, &w0_;
-    DevBuf &q_out_, &score_;
-    HostBuf &hq_out_, &hscore_;
+    Staged &feat_;
+    DevBuf &score_;
+    HostBuf &hscore_;
     uint64_t nodes_ = 0, waves_ = 0, launches_ = 0;
     // per-node bookkeeping of a wave (PEP, extension order, candidates, children):
     // host threads on large datasets; one (the caller) on small ones, whose waves
@@ -216,12 +219,28 @@ class Miner {
         if (free_slots_.empty()) return kNoSlot;
         uint32_t s = free_slots_.back();
         free_slots_.pop_back();
+        slot_refs_[s] = 0;
         return s;
     }
+    void drop_slot(uint32_t s) {
+        if (--slot_refs_[s] == 0) free_slots_.push_back(s);
+    }
+    // launches qs in query buffer `which` (0 or 1); collect_queries(), after a synchronisation,
+    // brings the results
+    void launch_query_set(const QuerySet &qs, const uint64_t *rows, uint64_t stride, uint64_t n_words, uint32_t d,
+                          int mode, int which, const uint64_t *w0 = nullptr,
+                          const std::vector<uint32_t> *mask_sup = nullptr);
+    void collect_queries(const QuerySet &qs, int which, std::vector<uint32_t> &out);
     void run_queries(const QuerySet &qs, const uint64_t *rows, uint64_t stride, uint64_t n_words, uint32_t d,
-                     int mode, std::vector<uint32_t> &out, const uint64_t *w0 = nullptr);
+                     int mode, std::vector<uint32_t> &out, const uint64_t *w0 = nullptr) {
+        launch_query_set(qs, rows, stride, n_words, d, mode, 0, w0);
+        if (qs.size()) h_->sync();
+        collect_queries(qs, 0, out);
+    }
+    void launch_masks(const QuerySet &qs, const std::vector<uint32_t> &slots);
     void run_tail_counts(const std::vector<uint64_t> &ptr, const std::vector<uint32_t> &items,
-                         const std::vector<uint32_t> &slots, std::vector<uint32_t> &out);
+                         const std::vector<uint32_t> &slots, const std::vector<uint32_t> &pivs,
+                         std::vector<uint32_t> &out);
     void pool_reserve(uint64_t members);
     void flush_pool(uint64_t from);
     void load_cooc();
@@ -231,43 +250,75 @@ class Miner {
     int finish(sgfim_result **out);
 };
 
-void Miner::run_queries(const QuerySet &qs, const uint64_t *rows, uint64_t stride, uint64_t n_words, uint32_t d,
-                        int mode, std::vector<uint32_t> &out, const uint64_t *w0) {
-    const size_t n = qs.size();
-    out.assign(n, 0);
+void Miner::launch_query_set(const QuerySet &qs, const uint64_t *rows, uint64_t stride, uint64_t n_words, uint32_t d,
+                             int mode, int which, const uint64_t *w0, const std::vector<uint32_t> *mask_sup) {
+    const size_t n = qs.size(), ni = qs.items.size();
     if (n == 0) return;
     cudaStream_t st = h_->stream;
     QueryBatch qb;
-    qb.q_ptr = q_ptr_.put(qs.ptr.data(), n + 1, st);
-    qb.q_items = q_items_.put(qs.items.data(), qs.items.size(), st);
-    qb.mask_slot = q_slot_.put(qs.slot.data(), n, st);
-    if (w0) qb.q_w0 = w0_.put(w0, n, st);
-    q_out_.reserve(n * 4, st);
-    hq_out_.reserve(n * 4);
+    StagedPack &pk = w_.queries[which];
+    pk.begin(pk.room<uint64_t>(n + 1) + pk.room<uint32_t>(ni) + 2 * pk.room<uint32_t>(n) + pk.room<uint64_t>(n), st);
+    qb.q_ptr = pk.add(qs.ptr.data(), n + 1);
+    qb.q_items = pk.add(qs.items.data(), ni);
+    qb.mask_slot = pk.add(qs.slot.data(), n);
+    if (w0) qb.q_w0 = pk.add(w0, n);
+    if (mask_sup) {
+        qb.mask_sup = pk.add(mask_sup->data(), n);
+        qb.thr = thr_;
+    }
+    pk.send(st);
+    w_.q_out[which].reserve(n * 4, st);
+    w_.hq_out[which].reserve(n * 4);
     qb.rows = rows; qb.row_stride = stride; qb.n_words = n_words; qb.d = d;
     qb.arena = arena_.as<uint64_t>(); qb.arena_stride = slot_words_;
-    qb.n_q = n; qb.out = q_out_.as<uint32_t>(); qb.empty_value = ds_.n_txn; qb.mode = mode;
+    qb.n_q = n; qb.out = w_.q_out[which].as<uint32_t>(); qb.empty_value = ds_.n_txn; qb.mode = mode;
     launch_queries(qb, st, h_->n_sm);
     ++launches_;
-    SG_CUDA_TRY(cudaMemcpyAsync(hq_out_.ptr, q_out_.ptr, n * 4, cudaMemcpyDeviceToHost, st));
-    h_->sync();
-    memcpy(out.data(), hq_out_.ptr, n * 4);
+    SG_CUDA_TRY(cudaMemcpyAsync(w_.hq_out[which].ptr, w_.q_out[which].ptr, n * 4, cudaMemcpyDeviceToHost, st));
+}
+
+void Miner::collect_queries(const QuerySet &qs, int which, std::vector<uint32_t> &out) {
+    const size_t n = qs.size();
+    out.resize(n);
+    if (n) memcpy(out.data(), w_.hq_out[which].ptr, n * 4);
+}
+
+// Masks of new slots: the AND of each query's rows and, with a slot, that slot's mask.
+void Miner::launch_masks(const QuerySet &qs, const std::vector<uint32_t> &slots) {
+    const size_t n = qs.size();
+    if (n == 0) return;
+    cudaStream_t st = h_->stream;
+    StagedPack &pk = w_.masks;
+    pk.begin(pk.room<uint64_t>(n + 1) + pk.room<uint32_t>(qs.items.size()) + 2 * pk.room<uint32_t>(n), st);
+    const uint64_t *dptr = pk.add(qs.ptr.data(), n + 1);
+    const uint32_t *ditems = pk.add(qs.items.data(), qs.items.size());
+    const uint32_t *dps = pk.add(qs.slot.data(), n);
+    const uint32_t *dcs = pk.add(slots.data(), n);
+    pk.send(st);
+    launch_child_masks(arena_.as<uint64_t>(), slot_words_, vwords_, vrows_, vstride_, dptr, ditems, dps, dcs,
+                       (uint32_t)n, st, h_->n_sm);
+    ++launches_;
 }
 
 // Counts of the tail items of the wave's nodes that hold a mask: one record
-// per node (its slot and tail range), one result per tail entry.
+// per node (its slot, pivot row and tail range), one result per tail entry.
 void Miner::run_tail_counts(const std::vector<uint64_t> &ptr, const std::vector<uint32_t> &items,
-                            const std::vector<uint32_t> &slots, std::vector<uint32_t> &out) {
+                            const std::vector<uint32_t> &slots, const std::vector<uint32_t> &pivs,
+                            std::vector<uint32_t> &out) {
     const size_t n = items.size();
     out.resize(n);
     if (n == 0) return;
     cudaStream_t st = h_->stream;
-    const uint64_t *dptr = w_.t_ptr.put(ptr.data(), ptr.size(), st);
-    const uint32_t *ditems = w_.t_items.put(items.data(), n, st);
-    const uint32_t *dslot = w_.t_slot.put(slots.data(), slots.size(), st);
+    StagedPack &pk = w_.counts;
+    pk.begin(pk.room<uint64_t>(ptr.size()) + pk.room<uint32_t>(n) + 2 * pk.room<uint32_t>(slots.size()), st);
+    const uint64_t *dptr = pk.add(ptr.data(), ptr.size());
+    const uint32_t *ditems = pk.add(items.data(), n);
+    const uint32_t *dslot = pk.add(slots.data(), slots.size());
+    const uint32_t *dpiv = pk.add(pivs.data(), pivs.size());
+    pk.send(st);
     w_.t_out.reserve(n * 4, st);
     w_.ht_out.reserve(n * 4);
-    launch_tail_counts(vrows_, vstride_, vwords_, arena_.as<uint64_t>(), slot_words_, dslot,
+    launch_tail_counts(vrows_, vstride_, vwords_, arena_.as<uint64_t>(), slot_words_, dslot, dpiv,
                        dptr, (uint32_t)slots.size(), n, ditems, w_.t_out.as<uint32_t>(), st, h_->n_sm);
     ++launches_;
     SG_CUDA_TRY(cudaMemcpyAsync(w_.ht_out.ptr, w_.t_out.ptr, n * 4, cudaMemcpyDeviceToHost, st));
@@ -340,8 +391,11 @@ void Miner::flush_pool(uint64_t from) {
     const uint32_t cnt = (uint32_t)(n - from);
     std::vector<uint64_t> lp(cnt + 1);
     for (uint32_t i = 0; i <= cnt; ++i) lp[i] = cptr_[from + i] - cptr_[from];
-    const uint64_t *dp = p_ptr_.put(lp.data(), cnt + 1, h_->stream);
-    const uint32_t *di = p_items_.put(citems_.data() + cptr_[from], lp[cnt], h_->stream);
+    StagedPack &pk = w_.append;
+    pk.begin(pk.room<uint64_t>(cnt + 1) + pk.room<uint32_t>(lp[cnt]), h_->stream);
+    const uint64_t *dp = pk.add(lp.data(), cnt + 1);
+    const uint32_t *di = pk.add(citems_.data() + cptr_[from], lp[cnt]);
+    pk.send(h_->stream);
     launch_pool_append(pool_.as<uint64_t>(), pool_words_, dp, di, from, cnt, h_->stream);
     ++launches_;
     pool_n_ = n;
@@ -385,9 +439,13 @@ void Miner::flush_pool(uint64_t from) {
         }
     });
     spool_reserve(*std::max_element(spool_n_.begin(), spool_n_.end()));
-    launch_pool_append(w_.spool.as<uint64_t>(), spool_words_, w_.s_ptr.put(sp_ptr_.data(), sp_ptr_.size(), h_->stream),
-                       w_.s_items.put(sp_items_.data(), sp_items_.size(), h_->stream), 0, (uint32_t)sp_cols_.size(),
-                       h_->stream, w_.s_cols.put(sp_cols_.data(), sp_cols_.size(), h_->stream));
+    StagedPack &sk = w_.sappend;
+    sk.begin(sk.room<uint64_t>(sp_ptr_.size()) + sk.room<uint32_t>(sp_items_.size()) + sk.room<uint64_t>(n_ent), h_->stream);
+    const uint64_t *sptr = sk.add(sp_ptr_.data(), sp_ptr_.size());
+    const uint32_t *sitems = sk.add(sp_items_.data(), sp_items_.size());
+    const uint64_t *scols = sk.add(sp_cols_.data(), n_ent);
+    sk.send(h_->stream);
+    launch_pool_append(w_.spool.as<uint64_t>(), spool_words_, sptr, sitems, 0, (uint32_t)n_ent, h_->stream, scols);
     ++launches_;
 }
 
@@ -465,27 +523,26 @@ bool Miner::make_resident(const MNode &nd) {
     const uint32_t r = nd.proj;
     std::vector<uint32_t> items(nd.head.begin(), nd.head.end());
     items.insert(items.end(), nd.tail.begin(), nd.tail.end());
-    const uint32_t *ditems = w_.p_items_list.put(items.data(), items.size(), st);
-    // whole rows are cleared: a wave reads up to its widest projection, so every
-    // row must be zero past its own projection's words
-    launch_projection(ds_.bitmaps.as<uint64_t>(), ds_.stride, ds_.n_words, r, ditems, (uint32_t)items.size(),
-                      w_.pofs.as<uint32_t>(), w_.pmask.as<uint64_t>(),
-                      w_.pdb.as<uint64_t>() + (uint64_t)slot * ds_.d * proj_stride_,
-                      proj_stride_, proj_stride_, ds_.d, st, h_->n_sm);
-    launches_ += 3;
+    const uint32_t *ditems = w_.p_items_list[slot].put(items.data(), items.size(), st);
+    // the listed rows are cleared whole: a wave reads up to its widest projection, so
+    // a row must be zero past its own projection's words (other rows are not read)
+    if (projection_listed(ds_.sup[r], ds_.n_words)) w_.plist.reserve((size_t)ds_.sup[r] * 4, st);
+    launch_projection(ds_.bitmaps.as<uint64_t>(), ds_.stride, ds_.n_words, r, ds_.sup[r], ditems,
+                      (uint32_t)items.size(), w_.pofs.as<uint32_t>(), w_.plist.as<uint32_t>(), w_.pdb.as<uint64_t>() + (uint64_t)slot * ds_.d * proj_stride_,
+                      proj_stride_, proj_stride_, st);
+    launches_ += projection_listed(ds_.sup[r], ds_.n_words) ? 3 : 2;
     ++projections_;
     if (use_spool_) {
         // the pool projected on r's pool row: every candidate so far (all are in the
         // device pool: the previous wave flushed them) that holds r
         spool_reserve(cand_freq_[r]);
         const uint64_t pw = pool_n_ ? ((pool_n_ + 63) / 64 + 1) & ~1ull : 0;
-        w_.pofs.reserve(std::max<uint64_t>(pw, 1) * 4, st);
-        w_.pmask.reserve(std::max<uint64_t>(pw, 1) * 6 * 8, st);
-        launch_projection(pool_.as<uint64_t>(), pool_words_, pw, r, ditems, (uint32_t)items.size(),
-                          w_.pofs.as<uint32_t>(), w_.pmask.as<uint64_t>(),
-                          w_.spool.as<uint64_t>() + (uint64_t)slot * ds_.d * spool_words_,
-                          spool_words_, spool_words_, ds_.d, st, h_->n_sm);
-        launches_ += 3;
+        w_.pofs.reserve(std::max<uint64_t>(projection_chunks(pw), 1) * 4, st);
+        if (projection_listed(cand_freq_[r], pw)) w_.plist.reserve((size_t)cand_freq_[r] * 4, st);
+        launch_projection(pool_.as<uint64_t>(), pool_words_, pw, r, cand_freq_[r], ditems, (uint32_t)items.size(),
+                          w_.pofs.as<uint32_t>(), w_.plist.as<uint32_t>(), w_.spool.as<uint64_t>() + (uint64_t)slot * ds_.d * spool_words_,
+                          spool_words_, spool_words_, st);
+        launches_ += pw == 0 ? 1 : projection_listed(cand_freq_[r], pw) ? 3 : 2;
         spool_n_[slot] = cand_freq_[r];
     }
     slot_root_[slot] = r;
@@ -531,8 +588,8 @@ int Miner::run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *use
         n_proj_slots_ = (uint32_t)std::max<uint64_t>(
             1, std::min<uint64_t>(kProjSlots, (h_->hbm_budget / 8) / std::max<uint64_t>(slot_bytes, 1)));
         w_.pdb.reserve((size_t)n_proj_slots_ * slot_bytes, st);
-        w_.pofs.reserve((size_t)std::max<uint64_t>(ds_.n_words, 1) * 4, st);
-        w_.pmask.reserve((size_t)std::max<uint64_t>(ds_.n_words, 1) * 6 * 8, st);
+        w_.pofs.reserve((size_t)std::max<uint64_t>(projection_chunks(ds_.n_words), 1) * 4, st);
+        w_.plist.reserve((size_t)10 * ds_.n_words * 4, st);
         slot_root_.assign(n_proj_slots_, kNoProj);
         root_slot_.assign(d, -1);
         live_.assign(d, 0);
@@ -552,6 +609,7 @@ int Miner::run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *use
     if (max_slots < 64) max_slots = 64;
     arena_.reserve(max_slots * slot_bytes, st);
     free_slots_.resize(max_slots);
+    slot_refs_.assign(max_slots, 0);
     for (uint64_t i = 0; i < max_slots; ++i) free_slots_[i] = (uint32_t)(max_slots - 1 - i);
     pool_reserve(65536);
 
@@ -570,11 +628,12 @@ int Miner::run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *use
     }
     uint32_t next_ck = 0;
     std::vector<MNode> wave;
+    size_t roots_left = 0;   // with projections: root children not popped yet, the bottom of the stack
     QuerySet qs, qpool, qfhut, qchild;
     std::vector<uint32_t> counts, counts_q, pool_hit, fhut_cnt, tmp;
     // tail counts of nodes with a mask: concatenated tails, per-node ranges and slots
     std::vector<uint64_t> t_ptr;
-    std::vector<uint32_t> t_items, t_slot;
+    std::vector<uint32_t> t_items, t_slot, t_piv, fhut_sup;
     std::vector<std::pair<uint8_t, uint64_t>> count_src;   // per wave node: (0 tail path | 1 query path, offset)
     std::vector<float> wfeat, wscore;
     int status = SGFIM_OK;
@@ -589,10 +648,10 @@ int Miner::run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *use
         size_t e0 = 0, ei0 = 0;                        // its candidate's index and item offset in the wave
         size_t feat0 = 0;                              // first feature row of its extensions
         size_t kid0 = 0, nkids = 0;                    // range in the wave's kid list
+        uint32_t kslot = kNoSlot;                      // the mask its children start from
     };
     std::vector<Work> work;
     std::vector<MNode> kids;
-    std::vector<std::pair<uint32_t, uint32_t>> kid_src;  // (parent slot, added item)
     std::vector<uint32_t> child_slot;
 
     while (!stack.empty()) {
@@ -614,6 +673,7 @@ int Miner::run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *use
         uint64_t nq = 0;
         bool wave_global = !use_proj_;
         uint64_t wave_words = 0;
+        uint32_t wave_roots = 0, last_root = kNoProj;   // (a subtree's nodes are next to each other on the stack)
         while (!stack.empty() && wave.size() < nmax) {
             if (use_proj_) {
                 const MNode &top = stack.back();
@@ -623,7 +683,10 @@ int Miner::run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *use
                 } else {
                     if (wave_global && !wave.empty()) break;
                     wave_global = false;
+                    if (top.proj != last_root && wave_roots == kWaveRoots) break;
                     if (root_slot_[top.proj] < 0 && !make_resident(top)) break;
+                    wave_roots += top.proj != last_root;
+                    last_root = top.proj;
                     wave_words = std::max(wave_words, wp_[top.proj]);
                 }
             }
@@ -654,22 +717,17 @@ int Miner::run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *use
             add_query(qchild, nd, nd.head.data(), nd.head.size(), kNoSlot);
             child_slot.push_back(s);
             nd.slot = s;
+            nd.piv = kNoItem;
+            slot_refs_[s] = 1;
         }
-        if (qchild.size()) {
-            const size_t n = qchild.size();
-            launch_child_masks(arena_.as<uint64_t>(), slot_words_, vwords_, vrows_, vstride_,
-                               c_ptr_.put(qchild.ptr.data(), n + 1, st),
-                               c_items_.put(qchild.items.data(), qchild.items.size(), st),
-                               c_ps_.put(qchild.slot.data(), n, st), c_cs_.put(child_slot.data(), n, st), (uint32_t)n,
-                               st, h_->n_sm);
-            ++launches_;
-        }
+        launch_masks(qchild, child_slot);
         // ---- phase A: s_e for every tail item (nodes with a mask: one record per node;
         // nodes without one, created while the arena was full: a query per item)
         // (positions in wave order here, the masked nodes' tail rows copied in parallel below)
         qs.clear();
         t_ptr.assign(1, 0);
         t_slot.clear();
+        t_piv.clear();
         count_src.resize(wave.size());
         uint64_t n_ti = 0;
         for (size_t i = 0; i < wave.size(); ++i) {
@@ -680,6 +738,7 @@ int Miner::run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *use
                 n_ti += nd.tail.size();
                 t_ptr.push_back(n_ti);
                 t_slot.push_back(nd.slot);
+                t_piv.push_back(nd.piv == kNoItem ? kNoSlot : prow(nd, nd.piv));
             } else {
                 count_src[i] = {1, qs.size()};
                 for (uint32_t e : nd.tail) {
@@ -700,9 +759,15 @@ int Miner::run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *use
             }
         });
         timed(0, [&] {
-            run_tail_counts(t_ptr, t_items, t_slot, counts);
+            run_tail_counts(t_ptr, t_items, t_slot, t_piv, counts);
             run_queries(qs, vrows_, vstride_, vwords_, vd_, QUERY_COUNT, counts_q);
         });
+        // the next root subtrees' projections, in the slots that are free, while the host
+        // works on this wave (they are resident from here on: flush_pool adds the wave's
+        // candidates to their pools)
+        roots_left = std::min(roots_left, stack.size());
+        for (size_t i = roots_left; i-- > 0;)
+            if (root_slot_[stack[i].proj] < 0 && !make_resident(stack[i])) break;
         // ---- phase B: PEP, extension order, pool and FHUT queries; each node on
         // the host pool, then the query lists concatenated in wave order
         auto t_exp = Clock::now();
@@ -732,6 +797,8 @@ int Miner::run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *use
                         (use_proj_ && nd.proj != kNoProj) ? (uint32_t)root_slot_[nd.proj] * ds_.d : 0u;
                     if (nd.slot == kNoSlot)
                         for (uint32_t h : wk.head) wk.fq.push_back(h + off);
+                    else if (nd.piv != kNoItem)
+                        wk.fq.push_back(nd.piv + off);
                     for (auto &pr : wk.f) wk.fq.push_back(pr.second + off);
                 }
                 // the pool query lists the rarest pool rows first: the device AND empties
@@ -754,6 +821,7 @@ int Miner::run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *use
         qpool.slot.assign(wave.size(), kNoSlot);
         qfhut.ptr.assign(1, 0);
         qfhut.slot.clear();
+        fhut_sup.clear();
         for (size_t i = 0; i < wave.size(); ++i) {
             Work &wk = work[i];
             wk.pool_q = i;
@@ -764,7 +832,9 @@ int Miner::run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *use
                 wk.fi0 = n_fi;
                 n_fi += wk.fq.size();
                 qfhut.ptr.push_back(n_fi);
-                qfhut.slot.push_back(wave[i].slot);
+                const MNode &nd = wave[i];
+                qfhut.slot.push_back(nd.slot == kNoSlot || nd.piv == kNoItem ? nd.slot : nd.slot | kLeadRow);
+                fhut_sup.push_back(wave[i].sup);
             }
             if (slot_pools) spool_max = std::max(spool_max, spool_n_[root_slot_[wave[i].proj]]);
         }
@@ -778,18 +848,23 @@ int Miner::run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *use
             }
         });
         add_since(6, t_exp);
-        if (slot_pools && spool_max > 0) {
-            const uint64_t pw = ((spool_max + 63) / 64 + 1) & ~1ull;
-            timed(1, [&] {
-                run_queries(qpool, w_.spool.as<uint64_t>(), spool_words_, pw, n_proj_slots_ * d, QUERY_ANY, pool_hit);
-            });
-        } else if (!slot_pools && pool_n_ > 0) {
-            const uint64_t pw = ((pool_n_ + 63) / 64 + 1) & ~1ull;
-            timed(1, [&] { run_queries(qpool, pool_.as<uint64_t>(), pool_words_, pw, d, QUERY_ANY, pool_hit); });
-        } else {
-            pool_hit.assign(qpool.size(), 0);
-        }
-        timed(2, [&] { run_queries(qfhut, vrows_, vstride_, vwords_, vd_, QUERY_COUNT, fhut_cnt); });
+        // both in one round trip
+        timed(2, [&] {
+            bool pool = true;
+            if (slot_pools && spool_max > 0)
+                launch_query_set(qpool, w_.spool.as<uint64_t>(), spool_words_, ((spool_max + 63) / 64 + 1) & ~1ull,
+                                 n_proj_slots_ * d, QUERY_ANY, 0);
+            else if (!slot_pools && pool_n_ > 0)
+                launch_query_set(qpool, pool_.as<uint64_t>(), pool_words_, ((pool_n_ + 63) / 64 + 1) & ~1ull, d,
+                                 QUERY_ANY, 0);
+            else
+                pool = false;
+            launch_query_set(qfhut, vrows_, vstride_, vwords_, vd_, QUERY_COUNT, 1, nullptr, &fhut_sup);
+            if (pool || qfhut.size()) h_->sync();
+            if (pool) collect_queries(qpool, 0, pool_hit);
+            else pool_hit.assign(qpool.size(), 0);
+            collect_queries(qfhut, 1, fhut_cnt);
+        });
         // ---- phase C: leaf and FHUT candidates, HUT, expanding nodes
         t_exp = Clock::now();
         const uint64_t pool_before = csup_.size();
@@ -875,8 +950,32 @@ int Miner::run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *use
         // extensions after it, and the first is searched first
         // (kids keeps its elements from wave to wave: they were moved to the stack, so
         // each is reset below; the spare vectors are handed out by position)
+        // A child's mask is its parent's AND its own item's row: the parent's is made here, for
+        // the expanding nodes alone (a mask per child was 22 ms of a 2,000,000-transaction search).
+        // The root's children have none: their own rows, or their projections once resident.
+        qchild.clear();
+        child_slot.clear();
+        for (size_t i = 0; i < wave.size(); ++i) {
+            Work &wk = work[i];
+            wk.kslot = kNoSlot;
+            const MNode &nd = wave[i];
+            if (wk.kind != 3 || wk.nkids < 2 || nd.head.empty()) continue;
+            if (nd.slot != kNoSlot && nd.piv == kNoItem) {
+                wk.kslot = nd.slot;
+            } else {
+                wk.kslot = alloc_slot();
+                if (wk.kslot == kNoSlot) continue;
+                if (nd.slot != kNoSlot) {
+                    const uint32_t e = prow(nd, nd.piv);
+                    qchild.add(&e, 1, nd.slot);
+                } else {
+                    add_query(qchild, nd, nd.head.data(), nd.head.size(), kNoSlot);
+                }
+                child_slot.push_back(wk.kslot);
+            }
+            slot_refs_[wk.kslot] += (uint32_t)wk.nkids - 1;   // the last child has no tail to count
+        }
         if (kids.size() < n_ext) kids.resize(n_ext);
-        kid_src.resize(n_ext);
         const uint64_t n_spare = std::min<uint64_t>(spare_.size() / 2, n_ext), sp0 = spare_.size() - 2 * n_spare;
         const uint64_t id0 = parent_.size(), tr0 = tnode_.size();
         parent_.resize(id0 + n_ext);
@@ -910,7 +1009,8 @@ int Miner::run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *use
                         c.head = std::move(spare_[sp0 + 2 * k]);
                         c.tail = std::move(spare_[sp0 + 2 * k + 1]);
                     }
-                    c.slot = kNoSlot;
+                    c.slot = p + 1 < nf ? wk.kslot : kNoSlot;
+                    c.piv = c.slot != kNoSlot ? wk.f[j].second : kNoItem;
                     c.head.assign(wk.head.begin(), wk.head.end());
                     c.head.push_back(wk.f[j].second);
                     c.sup = wk.f[j].first;
@@ -923,39 +1023,12 @@ int Miner::run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *use
                         std::copy_n(wfeat.data() + (wk.feat0 + j) * kDim, kDim, tfeat_.data() + (tr0 + k) * kDim);
                         tnode_[tr0 + k] = c.id;
                     }
-                    kid_src[k] = {nd.slot, wk.f[j].second};
                 }
             }
         });
         spare_.resize(sp0);
         add_since(6, t_exp);
-        // child masks for the children searched next: mask(child) = mask(parent) & row(e)
-        qchild.clear();
-        child_slot.clear();
-        for (size_t k = 0; k < n_ext; ++k) {
-            MNode &c = kids[k];
-            // leaves need no mask; a root child gets its mask once its projection is resident
-            if (c.tail.empty() || (use_proj_ && (c.proj == kNoProj || root_slot_[c.proj] < 0))) continue;
-            c.slot = alloc_slot();
-            if (c.slot == kNoSlot) continue;
-            if (kid_src[k].first != kNoSlot) {
-                const uint32_t e = prow(c, kid_src[k].second);
-                qchild.add(&e, 1, kid_src[k].first);
-            } else {
-                add_query(qchild, c, c.head.data(), c.head.size(), kNoSlot);
-            }
-            child_slot.push_back(c.slot);
-        }
-        if (qchild.size()) {
-            const size_t n = qchild.size();
-            const uint64_t *dptr = c_ptr_.put(qchild.ptr.data(), n + 1, st);
-            const uint32_t *ditems = c_items_.put(qchild.items.data(), qchild.items.size(), st);
-            const uint32_t *dps = c_ps_.put(qchild.slot.data(), n, st);
-            const uint32_t *dcs = c_cs_.put(child_slot.data(), n, st);
-            launch_child_masks(arena_.as<uint64_t>(), slot_words_, vwords_, vrows_, vstride_, dptr, ditems, dps,
-                               dcs, (uint32_t)n, st, h_->n_sm);
-            ++launches_;
-        }
+        launch_masks(qchild, child_slot);
         // the stack is LIFO: push in reverse so that the wave's first node's first
         // child is popped first
         t_exp = Clock::now();
@@ -971,10 +1044,11 @@ int Miner::run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *use
                     stack[sb + n_ext - 1 - k] = std::move(kids[k]);
                 }
             });
+            if (use_proj_ && wave_global) roots_left = stack.size();
         }
         // parents' masks are no longer needed once the child-mask kernel ran (stream order)
         for (MNode &nd : wave) {
-            if (nd.slot != kNoSlot) free_slots_.push_back(nd.slot);
+            if (nd.slot != kNoSlot) drop_slot(nd.slot);
             if (use_proj_ && nd.proj != kNoProj) --live_[nd.proj];
         }
         add_since(6, t_exp);

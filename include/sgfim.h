@@ -281,8 +281,9 @@ typedef struct {
     uint8_t *trace_labels;   /* trace_n */
     /* wall time of the search phases (each device phase ends in a stream
      * synchronisation, so device time of asynchronous launches is charged to
-     * the next phase): [0] extension counts, [1] pool (HUT / leaf) queries,
-     * [2] FHUT counts, [3] final maximality filter, [4] scoring, [5] the rest
+     * the next phase): [0] extension counts, [1] zero (the pool queries share a
+     * round trip with the FHUT counts), [2] pool (HUT / leaf) queries and FHUT
+     * counts, [3] final maximality filter, [4] scoring, [5] the rest
      * (wave assembly, staging, launches, checkpoints), [6] host expansion (PEP,
      * extension order, candidates, children), [7] result assembly after the
      * search */
