@@ -37,9 +37,13 @@ __device__ __forceinline__ float bf2f(uint16_t b) { return __uint_as_float(((uin
 //
 // Bound: shared memory (weights and activations of layer 1, the parts written
 // and read by the MMAs), about 3,800 clocks per tile of 128 rows at H = 128.
-// Measured (300,000 rows, H = 128, whole call): 74 us against 1,560 us for one
+// Measured (300,000 rows, H = 128, whole call): 68 us against 1,560 us for one
 // thread per hidden unit with scalar multiply-adds (a shared-memory load for each);
-// error against float64 5.0e-8 (5.3e-8 before).
+// error against float64 5.1e-8 (5.4e-8 before).  Of that, 6 us came from two-float
+// multiply-adds and the next tile's inputs fetched ahead.  What bounds it now is the
+// chain of a tile (about 15,000 clocks a CTA, of which 2,000 wait for MMAs) over
+// 16 warps an SM: layer 1 on the tensor cores too took a fifth of the instructions
+// out and gave 66 us, 32 warps an SM 72 us.
 constexpr uint32_t kFwdRows = 128;
 constexpr uint32_t kFwdThreads = 256;
 constexpr uint32_t kFwdPart = kFwdRows * 128;   // one part's atom: 128 rows x 64 bf16
@@ -72,6 +76,26 @@ inline FwdLayout mlp_fwd_layout(uint32_t F, uint32_t H, bool w2_resident) {
     return l;
 }
 
+// Two floats in one 64-bit register: Blackwell adds and multiplies them in one instruction.
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float &lo, float &hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
 // Eight consecutive non-negative values of row r -> their three bf16 parts, as
 // 16-byte piece c of the row in the three atoms.
 __device__ __forceinline__ void store_parts(uint8_t *a, uint32_t r, uint32_t c, const float (&h)[8]) {
@@ -80,16 +104,22 @@ __device__ __forceinline__ void store_parts(uint8_t *a, uint32_t r, uint32_t c, 
     for (int q = 0; q < 4; ++q) {
         uint32_t v[2] = {__float_as_uint(h[2 * q]), __float_as_uint(h[2 * q + 1])};
         p[0][q] = __byte_perm(v[0], v[1], 0x7632);
+        // what the top part leaves (a value minus its top part: an add of the negated part); an
+        // infinite value keeps its top part alone (inf - inf is NaN, whose maximum with 0 is 0)
+        auto rest = [](uint32_t (&x)[2]) {
+            float lo, hi;
+            unpack2(add2(pack2(__uint_as_float(x[0]), __uint_as_float(x[1])),
+                         pack2(__uint_as_float((x[0] & 0xffff0000u) | 0x80000000u),
+                               __uint_as_float((x[1] & 0xffff0000u) | 0x80000000u))),
+                    lo, hi);
+            x[0] = __float_as_uint(lo);
+            x[1] = __float_as_uint(hi);
+        };
+        rest(v);
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            // an infinite value keeps its top part alone (inf - inf is NaN, whose maximum with 0 is 0)
-            const float r1 = fmaxf(__uint_as_float(v[e]) - __uint_as_float(v[e] & 0xffff0000u), 0.f);
-            v[e] = __float_as_uint(r1);
-        }
+        for (int e = 0; e < 2; ++e) v[e] = __float_as_uint(fmaxf(__uint_as_float(v[e]), 0.f));
         p[1][q] = __byte_perm(v[0], v[1], 0x7632);
-#pragma unroll
-        for (int e = 0; e < 2; ++e)
-            v[e] = __float_as_uint(__uint_as_float(v[e]) - __uint_as_float(v[e] & 0xffff0000u));
+        rest(v);
         p[2][q] = __byte_perm(v[0], v[1], 0x7632);
     }
     uint8_t *dst = a + r * 128 + ((c ^ (r & 7)) << 4);
@@ -181,11 +211,29 @@ __global__ void __launch_bounds__(kFwdThreads) mlp_fwd_kernel(
     const uint32_t tiles = n / kFwdRows + (n % kFwdRows != 0);
     uint32_t parity = 0;
     bool ok = true;
+    // eight aligned inputs a row (the search's features): a 16-byte load per thread and tile, one
+    // tile ahead
+    const bool quad = F == 8 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
+    float4 xq = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto fetch_quad = [&](uint64_t tile) {
+        const uint64_t row = tile * kFwdRows + (tid >> 1);
+        xq = row < n ? __ldg(reinterpret_cast<const float4 *>(X + row * 8) + (tid & 1)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    if (quad) fetch_quad(blockIdx.x);
     for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const uint64_t r0 = (uint64_t)tile * kFwdRows;
-        for (uint32_t i = tid; i < kFwdRows * F; i += kFwdThreads) {
-            const uint32_t r = i / F, f = i - r * F;
-            xs[f * kFwdXs + r] = r0 + r < n ? X[r0 * F + i] : 0.f;
+        if (quad) {
+            const uint32_t r = tid >> 1, f = (tid & 1) * 4;
+            xs[f * kFwdXs + r] = xq.x;
+            xs[(f + 1) * kFwdXs + r] = xq.y;
+            xs[(f + 2) * kFwdXs + r] = xq.z;
+            xs[(f + 3) * kFwdXs + r] = xq.w;
+            fetch_quad(tile + gridDim.x);
+        } else {
+            for (uint32_t i = tid; i < kFwdRows * F; i += kFwdThreads) {
+                const uint32_t r = i / F, f = i - r * F;
+                xs[f * kFwdXs + r] = r0 + r < n ? X[r0 * F + i] : 0.f;
+            }
         }
         __syncthreads();
         const uint32_t p = tid & 63, cq = tid >> 6;
@@ -204,21 +252,33 @@ __global__ void __launch_bounds__(kFwdThreads) mlp_fwd_kernel(
                 const uint32_t jc = cq * 16 + g * 8;   // column of the chunk
                 if (jc >= cw) break;
                 const uint32_t j0 = kc * 64 + jc;
-                float z[2][8];
-#pragma unroll
-                for (int q = 0; q < 8; ++q) z[0][q] = z[1][q] = b1s[j0 + q];
+                uint64_t zz[2][4];   // rows p and p + 64, two units each
+                {
+                    const ulonglong2 ba = *reinterpret_cast<const ulonglong2 *>(b1s + j0);
+                    const ulonglong2 bb = *reinterpret_cast<const ulonglong2 *>(b1s + j0 + 4);
+                    zz[0][0] = zz[1][0] = ba.x;
+                    zz[0][1] = zz[1][1] = ba.y;
+                    zz[0][2] = zz[1][2] = bb.x;
+                    zz[0][3] = zz[1][3] = bb.y;
+                }
 #pragma unroll 4
                 for (uint32_t f = 0; f < F; ++f) {
-                    const float4 wa = *reinterpret_cast<const float4 *>(w1s + f * H + j0);
-                    const float4 wb = *reinterpret_cast<const float4 *>(w1s + f * H + j0 + 4);
-                    const float w[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+                    const ulonglong2 wa = *reinterpret_cast<const ulonglong2 *>(w1s + f * H + j0);
+                    const ulonglong2 wb = *reinterpret_cast<const ulonglong2 *>(w1s + f * H + j0 + 4);
+                    const uint64_t w[4] = {wa.x, wa.y, wb.x, wb.y};
                     const float x0 = xs[f * kFwdXs + p], x1 = xs[f * kFwdXs + p + 64];
+                    const uint64_t xx0 = pack2(x0, x0), xx1 = pack2(x1, x1);
 #pragma unroll
-                    for (int q = 0; q < 8; ++q) {
-                        z[0][q] = fmaf(w[q], x0, z[0][q]);
-                        z[1][q] = fmaf(w[q], x1, z[1][q]);
+                    for (int q = 0; q < 4; ++q) {
+                        zz[0][q] = fma2(w[q], xx0, zz[0][q]);
+                        zz[1][q] = fma2(w[q], xx1, zz[1][q]);
                     }
                 }
+                float z[2][8];
+#pragma unroll
+                for (int e = 0; e < 2; ++e)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) unpack2(zz[e][q], z[e][2 * q], z[e][2 * q + 1]);
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     const uint64_t row = r0 + p + 64 * e;
@@ -269,7 +329,7 @@ __global__ void __launch_bounds__(kFwdThreads) mlp_fwd_kernel(
         // layer 3: warp w reads the 32 rows of TMEM quadrant w % 4, columns half w / 4
         const uint32_t row_l = (warp & 3) * 32 + lane, half = warp >> 2, c0 = half * (H / 2);
         const uint64_t row = r0 + row_l;
-        float s[4] = {0.f, 0.f, 0.f, 0.f};
+        uint64_t s[2] = {0, 0};   // four sums
         for (uint32_t c = c0; c < c0 + H / 2; c += 16) {
             float z[16];
             if (!scalar) {
@@ -279,7 +339,10 @@ __global__ void __launch_bounds__(kFwdThreads) mlp_fwd_kernel(
                 tmem_ld16(d_low + lanes + c, l);
                 tmem_wait_ld();
 #pragma unroll
-                for (int q = 0; q < 16; ++q) z[q] = __uint_as_float(t[q]) + __uint_as_float(l[q]);
+                for (int q = 0; q < 16; q += 2)
+                    unpack2(add2(pack2(__uint_as_float(t[q]), __uint_as_float(t[q + 1])),
+                                 pack2(__uint_as_float(l[q]), __uint_as_float(l[q + 1]))),
+                            z[q], z[q + 1]);
             } else {
                 // non-finite weights: the plain sum, so that they meet the whole activation
 #pragma unroll 1
@@ -294,9 +357,13 @@ __global__ void __launch_bounds__(kFwdThreads) mlp_fwd_kernel(
                 }
             }
 #pragma unroll
-            for (int q = 0; q < 16; ++q) {
-                z[q] += b2s[c + q];
-                s[q & 3] = fmaf(w3s[c + q], fmaxf(z[q], 0.f), s[q & 3]);
+            for (int q = 0; q < 16; q += 4) {
+                const ulonglong2 b = *reinterpret_cast<const ulonglong2 *>(b2s + c + q);
+                const ulonglong2 w = *reinterpret_cast<const ulonglong2 *>(w3s + c + q);
+                unpack2(add2(pack2(z[q], z[q + 1]), b.x), z[q], z[q + 1]);
+                unpack2(add2(pack2(z[q + 2], z[q + 3]), b.y), z[q + 2], z[q + 3]);
+                s[0] = fma2(w.x, pack2(fmaxf(z[q], 0.f), fmaxf(z[q + 1], 0.f)), s[0]);
+                s[1] = fma2(w.y, pack2(fmaxf(z[q + 2], 0.f), fmaxf(z[q + 3], 0.f)), s[1]);
             }
             if (Z2 && row < n) {
                 float *dst = Z2 + row * H + c;
@@ -310,7 +377,10 @@ __global__ void __launch_bounds__(kFwdThreads) mlp_fwd_kernel(
                 }
             }
         }
-        red[half * kFwdRows + row_l] = (s[0] + s[1]) + (s[2] + s[3]);
+        float s0, s1, s2, s3;
+        unpack2(s[0], s0, s1);
+        unpack2(s[1], s2, s3);
+        red[half * kFwdRows + row_l] = (s0 + s1) + (s2 + s3);
         tc_fence_before();
         __syncthreads();
         tc_fence_after();

@@ -116,3 +116,47 @@ def test_forward_infinite_values(engine):
     fin = np.delete(np.arange(64), 9)
     w["W2"][9, 3] = 0
     assert np.abs(z2[:, fin] - _ref(w)["Z2"][:, fin]).max() < 1e-4 * np.abs(_ref(w)["Z2"]).max()
+
+
+@pytest.mark.parametrize("n,H", [(1, 32), (127, 64), (128, 96), (129, 128), (256, 32), (5000, 128)])
+def test_eight_inputs_shapes(engine, n, H):
+    """Eight aligned inputs a row are fetched a tile ahead: inputs of both signs and of magnitudes
+    from 1e-30 to 1e3."""
+    torch = pytest.importorskip("torch")
+    w = _net(torch, n, 8, H, n + H)
+    rng = np.random.default_rng(n)
+    w["X"] = (rng.uniform(-1, 1, (n, 8)) * 10.0 ** rng.choice([-30, -3, 0, 0, 0, 3], (n, 8))).astype(np.float32)
+    got, want = _run(torch, engine, w, backward=False), _ref(w)
+    # sums of at most 8 + H exact products: 400 * 2^-24 of the terms' magnitudes
+    t1 = np.abs(w["X"].astype(np.float64)) @ np.abs(w["W1"].astype(np.float64)).T + np.abs(w["b1"])
+    t2 = t1 @ np.abs(w["W2"].astype(np.float64)).T + np.abs(w["b2"])
+    assert (np.abs(got["Z1"].reshape(n, H) - want["Z1"]) <= 2.4e-5 * t1).all()
+    assert (np.abs(got["Z2"].reshape(n, H) - want["Z2"]) <= 2.4e-5 * t2).all()
+    t3 = t2 @ np.abs(w["w3"].astype(np.float64)) + np.abs(w["b3"])
+    assert (np.abs(got["P"] - want["P"]) <= 2.4e-5 * t3 / 4 + 1e-7).all()
+
+
+def test_eight_inputs_infinite_values(engine):
+    """Infinite and NaN inputs and an infinite layer-1 weight give what the plain sums give."""
+    torch = pytest.importorskip("torch")
+    w = _net(torch, 300, 8, 128, 9)
+    w["W1"] = np.where(w["W1"] == 0, np.float32(0.5), w["W1"])
+    w["X"][3, 1], w["X"][4, 6], w["X"][131, 0] = np.inf, -np.inf, np.nan
+    z1 = _run(torch, engine, w, backward=False)["Z1"].reshape(300, 128)
+    assert (z1[3] == np.inf * np.sign(w["W1"][:, 1])).all() and (z1[4] == -np.inf * np.sign(w["W1"][:, 6])).all()
+    assert np.isnan(z1[131]).all()
+    rest = np.delete(np.arange(300), [3, 4, 131])
+    want = _ref({k: (v[rest] if k in ("X", "Y", "WT") else v) for k, v in w.items()})["Z1"]
+    assert np.abs(z1[rest] - want).max() < 1e-4 * np.abs(want).max()
+    w = _net(torch, 300, 8, 128, 10)
+    w["X"] = np.abs(w["X"]) + np.float32(0.01)
+    w["W1"][17, 5] = -np.inf
+    got = _run(torch, engine, w, backward=False)
+    z1, z2 = got["Z1"].reshape(300, 128), got["Z2"].reshape(300, 128)
+    assert (z1[:, 17] == -np.inf).all()
+    fin = np.delete(np.arange(128), 17)
+    w["W1"][17] = 0
+    w["b1"][17] = -1                 # its activation is zero either way
+    want = _ref(w)
+    assert np.abs(z1[:, fin] - want["Z1"][:, fin]).max() < 1e-4 * np.abs(want["Z1"]).max()
+    assert np.abs(z2 - want["Z2"]).max() < 1e-4 * np.abs(want["Z2"]).max()
