@@ -229,6 +229,8 @@ struct sgfim_handle {
     sg::Scorer scorer;
     // scratch
     sg::DevBuf support_scratch, cand_ptr_dev, cand_items_dev, out_dev, dev_err;
+    sg::StagedPack support_in;   // a small call's candidates
+    sg::HostBuf support_out;     // its supports and the device error word
     sg::DevBuf cooc_scratch;
     sg::MinerWorkspace mws;
     sg::WindowWorkspace wws;
