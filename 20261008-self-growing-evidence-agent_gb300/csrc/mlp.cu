@@ -37,10 +37,11 @@ __device__ __forceinline__ float bf2f(uint16_t b) { return __uint_as_float(((uin
 //
 // Bound: shared memory (weights and activations of layer 1, the parts written
 // and read by the MMAs), about 3,800 clocks per tile of 128 rows at H = 128.
-// Measured (300,000 rows, H = 128, whole call): 68 us against 1,560 us for one
+// Measured (300,000 rows, H = 128, whole call): 64 us against 1,560 us for one
 // thread per hidden unit with scalar multiply-adds (a shared-memory load for each);
-// error against float64 5.1e-8 (5.4e-8 before).  Of that, 6 us came from two-float
-// multiply-adds and the next tile's inputs fetched ahead.  What bounds it now is the
+// error against float64 4.5e-8 (4.7e-8 before).  Of that, 6 us came from two-float
+// multiply-adds and the next tile's inputs fetched ahead, 4 from reading W2 once, its
+// loads in flight together.  What bounds it now is the
 // chain of a tile (about 15,000 clocks a CTA, of which 2,000 wait for MMAs) over
 // 16 warps an SM: layer 1 on the tensor cores too took a fifth of the instructions
 // out and gave 66 us, 32 warps an SM 72 us.
@@ -141,14 +142,19 @@ __device__ __forceinline__ bool bf2_nonfinite(uint32_t w) {
     return (w & 0x7f80u) == 0x7f80u || (w & 0x7f800000u) == 0x7f800000u;
 }
 
-// K chunk kc of W2 as a swizzled K-major atom of H rows x 64 columns.
-__device__ __forceinline__ void load_w2_chunk(uint8_t *dst, const uint16_t *W2, uint32_t H, uint32_t kc, bool aligned) {
-    const uint32_t pieces = min(64u, H - kc * 64) / 8;
+// K chunk kc of W2 as a swizzled K-major atom of H rows x 64 columns; true when
+// this thread met an infinite or NaN weight.
+__device__ __forceinline__ bool load_w2_chunk(uint8_t *dst, const uint16_t *W2, uint32_t H, uint32_t kc, bool aligned) {
+    const uint32_t shift = H - kc * 64 >= 64 ? 3 : 2, pieces = 1u << shift;   // H is a multiple of 32
+    bool odd = false;
+#pragma unroll 4
     for (uint32_t i = threadIdx.x; i < H * pieces; i += kFwdThreads) {
-        const uint32_t j = i / pieces, c = i - j * pieces;
-        *reinterpret_cast<uint4 *>(dst + j * 128 + ((c ^ (j & 7)) << 4)) =
-            load_w8(W2 + (size_t)j * H + kc * 64 + c * 8, aligned);
+        const uint32_t j = i >> shift, c = i & (pieces - 1);
+        const uint4 w = load_w8(W2 + (size_t)j * H + kc * 64 + c * 8, aligned);
+        odd |= bf2_nonfinite(w.x) || bf2_nonfinite(w.y) || bf2_nonfinite(w.z) || bf2_nonfinite(w.w);
+        *reinterpret_cast<uint4 *>(dst + j * 128 + ((c ^ (j & 7)) << 4)) = w;
     }
+    return odd;
 }
 
 __device__ __forceinline__ void mma_bf16(uint32_t tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
@@ -163,7 +169,7 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem, uint64_t adesc, uint64_t
 // Z1/Z2 (pre-activations) are written when non-null (training); vec: both
 // allow 16-byte stores.  tm_cols: allocated TMEM columns (the two accumulators
 // are its halves).
-__global__ void __launch_bounds__(kFwdThreads) mlp_fwd_kernel(
+__global__ void __launch_bounds__(kFwdThreads, 2) mlp_fwd_kernel(
     const float *__restrict__ X, uint32_t n, uint32_t F, uint32_t H, const uint16_t *__restrict__ W1,
     const float *__restrict__ b1, const uint16_t *__restrict__ W2, const float *__restrict__ b2,
     const uint16_t *__restrict__ w3, const float *__restrict__ b3, float *__restrict__ Z1, float *__restrict__ Z2,
@@ -195,12 +201,15 @@ __global__ void __launch_bounds__(kFwdThreads) mlp_fwd_kernel(
         w3s[i] = bf2f(w3[i]);
     }
     bool odd = false;   // an infinite or NaN weight: 0 parts times it would be NaN
-    for (uint32_t i = tid; i < H * H / 8; i += kFwdThreads) {
-        const uint4 w = load_w8(W2 + (size_t)i * 8, w2_aligned);
-        odd |= bf2_nonfinite(w.x) || bf2_nonfinite(w.y) || bf2_nonfinite(w.z) || bf2_nonfinite(w.w);
+    if (lay.w2_resident) {
+        for (uint32_t kc = 0; kc < chunks; ++kc) odd |= load_w2_chunk(sm + kc * H * 128, W2, H, kc, w2_aligned);
+    } else {
+#pragma unroll 8
+        for (uint32_t i = tid; i < H * H / 8; i += kFwdThreads) {
+            const uint4 w = load_w8(W2 + (size_t)i * 8, w2_aligned);
+            odd |= bf2_nonfinite(w.x) || bf2_nonfinite(w.y) || bf2_nonfinite(w.z) || bf2_nonfinite(w.w);
+        }
     }
-    if (lay.w2_resident)
-        for (uint32_t kc = 0; kc < chunks; ++kc) load_w2_chunk(sm + kc * H * 128, W2, H, kc, w2_aligned);
     tc_fence_before();
     const bool scalar = __syncthreads_or(odd);
     tc_fence_after();
@@ -413,10 +422,13 @@ __global__ void __launch_bounds__(kFwdThreads) mlp_fwd_kernel(
 // (T = 64 for H <= 64, else 128; nb = ceil(H / T).)  The dW2 atomics are
 // 16-byte vectors of consecutive columns, so a warp's instruction covers whole
 // sectors.
-// Measured (4,096 rows, H = 128, forward, backward and their fills): 66 us a
-// call, the host's launches, against 150 us with 256 CTAs whose threads each
+// Bound: latency (one batch of rows a CTA), so every load of a batch is in flight at
+// once; loads in loops of four and weights two bytes at a time took 35 us at 4,096
+// rows and H = 128, now 23.
+// Measured (4,096 rows, H = 128, forward, backward and their fills): 63 us a
+// call, the host's launches, against 145 us with 256 CTAs whose threads each
 // added single dW2 columns 512 bytes apart; gradients' error against float64
-// 3.9e-7 (1.2e-6 before).
+// 2.8e-7 (1.2e-6 before).
 constexpr int kBwdRows = 32;
 constexpr int kBwdThreads = 256;
 
@@ -454,6 +466,7 @@ template <int T, int KF> __global__ void __launch_bounds__(kBwdThreads) mlp_bwd_
     __shared__ float dz3[kBwdRows];
     const uint32_t tid = threadIdx.x, H = g.H, nb = (H + T - 1) / T;
     constexpr uint32_t kCols = kBwdThreads / T;   // threads sharing a column
+    constexpr uint32_t kMine = kBwdRows / kCols;  // rows of a batch per thread
     const uint32_t col = tid % T, part = tid / T;
     float *dz2 = sm;   // [32][T]
     if (blockIdx.y < nb * nb) {
@@ -471,20 +484,23 @@ template <int T, int KF> __global__ void __launch_bounds__(kBwdThreads) mlp_bwd_
         float gw3 = 0.f, gb2 = 0.f, gb3 = 0.f, loss = 0.f;
         for (uint32_t b = blockIdx.x; b < g.batches; b += gridDim.x) {
             const uint64_t r0 = (uint64_t)b * kBwdRows;
+            float z1s[kMine], z2s[kMine];   // this thread's rows of its column, all on their way at once
+#pragma unroll
+            for (uint32_t m = 0; m < kMine; ++m) {
+                const uint64_t row = r0 + part + m * kCols;
+                z2s[m] = row < g.n && j < H ? g.Z2[row * H + j] : 0.f;
+                z1s[m] = row < g.n && i < H ? g.Z1[row * H + i] : 0.f;
+            }
             __syncthreads();
             if (tid < kBwdRows) {
                 loss += bwd_dz3(g, r0 + tid, dz3);
                 gb3 += dz3[tid];
             }
             __syncthreads();
-#pragma unroll 4
-            for (uint32_t r = part; r < kBwdRows; r += kCols) {
-                const uint64_t row = r0 + r;
-                float z1 = 0.f, z2 = 0.f;
-                if (row < g.n) {
-                    if (j < H) z2 = g.Z2[row * H + j];
-                    if (i < H) z1 = g.Z1[row * H + i];
-                }
+#pragma unroll
+            for (uint32_t m = 0; m < kMine; ++m) {
+                const uint32_t r = part + m * kCols;
+                const float z1 = z1s[m], z2 = z2s[m];
                 const float d = dz3[r];
                 const float g2 = z2 > 0.f ? d * wj3 : 0.f;
                 gw3 = fmaf(d, fmaxf(z2, 0.f), gw3);
@@ -548,6 +564,7 @@ template <int T, int KF> __global__ void __launch_bounds__(kBwdThreads) mlp_bwd_
     float *w2 = sm + kBwdRows * T;          // [T (out)][T (in)] of the current output block
     float *xs = w2 + T * T;                 // [32][F]
     float *g1 = dz2;                        // [32][T], once dz2 has been read
+    const bool w2_aligned = (reinterpret_cast<uintptr_t>(g.W2) & 15) == 0;
     constexpr int R = kBwdRows * T / kBwdThreads / 4;   // rows per thread, four columns each
     constexpr uint32_t kQuads = T / 4;
     const uint32_t iq = (tid % kQuads) * 4, rg = (tid / kQuads) * R;
@@ -556,6 +573,15 @@ template <int T, int KF> __global__ void __launch_bounds__(kBwdThreads) mlp_bwd_
     for (int k = 0; k < KF; ++k) gw[k] = 0.f;
     for (uint32_t b = blockIdx.x; b < g.batches; b += gridDim.x) {
         const uint64_t r0 = (uint64_t)b * kBwdRows;
+        float z1s[R][4];
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint64_t row = r0 + rg + r;
+                const uint32_t i = bi * T + iq + q;
+                z1s[r][q] = row < g.n && i < H ? g.Z1[row * H + i] : 0.f;
+            }
         __syncthreads();
         if (tid < kBwdRows) bwd_dz3(g, r0 + tid, dz3);
         for (uint32_t k = tid; k < kBwdRows * g.F; k += kBwdThreads)
@@ -566,20 +592,39 @@ template <int T, int KF> __global__ void __launch_bounds__(kBwdThreads) mlp_bwd_
 #pragma unroll
             for (int q = 0; q < 4; ++q) acc[r][q] = 0.f;
         for (uint32_t bj = 0; bj < nb; ++bj) {
-            __syncthreads();
             const uint32_t j = bj * T + col;
             const float wj3 = j < H ? bf2f(g.w3[j]) : 0.f;
-#pragma unroll 4
-            for (uint32_t r = part; r < kBwdRows; r += kCols) {
-                const uint64_t row = r0 + r;
-                const float z2 = row < g.n && j < H ? g.Z2[row * H + j] : 0.f;
-                dz2[r * T + col] = z2 > 0.f ? dz3[r] * wj3 : 0.f;
+            float z2s[kMine];
+#pragma unroll
+            for (uint32_t m = 0; m < kMine; ++m) {
+                const uint64_t row = r0 + part + m * kCols;
+                z2s[m] = row < g.n && j < H ? g.Z2[row * H + j] : 0.f;
             }
-            if (nb > 1 || b == blockIdx.x)
-                for (uint32_t k = part; k < (uint32_t)T; k += kCols) {
-                    const uint32_t o = bj * T + k, i = bi * T + col;
-                    w2[k * T + col] = o < H && i < H ? bf2f(g.W2[(size_t)o * H + i]) : 0.f;
+            __syncthreads();
+            if (nb > 1 || b == blockIdx.x) {
+                constexpr uint32_t kPieces = T * T / 8 / kBwdThreads, kRow = T / 8;   // eight weights a piece
+                uint4 w[kPieces];
+#pragma unroll
+                for (uint32_t x = 0; x < kPieces; ++x) {
+                    const uint32_t at = tid + x * kBwdThreads, o = bj * T + at / kRow, i = bi * T + at % kRow * 8;
+                    w[x] = o < H && i < H ? load_w8(g.W2 + (size_t)o * H + i, w2_aligned) : make_uint4(0, 0, 0, 0);
                 }
+#pragma unroll
+                for (uint32_t x = 0; x < kPieces; ++x) {
+                    const uint32_t v[4] = {w[x].x, w[x].y, w[x].z, w[x].w};
+                    float *dst = w2 + (size_t)(tid + x * kBwdThreads) * 8;
+#pragma unroll
+                    for (int q = 0; q < 4; q += 2)
+                        *reinterpret_cast<float4 *>(dst + 2 * q) =
+                            make_float4(__uint_as_float(v[q] << 16), __uint_as_float(v[q] & 0xffff0000u),
+                                        __uint_as_float(v[q + 1] << 16), __uint_as_float(v[q + 1] & 0xffff0000u));
+                }
+            }
+#pragma unroll
+            for (uint32_t m = 0; m < kMine; ++m) {
+                const uint32_t r = part + m * kCols;
+                dz2[r * T + col] = z2s[m] > 0.f ? dz3[r] * wj3 : 0.f;
+            }
             __syncthreads();
             // every column of a padded block is zero on the dz2 side
 #pragma unroll 2
@@ -605,15 +650,9 @@ template <int T, int KF> __global__ void __launch_bounds__(kBwdThreads) mlp_bwd_
         __syncthreads();
         // the ReLU of layer 1
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const uint64_t row = r0 + rg + r;
+        for (int r = 0; r < R; ++r)
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const uint32_t i = bi * T + iq + q;
-                const float z1 = row < g.n && i < H ? g.Z1[row * H + i] : 0.f;
-                g1[(rg + r) * T + iq + q] = z1 > 0.f ? acc[r][q] : 0.f;
-            }
-        }
+            for (int q = 0; q < 4; ++q) g1[(rg + r) * T + iq + q] = z1s[r][q] > 0.f ? acc[r][q] : 0.f;
         __syncthreads();
 #pragma unroll 4
         for (int r = 0; r < kBwdRows; ++r) {

@@ -52,7 +52,10 @@ class Trainer:
             "b3": np.zeros(1),
         }
         self.p = {k: torch.tensor(v, dtype=torch.float32, device=self.dev).contiguous() for k, v in init.items()}
-        self.g = {k: torch.zeros_like(v) for k, v in self.p.items()}
+        # the gradients are slices of one buffer (64-float boundaries), cleared by one launch per step
+        ends = np.cumsum([0] + [(v.numel() + 63) // 64 * 64 for v in self.p.values()])
+        self._g_all = torch.zeros(int(ends[-1]), dtype=torch.float32, device=self.dev)
+        self.g = {k: self._g_all[int(o):int(o) + v.numel()].view(v.shape) for (k, v), o in zip(self.p.items(), ends)}
         self.m = {k: torch.zeros_like(v) for k, v in self.p.items()}
         self.v = {k: torch.zeros_like(v) for k, v in self.p.items()}
         self.b16 = {k: torch.zeros(v.shape, dtype=torch.int16, device=self.dev) for k, v in self.p.items()
@@ -89,7 +92,7 @@ class Trainer:
         WT = WT.to(self.dev, torch.float32).contiguous() if WT is not None else None
         n = X.shape[0]
         P, Z1, Z2 = self.forward(X, keep=True)
-        torch._foreach_zero_(list(self.g.values()))
+        self._g_all.zero_()
         loss = torch.zeros(1, dtype=torch.float32, device=self.dev)
         self.eng.mlp_backward(X.data_ptr(), n, self.in_dim, self.hidden, self.b16["W2"].data_ptr(),
                               self.b16["w3"].data_ptr(), Z1.data_ptr(), Z2.data_ptr(), P.data_ptr(), Y.data_ptr(),
