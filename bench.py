@@ -15,10 +15,14 @@ Prints one JSON line (rank 0).  ``value`` is supports/s with inputs resident
 in HBM (CUDA events on the launching stream, L2 flushed by a 512 MiB write
 before every step); ``e2e`` is the same metric through the C ABI with pinned
 host buffers (bitmaps and candidates copied in, supports copied out, every
-step).  ``roofline`` relates the counting kernel's algorithmic bytes (k * N / 8
-per candidate, all read from shared memory once TMA has staged a chunk) to the
-shared-memory bandwidth (SMs x 128 B/clk x the SM clock sampled during the
-timed region); the HBM ratio and the DRAM traffic are kept beside it.
+step).  ``roofline`` relates the shared-memory
+bytes that the counting kernel moves (its profiled wavefronts; the algorithmic
+k * N / 8 per candidate where no profile is committed) to the shared-memory
+bandwidth (SMs x 128 B/clk x the SM clock sampled during the timed region).
+The default kernel ANDs a pair of rows once for all candidates that share it
+and reads further rows only where bits are left, so it moves fewer than the
+algorithmic bytes, whose rate, the HBM ratio and the DRAM traffic are kept
+beside it.
 ``cpu_baseline`` times the CPU oracle (a restatement of the reference's
 counting loop, kernel_bitmap.cu:390-408) on every host core;
 ``cpu_baseline_numpy`` times the reference's numpy AND + byte-LUT popcount
@@ -55,9 +59,9 @@ WORKLOAD = dict(name="support-1m", n_txn=1 << 20, d=1024, n_regimes=16, dens_lo=
 METRIC = "supports/s (frac of HBM peak)"
 UNIT = "supports/s"
 SMEM_BYTES_PER_CLK = 128        # shared-memory bandwidth of one SM (32 banks x 4 B)
-KERNEL_NAMES = {"auto": "k1_lane_tm_kernel", "lane_tm": "k1_lane_tm_kernel", "lane": "k1_lane_kernel",
+KERNEL_NAMES = {"auto": "pair_lane_kernel", "pair": "pair_lane_kernel", "lane_tm": "k1_lane_tm_kernel", "lane": "k1_lane_kernel",
                 "sorted": "k1_sorted_kernel", "staged": "k1_staged_kernel", "staged4": "k1_staged4_kernel",
-                "stream": "query_kernel"}
+                "stream": "cand_stream_kernel"}
 LEARNED_WEIGHTS = os.path.join(ROOT, "20261008-self-growing-evidence-agent_gb300", "sgfim", "data",
                                "scorer_weights.npz")
 
@@ -110,7 +114,8 @@ def measured_peaks():
 
 def ncu_traffic(kernel):
     """DRAM bytes per launch of the counting kernel from the committed ncu summary
-    (a one-pass capture of this workload: dram__bytes_read.sum + dram__bytes_write.sum)."""
+    (a capture of this workload: dram__bytes_read.sum + dram__bytes_write.sum), and where
+    given its shared-memory wavefronts of 128 bytes."""
     path = os.path.join(ROOT, "profiles", f"{kernel}_support-1m.json")
     if os.path.exists(path):
         with open(path) as f:
@@ -512,20 +517,23 @@ def main():
     k = np.diff(cp).astype(np.int64)
     alg_bytes = float(k.sum()) * (wr * 64 / 8.0)
     count_ms = ps["count_ms"] / max(1, ps["calls"])
-    achieved = alg_bytes / (count_ms / 1000.0) / 1e9
+    alg_rate = alg_bytes / (count_ms / 1000.0) / 1e9
     n_sm = torch.cuda.get_device_properties(dev).multi_processor_count
     sm_mhz = clocks["sm_mhz"] or peaks.get("sm_max_mhz", 2070.0)
     smem_peak = n_sm * SMEM_BYTES_PER_CLK * sm_mhz * 1e6 / 1e9
     kname = KERNEL_NAMES[args.kernel]
     tr = ncu_traffic(kname.replace("_kernel", ""))
     traffic = tr["dram_bytes_per_launch"] if tr else None
+    moved = tr["shared_wavefronts_per_launch"] * SMEM_BYTES_PER_CLK if tr and "shared_wavefronts_per_launch" in tr else None
+    achieved = moved / (count_ms / 1000.0) / 1e9 if moved else alg_rate
     roofline = {"bound": "smem", "achieved": achieved, "peak": smem_peak, "unit": "GB/s", "frac": achieved / smem_peak,
                 "traffic": traffic,
                 "peak_source": f"{n_sm} SMs x {SMEM_BYTES_PER_CLK} B/clk x {sm_mhz:.0f} MHz "
                                f"({'median SM clock sampled in the timed region' if clocks['sm_mhz'] else 'max SM clock'})",
                 "kernel": kname, "kernel_ms": count_ms, "alg_bytes_per_launch": alg_bytes,
+                "shared_bytes_per_launch": moved, "alg_gbs": alg_rate,
                 "hbm": {"peak_gbs": peaks["hbm_gbs"], "peak_source": peak_src,
-                        "alg_bytes_over_hbm_peak": achieved / peaks["hbm_gbs"],
+                        "alg_bytes_over_hbm_peak": alg_rate / peaks["hbm_gbs"],
                         "dram_traffic_gbs": (traffic / (count_ms / 1000.0) / 1e9) if traffic else None,
                         "dram_frac": (traffic / (count_ms / 1000.0) / 1e9 / peaks["hbm_gbs"]) if traffic else None,
                         "note": "each staged chunk is read from shared memory by every candidate that holds one "
@@ -567,8 +575,9 @@ def main():
     # the 1,024 x 1,024 co-occurrence matrix of the same bitmaps (every kernel kind)
     cooc = {}
     if not args.no_cooc and world == 1:
-        t_co = {k: torch.zeros(d * d, dtype=torch.int32, device=dev) for k in (1, 2, 3, 4)}
-        for kind, name in ((1, "popc"), (2, "bmma_b1"), (3, "tcgen05_e4m3"), (4, "tcgen05_e4m3_256")):
+        t_co = {k: torch.zeros(d * d, dtype=torch.int32, device=dev) for k in (1, 2, 3, 4, 5)}
+        for kind, name in ((1, "popc"), (2, "bmma_b1"), (3, "tcgen05_e4m3"), (4, "tcgen05_e4m3_256"),
+                           (5, "tcgen05_mxf4")):
             for _ in range(2):
                 eng.cooccurrence_device(t_bm.data_ptr(), d, n_words, n_words, t_co[kind].data_ptr(), kind,
                                         stream.cuda_stream)
@@ -586,7 +595,7 @@ def main():
             ms_c = statistics.median(times)
             bitops = float(d) * d * WORKLOAD["n_txn"]
             cooc[name] = {"ms": ms_c, "tbitops": bitops / (ms_c / 1000.0) / 1e12}
-        cooc["kinds_agree"] = bool(all(torch.equal(t_co[1], t_co[k]) for k in (2, 3, 4)))
+        cooc["kinds_agree"] = bool(all(torch.equal(t_co[1], t_co[k]) for k in (2, 3, 4, 5)))
 
     cpu = cpu_np = None
     gpu_sup = t_out.cpu().numpy().view(np.uint32)
