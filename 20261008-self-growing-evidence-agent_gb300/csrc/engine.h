@@ -7,6 +7,7 @@
 
 #include <cstring>
 #include <new>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -176,6 +177,7 @@ struct MinerWorkspace {
     HostBuf hq_out[2], hscore, ht_out;
     StagedPack queries[2], counts, masks, append, sappend;
     Staged feat, p_items_list[16];
+    std::shared_ptr<void> host;   // the miner's host storage
     void release() {
         for (DevBuf *b : {&arena, &pool, &q_out[0], &q_out[1], &score, &cooc, &t_out, &pdb, &pofs, &plist, &spool})
             b->release();
@@ -183,6 +185,7 @@ struct MinerWorkspace {
         for (StagedPack *s : {&queries[0], &queries[1], &counts, &masks, &append, &sappend}) s->release();
         feat.release();
         for (Staged &s : p_items_list) s.release();
+        host.reset();
     }
 };
 

@@ -46,6 +46,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <deque>
 #include <memory>
 #include <numeric>
 #include <thread>
@@ -70,17 +71,68 @@ constexpr uint32_t kProjSlots = 16;   // MinerWorkspace::p_items_list has one li
 constexpr uint32_t kWaveRoots = 8;    // root subtrees of a wave; the other slots take the next ones meanwhile
 constexpr uint32_t kDim = SGFIM_TRACE_DIM;
 
+// What the children of an expanded node share: its head (after PEP), then its
+// frequent tail in the order's sequence.  Kept while a child is on the stack or in
+// the wave; reused with its storage afterwards.
+struct Rec {
+    std::vector<uint32_t> data;  // dense ids
+    uint32_t nh = 0, nf = 0;     // head, tail
+    uint32_t refs = 0;           // children left
+};
+
+// An item and its support in a node's context, ascending by (support, item); one word,
+// so that sorting compares it at once.
+struct Ext {
+    uint64_t key;
+    Ext(uint32_t sup, uint32_t item) : key((uint64_t)sup << 32 | item) {}
+    uint32_t sup() const { return (uint32_t)(key >> 32); }
+    uint32_t item() const { return (uint32_t)key; }
+    bool operator<(const Ext &o) const { return key < o.key; }
+};
+
+// Child pos of a record: its head is the record's and the tail item pos, its tail the
+// items after that one.  The root has no item and the whole tail.
 struct MNode {
-    std::vector<uint32_t> head;  // dense ids
-    std::vector<uint32_t> tail;  // dense ids, in the order's sequence
+    Rec *rec = nullptr;
+    uint32_t pos = kNoItem;
     uint32_t sup = 0;
-    // tidset mask: slot's (its own) or, with a pivot, slot's (its parent's) AND the pivot's row;
+    // tidset mask: slot's, its own, or without `own` its parent's AND its item's row;
     // kNoSlot = AND of head rows
     uint32_t slot = kNoSlot;
-    uint32_t piv = kNoItem;
+    uint32_t own = 0;
     uint32_t id = 0;             // search-tree node id
     uint32_t proj = kNoProj;     // root item whose projected database the node's masks live in
+    bool is_root() const { return pos == kNoItem; }
+    uint32_t item() const { return rec->data[rec->nh + pos]; }
+    const uint32_t *tail() const { return rec->data.data() + rec->nh + (uint32_t)(pos + 1); }
+    uint32_t n_tail() const { return rec->nf - (uint32_t)(pos + 1); }
+    void head(std::vector<uint32_t> &out) const {
+        out.assign(rec->data.begin(), rec->data.begin() + rec->nh);
+        if (!is_root()) out.push_back(item());
+    }
 };
+
+// A wave node's bookkeeping.
+struct Work {
+    std::vector<uint32_t> head;                    // after PEP
+    std::vector<Ext> f;                            // frequent extensions, ascending
+    std::vector<uint32_t> pq, fq;                  // pool query (rarest row first), FHUT query rows
+    int kind = 0;                                  // 0 leaf, 1 internal, 2 pruned or FHUT, 3 expands
+    int emit = 0;                                  // a candidate: head (leaf) or head u F (FHUT)
+    size_t pool_q = 0, fhut_q = 0, fi0 = 0;        // its queries; fi0: its FHUT rows' offset
+    size_t e0 = 0, ei0 = 0;                        // its candidate's index and item offset in the wave
+    size_t feat0 = 0;                              // first feature row of its extensions
+    size_t kid0 = 0, nkids = 0;                    // range in the wave's kid list
+    uint32_t kslot = kNoSlot;                      // the mask its children start from
+    Rec *rec = nullptr;                            // its children's record
+};
+
+// Host storage kept by the handle from call to call: a search of a few waves would
+// spend more on allocating its nodes' lists than on filling them.
+struct MinerHost {
+    std::vector<Work> work;
+};
+constexpr size_t kKeptWork = 4096;   // wave nodes whose lists are kept between calls
 
 struct QuerySet {
     std::vector<uint64_t> ptr{0};
@@ -114,7 +166,16 @@ class Miner {
   public:
     Miner(sgfim_handle *h, const sgfim_mine_params &p)
         : h_(h), ds_(h->ds), p_(p), w_(h->mws), arena_(w_.arena), pool_(w_.pool), feat_(w_.feat),
-          score_(w_.score), hscore_(w_.hscore) {}
+          score_(w_.score), hscore_(w_.hscore) {
+        if (!w_.host) w_.host = std::make_shared<MinerHost>();
+        host_ = std::static_pointer_cast<MinerHost>(w_.host);
+    }
+    ~Miner() {
+        if (host_->work.size() > kKeptWork) {
+            host_->work.resize(kKeptWork);
+            host_->work.shrink_to_fit();
+        }
+    }
 
     int run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *user, sgfim_result **out);
 
@@ -123,6 +184,7 @@ class Miner {
     Dataset &ds_;
     sgfim_mine_params p_;
     MinerWorkspace &w_;
+    std::shared_ptr<MinerHost> host_;
     uint32_t thr_ = 1;
     Clock::time_point t0_;
     // tidset masks (slots of the workspace arena)
@@ -202,8 +264,18 @@ class Miner {
     // host threads on large datasets; one (the caller) on small ones, whose waves
     // are small and whose callers may run many miners at once (one per window)
     std::unique_ptr<HostPool> hp_;
-    // vectors of finished nodes, reused for new children (no allocation per node once warm)
-    std::vector<std::vector<uint32_t>> spare_;
+    // records of expanded nodes, and those that no child uses any more
+    std::deque<Rec> recs_;
+    std::vector<Rec *> free_recs_;
+    Rec *new_rec() {
+        if (free_recs_.empty()) {
+            recs_.emplace_back();
+            return &recs_.back();
+        }
+        Rec *r = free_recs_.back();
+        free_recs_.pop_back();
+        return r;
+    }
     std::vector<uint64_t> cand_freq_;   // candidates holding each dense item (pool row density)
     double phase_[8] = {0, 0, 0, 0, 0, 0, 0, 0};   // see sgfim_result.phase_s
     // adds the wall time of f() to phase_[i]
@@ -521,8 +593,9 @@ bool Miner::make_resident(const MNode &nd) {
     if (slot_root_[slot] != kNoProj) root_slot_[slot_root_[slot]] = -1;
     cudaStream_t st = h_->stream;
     const uint32_t r = nd.proj;
-    std::vector<uint32_t> items(nd.head.begin(), nd.head.end());
-    items.insert(items.end(), nd.tail.begin(), nd.tail.end());
+    std::vector<uint32_t> items;
+    nd.head(items);
+    items.insert(items.end(), nd.tail(), nd.tail() + nd.n_tail());
     const uint32_t *ditems = w_.p_items_list[slot].put(items.data(), items.size(), st);
     // the listed rows are cleared whole: a wave reads up to its widest projection, so
     // a row must be zero past its own projection's words (other rows are not read)
@@ -620,7 +693,10 @@ int Miner::run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *use
     std::vector<MNode> stack;
     if (!freq.empty()) {
         MNode root;
-        root.tail = freq;
+        root.rec = new_rec();
+        root.rec->data = freq;
+        root.rec->nf = (uint32_t)freq.size();
+        root.rec->refs = 1;
         root.sup = (uint32_t)ds_.n_txn;
         root.id = 0;
         parent_.push_back(kNoNode);
@@ -638,37 +714,11 @@ int Miner::run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *use
     std::vector<float> wfeat, wscore;
     int status = SGFIM_OK;
 
-    struct Work {
-        std::vector<uint32_t> head;                    // after PEP
-        std::vector<std::pair<uint32_t, uint32_t>> f;  // (support, item), ascending
-        std::vector<uint32_t> pq, fq;                  // pool query (rarest row first), FHUT query rows
-        int kind = 0;                                  // 0 leaf, 1 internal, 2 pruned or FHUT, 3 expands
-        int emit = 0;                                  // a candidate: head (leaf) or head u F (FHUT)
-        size_t pool_q = 0, fhut_q = 0, fi0 = 0;        // its queries; fi0: its FHUT rows' offset
-        size_t e0 = 0, ei0 = 0;                        // its candidate's index and item offset in the wave
-        size_t feat0 = 0;                              // first feature row of its extensions
-        size_t kid0 = 0, nkids = 0;                    // range in the wave's kid list
-        uint32_t kslot = kNoSlot;                      // the mask its children start from
-    };
-    std::vector<Work> work;
-    std::vector<MNode> kids;
+    std::vector<Work> &work = host_->work;
     std::vector<uint32_t> child_slot;
 
     while (!stack.empty()) {
         // ---- pop a wave
-        // the previous wave's nodes are done: keep their vectors for the next children
-        {
-            const size_t s0 = spare_.size();
-            spare_.resize(s0 + 2 * wave.size());
-            hp_->run(wave.size(), 2048, [&](uint64_t lo, uint64_t hi) {
-                for (uint64_t i = lo; i < hi; ++i) {
-                    wave[i].head.clear();
-                    wave[i].tail.clear();
-                    spare_[s0 + 2 * i] = std::move(wave[i].head);
-                    spare_[s0 + 2 * i + 1] = std::move(wave[i].tail);
-                }
-            });
-        }
         wave.clear();
         uint64_t nq = 0;
         bool wave_global = !use_proj_;
@@ -690,10 +740,10 @@ int Miner::run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *use
                     wave_words = std::max(wave_words, wp_[top.proj]);
                 }
             }
-            const uint64_t w = stack.back().tail.size();
+            const uint64_t w = stack.back().n_tail();
             if (!wave.empty() && nq + w > qmax) break;
             nq += w;
-            wave.push_back(std::move(stack.back()));
+            wave.push_back(stack.back());
             stack.pop_back();
         }
         if (wave_global) {
@@ -711,13 +761,14 @@ int Miner::run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *use
         qchild.clear();
         child_slot.clear();
         for (MNode &nd : wave) {
-            if (nd.slot != kNoSlot || nd.head.empty() || nd.tail.size() < 2) continue;
+            if (nd.slot != kNoSlot || nd.is_root() || nd.n_tail() < 2) continue;
             const uint32_t s = alloc_slot();
             if (s == kNoSlot) break;
-            add_query(qchild, nd, nd.head.data(), nd.head.size(), kNoSlot);
+            nd.head(tmp);
+            add_query(qchild, nd, tmp.data(), tmp.size(), kNoSlot);
             child_slot.push_back(s);
             nd.slot = s;
-            nd.piv = kNoItem;
+            nd.own = 1;
             slot_refs_[s] = 1;
         }
         launch_masks(qchild, child_slot);
@@ -734,16 +785,17 @@ int Miner::run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *use
             const MNode &nd = wave[i];
             if (nd.slot != kNoSlot) {
                 count_src[i] = {0, n_ti};
-                if (nd.tail.empty()) continue;
-                n_ti += nd.tail.size();
+                if (nd.n_tail() == 0) continue;
+                n_ti += nd.n_tail();
                 t_ptr.push_back(n_ti);
                 t_slot.push_back(nd.slot);
-                t_piv.push_back(nd.piv == kNoItem ? kNoSlot : prow(nd, nd.piv));
+                t_piv.push_back(nd.own ? kNoSlot : prow(nd, nd.item()));
             } else {
                 count_src[i] = {1, qs.size()};
-                for (uint32_t e : nd.tail) {
-                    tmp.assign(nd.head.begin(), nd.head.end());
-                    tmp.push_back(e);
+                nd.head(tmp);
+                tmp.push_back(0);
+                for (uint32_t j = 0; j < nd.n_tail(); ++j) {
+                    tmp.back() = nd.tail()[j];
                     add_query(qs, nd, tmp.data(), tmp.size(), kNoSlot);
                 }
             }
@@ -752,10 +804,11 @@ int Miner::run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *use
         hp_->run(wave.size(), 1024, [&](uint64_t lo, uint64_t hi) {
             for (uint64_t i = lo; i < hi; ++i) {
                 const MNode &nd = wave[i];
-                if (nd.slot == kNoSlot || nd.tail.empty()) continue;
+                if (nd.slot == kNoSlot || nd.n_tail() == 0) continue;
                 const uint32_t off = (use_proj_ && nd.proj != kNoProj) ? (uint32_t)root_slot_[nd.proj] * d : 0u;
                 uint32_t *dst = t_items.data() + count_src[i].second;
-                for (size_t j = 0; j < nd.tail.size(); ++j) dst[j] = nd.tail[j] + off;
+                const uint32_t *tail = nd.tail();
+                for (uint32_t j = 0, n = nd.n_tail(); j < n; ++j) dst[j] = tail[j] + off;
             }
         });
         timed(0, [&] {
@@ -773,20 +826,22 @@ int Miner::run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *use
         auto t_exp = Clock::now();
         if (work.size() < wave.size()) work.resize(wave.size());
         hp_->run(wave.size(), 256, [&](uint64_t lo, uint64_t hi) {
+            std::vector<uint64_t> keys;
             for (uint64_t i = lo; i < hi; ++i) {
                 const MNode &nd = wave[i];
                 Work &wk = work[i];
-                wk.head.assign(nd.head.begin(), nd.head.end());
+                nd.head(wk.head);
                 wk.f.clear();
                 wk.emit = 0;
                 wk.pool_q = wk.fhut_q = wk.feat0 = wk.kid0 = wk.nkids = 0;
                 const uint32_t *cs =
                     (count_src[i].first == 0 ? counts.data() : counts_q.data()) + count_src[i].second;
-                for (size_t j = 0; j < nd.tail.size(); ++j) {
+                const uint32_t *tail = nd.tail();
+                for (uint32_t j = 0, n = nd.n_tail(); j < n; ++j) {
                     const uint32_t s = cs[j];
                     if (s < thr_) continue;
-                    if (s == nd.sup) wk.head.push_back(nd.tail[j]);
-                    else wk.f.emplace_back(s, nd.tail[j]);
+                    if (s == nd.sup) wk.head.push_back(tail[j]);
+                    else wk.f.emplace_back(s, tail[j]);
                 }
                 std::sort(wk.f.begin(), wk.f.end());
                 wk.kind = wk.f.empty() ? 0 : 1;
@@ -797,16 +852,21 @@ int Miner::run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *use
                         (use_proj_ && nd.proj != kNoProj) ? (uint32_t)root_slot_[nd.proj] * ds_.d : 0u;
                     if (nd.slot == kNoSlot)
                         for (uint32_t h : wk.head) wk.fq.push_back(h + off);
-                    else if (nd.piv != kNoItem)
-                        wk.fq.push_back(nd.piv + off);
-                    for (auto &pr : wk.f) wk.fq.push_back(pr.second + off);
+                    else if (!nd.own)
+                        wk.fq.push_back(nd.item() + off);
+                    for (const Ext &x : wk.f) wk.fq.push_back(x.item() + off);
                 }
                 // the pool query lists the rarest pool rows first: the device AND empties
                 // sooner and stops reading rows
-                wk.pq.assign(wk.head.begin(), wk.head.end());
-                for (auto &pr : wk.f) wk.pq.push_back(pr.second);
-                std::sort(wk.pq.begin(), wk.pq.end(),
-                          [&](uint32_t x, uint32_t y) { return cand_freq_[x] < cand_freq_[y]; });
+                keys.clear();
+                auto rank_key = [&](uint32_t x) {
+                    return std::min<uint64_t>(cand_freq_[x], 0xffffffffull) << 32 | x;
+                };
+                for (uint32_t x : wk.head) keys.push_back(rank_key(x));
+                for (const Ext &x : wk.f) keys.push_back(rank_key(x.item()));
+                std::sort(keys.begin(), keys.end());
+                wk.pq.resize(keys.size());
+                for (size_t j = 0; j < keys.size(); ++j) wk.pq[j] = (uint32_t)keys[j];
                 if (use_spool_ && nd.proj != kNoProj) {
                     const uint32_t off = (uint32_t)root_slot_[nd.proj] * ds_.d;
                     for (uint32_t &x : wk.pq) x += off;
@@ -833,7 +893,7 @@ int Miner::run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *use
                 n_fi += wk.fq.size();
                 qfhut.ptr.push_back(n_fi);
                 const MNode &nd = wave[i];
-                qfhut.slot.push_back(nd.slot == kNoSlot || nd.piv == kNoItem ? nd.slot : nd.slot | kLeadRow);
+                qfhut.slot.push_back(nd.slot == kNoSlot || nd.own ? nd.slot : nd.slot | kLeadRow);
                 fhut_sup.push_back(wave[i].sup);
             }
             if (slot_pools) spool_max = std::max(spool_max, spool_n_[root_slot_[wave[i].proj]]);
@@ -913,7 +973,7 @@ int Miner::run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *use
                     uint32_t *dst = citems_.data() + it0 + wk.ei0;
                     uint32_t *e = std::copy(wk.head.begin(), wk.head.end(), dst);
                     if (wk.kind == 2)
-                        for (auto &pr : wk.f) *e++ = pr.second;
+                        for (const Ext &x : wk.f) *e++ = x.item();
                     std::sort(dst, e);
                     for (const uint32_t *x = dst; x < e; ++x) ++freq[*x];
                     cptr_[c0 + 1 + wk.e0] = (uint64_t)(e - citems_.data());
@@ -937,7 +997,7 @@ int Miner::run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *use
                     if (wk.kind != 3) continue;
                     const size_t nf = wk.f.size();
                     for (size_t j = 0; j < nf; ++j)
-                        features(wk.head, wave[i].sup, wk.f[j].second, wk.f[j].first, (uint32_t)j, (uint32_t)nf,
+                        features(wk.head, wave[i].sup, wk.f[j].item(), wk.f[j].sup(), (uint32_t)j, (uint32_t)nf,
                                  wfeat.data() + (wk.feat0 + j) * kDim);
                 }
             });
@@ -948,8 +1008,6 @@ int Miner::run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *use
         t_exp = Clock::now();
         // children in the order's sequence: the p-th extension's tail is the
         // extensions after it, and the first is searched first
-        // (kids keeps its elements from wave to wave: they were moved to the stack, so
-        // each is reset below; the spare vectors are handed out by position)
         // A child's mask is its parent's AND its own item's row: the parent's is made here, for
         // the expanding nodes alone (a mask per child was 22 ms of a 2,000,000-transaction search).
         // The root's children have none: their own rows, or their projections once resident.
@@ -959,30 +1017,35 @@ int Miner::run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *use
             Work &wk = work[i];
             wk.kslot = kNoSlot;
             const MNode &nd = wave[i];
-            if (wk.kind != 3 || wk.nkids < 2 || nd.head.empty()) continue;
-            if (nd.slot != kNoSlot && nd.piv == kNoItem) {
+            if (wk.kind != 3) continue;
+            wk.rec = new_rec();
+            if (wk.nkids < 2 || nd.is_root()) continue;
+            if (nd.slot != kNoSlot && nd.own) {
                 wk.kslot = nd.slot;
             } else {
                 wk.kslot = alloc_slot();
                 if (wk.kslot == kNoSlot) continue;
                 if (nd.slot != kNoSlot) {
-                    const uint32_t e = prow(nd, nd.piv);
+                    const uint32_t e = prow(nd, nd.item());
                     qchild.add(&e, 1, nd.slot);
                 } else {
-                    add_query(qchild, nd, nd.head.data(), nd.head.size(), kNoSlot);
+                    nd.head(tmp);
+                    add_query(qchild, nd, tmp.data(), tmp.size(), kNoSlot);
                 }
                 child_slot.push_back(wk.kslot);
             }
             slot_refs_[wk.kslot] += (uint32_t)wk.nkids - 1;   // the last child has no tail to count
         }
-        if (kids.size() < n_ext) kids.resize(n_ext);
-        const uint64_t n_spare = std::min<uint64_t>(spare_.size() / 2, n_ext), sp0 = spare_.size() - 2 * n_spare;
         const uint64_t id0 = parent_.size(), tr0 = tnode_.size();
         parent_.resize(id0 + n_ext);
         if (p_.record_trace) {
             tfeat_.resize((tr0 + n_ext) * kDim);
             tnode_.resize(tr0 + n_ext);
         }
+        // The stack is LIFO: the wave's first node's first child goes on top.  The expanding nodes'
+        // child ranges ascend in wave order, so child k's place is known.
+        const size_t sb = stack.size();
+        stack.resize(sb + n_ext);
         hp_->run(wave.size(), 256, [&](uint64_t lo, uint64_t hi) {
             std::vector<uint32_t> rank;
             for (uint64_t i = lo; i < hi; ++i) {
@@ -994,30 +1057,33 @@ int Miner::run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *use
                 std::iota(rank.begin(), rank.end(), (uint32_t)0);
                 if (p_.order == SGFIM_ORDER_SUPPORT_DESC) {
                     std::sort(rank.begin(), rank.end(), [&](uint32_t a, uint32_t b) {
-                        const uint32_t x = wk.f[a].second, y = wk.f[b].second;
+                        const uint32_t x = wk.f[a].item(), y = wk.f[b].item();
                         return ds_.sup[x] != ds_.sup[y] ? ds_.sup[x] > ds_.sup[y] : x < y;
                     });
                 } else if (p_.order == SGFIM_ORDER_LEARNED) {
                     const float *sc = wscore.data() + wk.feat0;
                     std::stable_sort(rank.begin(), rank.end(), [&](uint32_t a, uint32_t b) { return sc[a] > sc[b]; });
                 }
+                Rec &r = *wk.rec;
+                r.nh = (uint32_t)wk.head.size();
+                r.nf = r.refs = (uint32_t)nf;
+                r.data.resize(wk.head.size() + nf);
+                uint32_t *items = std::copy(wk.head.begin(), wk.head.end(), r.data.data());
+                const bool roots = use_proj_ && nd.proj == kNoProj;   // the root's children: a subtree each
+                if (use_proj_ && !roots) __atomic_fetch_add(&live_[nd.proj], (uint32_t)nf, __ATOMIC_RELAXED);
                 for (size_t p = 0; p < nf; ++p) {
-                    const uint32_t j = rank[p];
+                    const uint32_t j = rank[p], e = wk.f[j].item();
                     const uint64_t k = wk.kid0 + p;
-                    MNode &c = kids[k];
-                    if (k < n_spare) {
-                        c.head = std::move(spare_[sp0 + 2 * k]);
-                        c.tail = std::move(spare_[sp0 + 2 * k + 1]);
-                    }
+                    items[p] = e;
+                    MNode &c = stack[sb + n_ext - 1 - k];
+                    c.rec = &r;
+                    c.pos = (uint32_t)p;
                     c.slot = p + 1 < nf ? wk.kslot : kNoSlot;
-                    c.piv = c.slot != kNoSlot ? wk.f[j].second : kNoItem;
-                    c.head.assign(wk.head.begin(), wk.head.end());
-                    c.head.push_back(wk.f[j].second);
-                    c.sup = wk.f[j].first;
-                    c.tail.resize(nf - p - 1);
-                    for (size_t q = p + 1; q < nf; ++q) c.tail[q - p - 1] = wk.f[rank[q]].second;
+                    c.own = 0;
+                    c.sup = wk.f[j].sup();
                     c.id = (uint32_t)(id0 + k);
-                    c.proj = (use_proj_ && nd.proj == kNoProj) ? wk.f[j].second : nd.proj;
+                    c.proj = roots ? e : nd.proj;
+                    if (roots) ++live_[e];
                     parent_[id0 + k] = nd.id;
                     if (p_.record_trace) {
                         std::copy_n(wfeat.data() + (wk.feat0 + j) * kDim, kDim, tfeat_.data() + (tr0 + k) * kDim);
@@ -1026,30 +1092,15 @@ int Miner::run(const double *ckpts, uint32_t n_ckpt, sgfim_ckpt_cb cb, void *use
                 }
             }
         });
-        spare_.resize(sp0);
+        if (use_proj_ && wave_global) roots_left = stack.size();
         add_since(6, t_exp);
         launch_masks(qchild, child_slot);
-        // the stack is LIFO: push in reverse so that the wave's first node's first
-        // child is popped first
         t_exp = Clock::now();
-        // (the expanding nodes' kid ranges ascend in wave order, so this is the kid
-        // list reversed)
-        {
-            const size_t sb = stack.size();
-            stack.resize(sb + n_ext);
-            hp_->run(n_ext, 4096, [&](uint64_t lo, uint64_t hi) {
-                for (uint64_t k = lo; k < hi; ++k) {
-                    if (use_proj_ && kids[k].proj != kNoProj)
-                        __atomic_fetch_add(&live_[kids[k].proj], 1u, __ATOMIC_RELAXED);
-                    stack[sb + n_ext - 1 - k] = std::move(kids[k]);
-                }
-            });
-            if (use_proj_ && wave_global) roots_left = stack.size();
-        }
         // parents' masks are no longer needed once the child-mask kernel ran (stream order)
         for (MNode &nd : wave) {
             if (nd.slot != kNoSlot) drop_slot(nd.slot);
             if (use_proj_ && nd.proj != kNoProj) --live_[nd.proj];
+            if (--nd.rec->refs == 0) free_recs_.push_back(nd.rec);
         }
         add_since(6, t_exp);
         flush_pool(pool_before);
