@@ -429,7 +429,7 @@ int sgfim_support_batch(sgfim_handle *h, const uint64_t *cand_ptr, const uint32_
     // (300 candidates over 8,192 transactions: 61 -> 42 us a call).  Above the line the kernels cover the
     // copies, and a second pass over the candidates would cost the host more.
     constexpr uint64_t kSmallCall = 1u << 18;   // bytes
-    const bool small = n_cand < kSmallCall / 8 && (n_cand + 1) * 8 + (uint64_t)n_items * 4 <= kSmallCall;
+    const bool small = n_cand < kSmallCall && n_items < kSmallCall && (n_cand + 1) * 8 + n_items * 4 <= kSmallCall;
     if (small)
         for (uint64_t c = 0; c < n_cand; ++c)
             if (cand_ptr[c + 1] < cand_ptr[c]) return fail(h, SGFIM_EINVAL, "cand_ptr must be non-decreasing");

@@ -204,10 +204,10 @@ struct ExtWorkspace {
 
 // Device buffers of the transactionisation calls.
 struct TxWorkspace {
-    DevBuf rows, cols, small, anom, items;
-    size_t bytes() const { return rows.bytes + cols.bytes + small.bytes + anom.bytes + items.bytes; }
+    DevBuf rows, cols, small, anom, items, list;
+    size_t bytes() const { return rows.bytes + cols.bytes + small.bytes + anom.bytes + items.bytes + list.bytes; }
     void release() {
-        for (DevBuf *b : {&rows, &cols, &small, &anom, &items}) b->release();
+        for (DevBuf *b : {&rows, &cols, &small, &anom, &items, &list}) b->release();
     }
 };
 

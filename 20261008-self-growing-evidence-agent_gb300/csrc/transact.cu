@@ -72,15 +72,22 @@ __global__ void __launch_bounds__(256) to_columns_kernel(const double *__restric
 // shared-memory histograms to global ones), and a select step moves every rank
 // to its digit.  Ranks with the same prefix share a histogram.
 //
+// After the third pass few values are left under the open prefixes (22 bits), so
+// that pass also lists them, and the others read the list; a column whose values
+// crowd under them (ties) has no list and is read whole.
+//
 // Bound: HBM/L2, one read of the columns per pass and group of prefixes, and
-// shared-memory atomics.  1,000,000 rows x 21 sensors, 13 ranks: 0.65 ms for the
-// six passes against 7.3 ms for one CTA per (sensor, rank) and eight passes;
-// the transpose 68 us (143 us when every lane stored to its own column).
+// shared-memory atomics.  1,000,000 rows x 21 sensors, 13 ranks: 0.36 ms for the
+// six passes (0.65 without lists) against 7.3 ms for one CTA per (sensor, rank)
+// and eight passes; the transpose 68 us (143 us when every lane stored to its own
+// column).
 constexpr int kDigitBits = 11;
 constexpr uint32_t kDigits = 1u << kDigitBits;
 constexpr int kPasses = 6;            // 5 x 11 + 9 bits
 constexpr uint32_t kHistGroup = 6;    // prefixes counted at a time: 48 KB of histograms
 constexpr int kHistThreads = 512;
+constexpr int kListPass = 2;          // the pass that lists the values under the open prefixes
+constexpr uint32_t kListBlock = 4096; // values a CTA lists at most: more, and the column has no list
 __host__ __device__ constexpr int digit_shift(int pass) {
     return 64 - kDigitBits * (pass + 1) > 0 ? 64 - kDigitBits * (pass + 1) : 0;
 }
@@ -91,6 +98,11 @@ __host__ __device__ constexpr int digit_shift(int pass) {
 struct SelectState {
     uint64_t *prefix, *left, *open;
     uint32_t *group, *n_open;
+    // values under the open prefixes after kListPass, as keys: list_n[s] of them at list + s * cap,
+    // or, above cap, none (cap 0: no lists)
+    uint64_t *list;
+    uint32_t *list_n;
+    uint32_t cap;
 };
 
 __global__ void select_init_kernel(SelectState st, uint32_t S, uint32_t R, const uint64_t *__restrict__ ranks) {
@@ -99,20 +111,39 @@ __global__ void select_init_kernel(SelectState st, uint32_t S, uint32_t R, const
         st.left[i] = ranks[i % R];
         st.group[i] = 0;
         st.open[i] = 0;
-        if (i < S) st.n_open[i] = 1;
+        if (i < S) {
+            st.n_open[i] = 1;
+            if (st.cap) st.list_n[i] = 0;
+        }
     }
 }
 
 // blockIdx.x: run of rows; blockIdx.y: sensor.  hist[s][group][digit].
+// kMode: the columns are read; read and the values found listed; or the lists read
+// where there are lists.
+enum SelectMode : int { SELECT_READ, SELECT_LIST, SELECT_FROM_LIST };
+template <int kMode>
 __global__ void __launch_bounds__(kHistThreads) select_hist_kernel(const double *__restrict__ cols, uint64_t n,
                                                                    SelectState st, uint32_t R, int pass,
                                                                    uint32_t *__restrict__ hist) {
     __shared__ uint32_t h[kHistGroup * kDigits];
+    __shared__ uint32_t listed, list_at;
+    extern __shared__ uint64_t found[];   // kListBlock keys in kListPass
     const uint32_t s = blockIdx.y;
+    constexpr bool listing = kMode == SELECT_LIST;
+    bool from_list = false;
+    const uint64_t *list = nullptr;
     const uint32_t n_open = st.n_open[s];
     const int shift = digit_shift(pass), up = pass ? digit_shift(pass - 1) : 64;
     const uint32_t digits = 1u << (up - shift);
     const double *col = cols + (uint64_t)s * n;
+    if (kMode == SELECT_FROM_LIST) {
+        const uint32_t have = st.list_n[s];
+        from_list = have <= st.cap;
+        list = st.list + (uint64_t)s * st.cap;
+        if (from_list) n = have;
+    }
+    if (listing && threadIdx.x == 0) listed = 0;
     const uint64_t per = (n + gridDim.x - 1) / gridDim.x;
     const uint64_t i0 = min(n, blockIdx.x * per), i1 = min(n, i0 + per);
     for (uint32_t g0 = 0; g0 < n_open; g0 += kHistGroup) {
@@ -123,24 +154,42 @@ __global__ void __launch_bounds__(kHistThreads) select_hist_kernel(const double 
         for (uint32_t i = threadIdx.x; i < ng * kDigits; i += kHistThreads) h[i] = 0;
         __syncthreads();
         for (uint64_t i = i0 + threadIdx.x; i < i1; i += kHistThreads) {
-            const uint64_t key = dkey(col[i]);
+            const uint64_t key = kMode == SELECT_FROM_LIST && from_list ? list[i] : dkey(col[i]);
             const uint64_t pre = pass ? key >> up : 0;
             uint32_t at = kHistGroup;
 #pragma unroll
             for (int g = kHistGroup - 1; g >= 0; --g) at = pre == want[g] ? (uint32_t)g : at;
-            if (at < ng) atomicAdd(&h[at * kDigits + ((uint32_t)(key >> shift) & (digits - 1))], 1u);
+            if (at < ng) {
+                atomicAdd(&h[at * kDigits + ((uint32_t)(key >> shift) & (digits - 1))], 1u);
+                if (listing && listed < kListBlock) {
+                    const uint32_t to = atomicAdd(&listed, 1u);
+                    if (to < kListBlock) found[to] = key;
+                }
+            }
         }
         __syncthreads();
         for (uint32_t i = threadIdx.x; i < ng * kDigits; i += kHistThreads)
             if (h[i]) atomicAdd(&hist[((uint64_t)s * R + g0) * kDigits + i], h[i]);
         __syncthreads();
     }
+    if (!listing) return;
+    const uint32_t m = listed;
+    // a full CTA may have left values out: the top bit then says that there is no list
+    if (threadIdx.x == 0)
+        list_at = m < kListBlock ? atomicAdd(&st.list_n[s], m) : atomicOr(&st.list_n[s], 0x80000000u);
+    __syncthreads();
+    const uint64_t to = list_at;
+    if (m < kListBlock)
+        for (uint32_t i = threadIdx.x; i < m; i += kHistThreads)
+            if (to + i < st.cap) st.list[(uint64_t)s * st.cap + to + i] = found[i];
 }
 
 // One CTA per sensor, a warp per rank: the digit that holds the rank; then the
 // distinct prefixes of the next pass, and the histograms cleared for it.  The
-// last pass writes the statistics.
-__global__ void __launch_bounds__(256) select_step_kernel(SelectState st, uint32_t R, int pass,
+// last pass writes the statistics.  A lane's 64 counts are loaded at once and kept
+// (11 us a pass; 22 us with 8 warps and counts read one by one).
+constexpr int kStepThreads = 512;
+__global__ void __launch_bounds__(kStepThreads) select_step_kernel(SelectState st, uint32_t R, int pass,
                                                           uint32_t *__restrict__ hist, double *__restrict__ out,
                                                           uint32_t out_stride) {
     const uint32_t s = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -149,10 +198,17 @@ __global__ void __launch_bounds__(256) select_step_kernel(SelectState st, uint32
     uint32_t *group = st.group + (uint64_t)s * R;
     uint32_t *hs = hist + (uint64_t)s * R * kDigits;
     const uint32_t n_open = st.n_open[s];
-    for (uint32_t r = warp; r < R; r += 8) {
-        const uint32_t *h = hs + (uint64_t)group[r] * kDigits + lane * (kDigits / 32);
-        uint32_t sum = 0;
-        for (uint32_t i = 0; i < kDigits / 32; ++i) sum += h[i];
+    constexpr uint32_t kMine = kDigits / 32;   // counts per lane
+    for (uint32_t r = warp; r < R; r += kStepThreads / 32) {
+        const uint4 *h = reinterpret_cast<const uint4 *>(hs + (uint64_t)group[r] * kDigits + lane * kMine);
+        uint32_t c[kMine], sum = 0;
+#pragma unroll
+        for (uint32_t i = 0; i < kMine / 4; ++i) {
+            const uint4 v = h[i];
+            c[4 * i] = v.x, c[4 * i + 1] = v.y, c[4 * i + 2] = v.z, c[4 * i + 3] = v.w;
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < kMine; ++i) sum += c[i];
         uint32_t incl = sum;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -165,8 +221,16 @@ __global__ void __launch_bounds__(256) select_step_kernel(SelectState st, uint32
         if (k >= below && k < incl) {   // exactly one lane
             k -= below;
             uint32_t d = 0;
-            while (k >= h[d]) k -= h[d++];
-            prefix[r] = (prefix[r] << (up - shift)) | (lane * (kDigits / 32) + d);
+            bool open_at = true;        // the counts before the rank's digit are taken off
+#pragma unroll
+            for (uint32_t i = 0; i < kMine; ++i) {
+                open_at = open_at && k >= c[i];
+                if (open_at) {
+                    k -= c[i];
+                    ++d;
+                }
+            }
+            prefix[r] = (prefix[r] << (up - shift)) | (lane * kMine + d);
             left[r] = k;
             if (pass == kPasses - 1) out[(uint64_t)s * out_stride + r] = dkey_inv(prefix[r]);
         }
@@ -705,17 +769,27 @@ extern "C" int sgfim_transactionize(sgfim_handle *h, const double *values, uint6
     sel.group = reinterpret_cast<uint32_t *>(sel.open + (size_t)S * batch);
     sel.n_open = sel.group + (size_t)S * batch;
     uint32_t *hist = reinterpret_cast<uint32_t *>(base + o_hist);
+    // lists for a sixteenth of each column; short columns are read whole
+    sel.cap = n_rows >= (1u << 16) ? (uint32_t)std::min<uint64_t>(n_rows / 16, 1u << 28) : 0u;
+    h->tx.list.reserve((size_t)S * sel.cap * 8 + (size_t)S * 4, st);
+    sel.list = h->tx.list.as<uint64_t>();
+    sel.list_n = reinterpret_cast<uint32_t *>(sel.list + (size_t)S * sel.cap);
     // runs of at least 8,192 rows (a CTA clears and adds its histograms once), up to four CTAs per SM
     const unsigned runs = (unsigned)std::min<uint64_t>((n_rows + 8191) / 8192, (uint64_t)h->n_sm * 4 / S + 1);
+    SG_CUDA_TRY(cudaFuncSetAttribute(select_hist_kernel<SELECT_LIST>, cudaFuncAttributeMaxDynamicSharedMemorySize, kListBlock * 8));
     for (uint32_t rank0 = 0; rank0 < R; rank0 += batch) {
         const uint32_t rb = std::min(batch, R - rank0);
         select_init_kernel<<<(S * rb + 255) / 256, 256, 0, st>>>(
             sel, S, rb, reinterpret_cast<const uint64_t *>(base + o_rank) + rank0);
         SG_CUDA_TRY(cudaGetLastError());
         for (int pass = 0; pass < kPasses; ++pass) {
-            select_hist_kernel<<<dim3(runs, S), kHistThreads, 0, st>>>(d_cols.as<double>(), n_rows, sel, rb, pass, hist);
+            const auto kernel = !sel.cap || pass < kListPass ? select_hist_kernel<SELECT_READ>
+                                : pass == kListPass          ? select_hist_kernel<SELECT_LIST>
+                                                             : select_hist_kernel<SELECT_FROM_LIST>;
+            const size_t found_b = sel.cap && pass == kListPass ? kListBlock * 8 : 0;
+            kernel<<<dim3(runs, S), kHistThreads, found_b, st>>>(d_cols.as<double>(), n_rows, sel, rb, pass, hist);
             SG_CUDA_TRY(cudaGetLastError());
-            select_step_kernel<<<S, 256, 0, st>>>(sel, rb, pass, hist, reinterpret_cast<double *>(base + o_stat) + rank0,
+            select_step_kernel<<<S, kStepThreads, 0, st>>>(sel, rb, pass, hist, reinterpret_cast<double *>(base + o_stat) + rank0,
                                                   R);
             SG_CUDA_TRY(cudaGetLastError());
         }

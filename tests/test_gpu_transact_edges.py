@@ -52,3 +52,24 @@ def test_quantile_edges(engine, n, S, bins):
     want = transact.fit_bins(vals, bins)
     for a, b in zip(edges, want):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("n", [65_535, 65_536, 200_001])
+def test_quantiles_with_and_without_lists(engine, n):
+    """Columns long enough that the later passes read a list of the values left (spread values), and
+    columns that crowd under the open prefixes so that no list holds them: constant, a few values,
+    values that differ in the last bits only, half constant and half spread."""
+    rng = np.random.default_rng(n)
+    v = np.empty((n, 6))
+    v[:, 0] = rng.standard_normal(n)
+    v[:, 1] = 3.25
+    v[:, 2] = rng.integers(0, 5, n) / 7.0
+    v[:, 3] = 1.0 + rng.integers(0, 1 << 20, n) * 2.0 ** -52
+    v[:, 4] = np.where(rng.random(n) < 0.5, -2.0, rng.random(n) * 1e6)
+    v[:, 5] = rng.random(n) * 10.0 ** rng.integers(-200, 200, n)
+    _, _, edges = engine.transactionize(v, 1, n // 50, 6)
+    for a, b in zip(edges, transact.fit_bins(v, 6)):
+        assert np.array_equal(a, b)
+    _, _, edges = engine.transactionize(v, 1, n // 50, 40)   # more ranks than a histogram group
+    for a, b in zip(edges, transact.fit_bins(v, 40)):
+        assert np.array_equal(a, b)
