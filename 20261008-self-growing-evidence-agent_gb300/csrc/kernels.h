@@ -168,8 +168,9 @@ size_t cooc_scratch_bytes(uint32_t d, uint64_t n_words, int kind);
 
 // Batched window miner (kernels_wmine.cu).  A task is a whole window or one
 // child's subtree of an expanded node: the root of a split window (wroot_kernel
-// fills the root records first) or a node below it (wsub_kernel).  Per-warp workspaces are warp-major: lists list_cap x MW
-// words, lmfi lmfi_cap, pool pool_cap x MW words + pool_cap supports, levels
+// fills the root records first) or a node below it (wsub_kernel).  Per-warp
+// workspaces are warp-major: lists list_cap x MW words (the vertical search:
+// list_cap 32-bit places), lmfi lmfi_cap, pool pool_cap x MW words + pool_cap supports, levels
 // wmine_level_bytes(MW).  task_status: 0 done, 1 workspace overflow (mine the
 // window elsewhere), 2 output arena full (retry the task).
 constexpr uint32_t kWholeWindow = 0xffffffffu;

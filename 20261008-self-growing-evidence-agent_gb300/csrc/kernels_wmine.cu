@@ -38,7 +38,7 @@
 // become the tasks, the costliest of these once more.  Tasks share no pool, so a
 // candidate of one subtree may sit inside a candidate of an earlier subtree
 // in depth-first order (never of a later one, by the argument above);
-// wfilter_kernel removes exactly those with a vertical bitmap of the window's
+// the wfilter kernels remove exactly those with a vertical bitmap of the window's
 // candidates, and wgather_kernel writes the kept candidates in window order.
 //
 // Work is distributed by atomic counters (costliest tasks first); every

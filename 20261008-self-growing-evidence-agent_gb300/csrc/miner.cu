@@ -14,8 +14,9 @@
 //   leaf:          F empty -> H is a candidate unless a pool member contains it
 //   HUT:           H u F contained in a pool member -> no new MFI below
 //   FHUT:          sup(H u F) >= thr -> H u F is the subtree's only candidate
-//   children:      H u {f_i} with tail f_{i+1..}, masks built on the device,
-//                  searched f_0 first
+//   children:      H u {f_i} with tail f_{i+1..}, searched f_0 first; a child's
+//                  mask is its parent's AND its item's row, made whole on the
+//                  device when it expands in turn
 //
 // The pool of candidates lives on the device as a vertical bitmap (one bit
 // per candidate in every item's row), so "is Q contained in a candidate" is an
@@ -30,8 +31,8 @@
 // tail counts, FHUT counts and child masks are sup(r)/N as long as on the
 // whole database.  Up to kProjSlots projections are resident in one buffer
 // (slot p's row e is row p*d + e of it), a projection is built on the device
-// when its root child is popped, and its slot is reused once no node of the
-// subtree is left; a wave may hold nodes of several resident projections, and
+// when its root child is popped, or before that in a free slot while the host
+// works on a wave, and its slot is reused once no node of the subtree is left; a wave may hold nodes of several resident projections, and
 // its queries address rows through the slot of each node's projection.
 //
 // The order of each node's extensions is a policy that shapes the tree (which
