@@ -18,6 +18,7 @@
 
 #include "common.cuh"
 #include "engine.h"
+#include "window_sizes.h"
 
 struct sgfim_ring {
     int device = 0;
@@ -365,14 +366,11 @@ int sgfim_ring_mine_windows(sgfim_ring *r, sgfim_handle *h, const uint64_t *star
                 max_len = std::max(max_len, lens[w]);
                 if (lens[w] >= kSplitMin) split.push_back((uint32_t)w);
             }
-            // the vertical search lists the task's transactions (4 bytes each); the horizontal one
-            // stacks every level's database as masks
             const bool vertical = !(h->flags & SGFIM_F_WINDOWS_HORIZONTAL);
-            const uint64_t list_cap = std::min<uint64_t>(
-                std::max<uint64_t>(8192, (vertical ? 1 : 2) * max_len + 1024) & ~3ull, 1ull << 30);
+            const WindowSizes sizes = window_sizes(max_len, vertical);
+            const uint64_t list_cap = sizes.list_cap, v_words = sizes.v_words;
             const size_t list_b = vertical ? 4 : mw * 8;
             const uint64_t lmfi_cap = 1u << 16, pool_cap = 1u << 16;
-            const uint64_t v_words = vertical ? ((max_len + 31) / 32 + 1 + 3) & ~3ull : 0;   // whole 16-byte pieces
             const size_t v_bytes = (size_t)(128 + wmine_depth()) * v_words * 4;
             const size_t per_warp =
                 list_cap * list_b + lmfi_cap * 4 + pool_cap * (mw * 8 + 4) + wmine_level_bytes(mw) + v_bytes;
