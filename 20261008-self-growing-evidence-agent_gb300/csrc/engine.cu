@@ -539,9 +539,11 @@ int sgfim_cooccurrence_device(sgfim_handle *h, const uint64_t *bitmaps, uint32_t
     API_GUARD_BEGIN
     cudaSetDevice(h->device);
     cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : (cudaStream_t)0;
-    // AUTO: the tcgen05 fp4 GEMM (the fastest on GB300 at 1,024 x 1,024 x 2^20: 0.30 ms, against
-    // 0.53 ms for e4m3 with 256 x 256 blocks, 1.29 ms with 128 x 128 tiles and 4.97 ms for the
-    // CUDA-core popcount); the popcount kernel when the layout does not suit it
+    // AUTO: the tcgen05 fp4 GEMM.  At 1,024 x 1,024 x 2^20 it takes 0.30 ms, against 0.53 ms for
+    // e4m3 with 256 x 256 blocks, 1.29 ms with 128 x 128 tiles and 4.97 ms for the CUDA-core popcount;
+    // against the 256 x 256 form over 1 to 2,500 rows x 2 to 16,384 words, at pitches of 2 to 16 words
+    // past a multiple of 16 and on it, it took 0.3 to 1.0 of the time (up to 1 us more on 32 rows x 48
+    // words and less, where both are launches).  The popcount kernel when the layout does not suit it.
     int rc = -1;
     if (kind == SGFIM_COOC_AUTO) {
         rc = cooc_device(bitmaps, d, n_words, row_stride, out, SGFIM_COOC_TC_F4, st, h->n_sm, nullptr, 0,

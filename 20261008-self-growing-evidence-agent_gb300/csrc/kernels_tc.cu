@@ -20,6 +20,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "cooc_plan.h"
 #include "kernels.h"
 #include "tcgen05.cuh"
 
@@ -453,8 +454,8 @@ __global__ void __launch_bounds__(kT2Threads, 1)
 //
 // The work is cut into runs of transactions, all tiles of a run next to each
 // other, so the CTAs that read the same rows read them at the same time (from L2:
-// with a tile's runs next to each other the bitmaps came 4 times from HBM).  It is
-// dealt evenly in steps, so a CTA may end one tile and begin the next; counts are added to out and its
+// with a tile's runs next to each other the bitmaps came 4 times from HBM).  How it is cut
+// and dealt is in cooc_plan.h; a CTA may end one tile and begin the next.  Counts are added to out and its
 // mirror with coalesced atomics (the mirror through a shared-memory transpose).
 // A diagonal tile's A rows are a half of its B rows: their bits are loaded once.
 //
@@ -479,14 +480,10 @@ constexpr int kF4Stages = 3;
 constexpr int kF4Ring = 5;
 constexpr int kF4RowBytes = kF4Words * 8;
 constexpr int kF4RingBytes = (kF4RowsA + kF4RowsB) * kF4RowBytes;   // 24 KB
+static_assert(kF4Words == 8 && kF4RowsA == 128 && kF4RowsB == 256, "f4_plan cuts the work for these tiles and steps");
 constexpr int kF4Turn = 32 * 17;                         // words of a warp's 32 x 16 transpose buffer
 constexpr uint32_t kF4ScaleCol = 256;                    // block scales: TMEM columns 256..319
 constexpr uint32_t kF4ColA = 320;                        // A: 32 columns (256 values per row) per stage
-constexpr uint64_t kF4MaxSteps = (1u << 20) / (kF4Words * 64);   // double steps summed in one accumulator
-// Double steps of a CTA, at least: its fixed part (tensor memory, barriers, counts
-// to out) is about 2 us, a double step 1 us.  126 rows x 65,536 transactions, a
-// call: 18 us at 2, 20 at 4, 23 at 8, 31 at 16.
-constexpr uint64_t kF4MinSteps = 2;
 // A, B e2m1; scale format ue8m0; N = 256, M = 128; K = 64
 constexpr uint32_t kF4Idesc = (1u << 7) | (1u << 10) | ((256u >> 3) << 17) | (1u << 23) | ((128u >> 4) << 24);
 
@@ -517,34 +514,6 @@ __device__ __forceinline__ void expand_f4(const uint4 &x, uint4 (&p)[4]) {
     p[3] = mask4(make_uint4(x.x >> 1, x.y >> 1, x.z >> 1, x.w >> 1), 0x44444444u);
 }
 constexpr uint32_t kF4ScaleLow = 0x7f807f80u, kF4ScaleHigh = 0x7e7e7e7eu;   // pieces 0 and 1; 2 and 3 (ue8m0)
-
-struct F4Work {
-    uint32_t d, col_tiles;      // rows; 256-row column tiles
-    uint64_t tiles;
-    uint64_t run, last;         // double steps of a run of transactions, and of the last run
-    uint64_t full;              // double steps of all tiles in the runs before the last
-    uint64_t total;             // double steps of the whole product
-    uint64_t share;             // double steps of a CTA
-};
-
-// The tile and double step at position g of the work, and how many follow in its
-// run (itself included).  Row tile bi (128 rows) meets the column tiles from
-// bi / 2 on.
-__device__ __forceinline__ uint64_t f4_unit(const F4Work &w, uint64_t g, uint32_t &bi, uint32_t &bj, uint64_t &step0) {
-    const uint64_t len = g < w.full ? w.run : w.last;
-    const uint64_t u = g < w.full ? g / w.run : (g - w.full) / w.last;
-    const uint64_t s = g < w.full ? g - u * w.run : g - w.full - u * w.last;
-    const uint64_t r = g < w.full ? u / w.tiles : w.full / (w.tiles * w.run);
-    uint64_t t = g < w.full ? u - r * w.tiles : u;
-    step0 = r * w.run + s;
-    bi = 0;
-    while (t >= w.col_tiles - (bi >> 1)) {
-        t -= w.col_tiles - (bi >> 1);
-        ++bi;
-    }
-    bj = (bi >> 1) + (uint32_t)t;
-    return len - s;
-}
 
 // 128 bits of a row -> 16 TMEM columns of e2m1 values.
 __device__ __forceinline__ void tmem_st_f4(uint32_t taddr, const uint4 &x) {
@@ -583,7 +552,8 @@ __global__ void __launch_bounds__(kF4Threads, 1)
     uint8_t *base = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem) + 1023) & ~uintptr_t(1023));
     uint8_t *ring = base + (size_t)kF4Stages * kF4StageBytes;
     uint32_t *turn = reinterpret_cast<uint32_t *>(base);   // transposes, while no stage is in use
-    const uint64_t g0 = work.share * blockIdx.x, g1 = min(work.total, g0 + work.share);
+    uint64_t g0, g1;
+    f4_part(work, blockIdx.x, g0, g1);
 
     if (warp == 0) tmem_alloc(&tmem_slot, 512);
     if (tid == 0) {
@@ -848,25 +818,10 @@ int cooc_f4_device(const uint64_t *bitmaps, uint32_t d, uint64_t n_words, uint64
         return -1;
     SG_CUDA_TRY(cudaMemsetAsync(out, 0, (size_t)d * d * 4, st));
     if (n_words == 0) return 0;
-    F4Work w;
-    w.d = d;
-    w.col_tiles = (d + kF4RowsB - 1) / kF4RowsB;
-    const uint32_t row_tiles = (d + kF4RowsA - 1) / kF4RowsA;
-    uint64_t tiles = 0;
-    for (uint32_t bi = 0; bi < row_tiles; ++bi) tiles += w.col_tiles - (bi >> 1);
-    w.tiles = tiles;
-    const uint64_t steps = (n_words + kF4Words - 1) / kF4Words;
-    w.total = tiles * steps;
-    // a CTA's share is a run where runs allow it: most CTAs then have one tile
-    w.share = std::max<uint64_t>(kF4MinSteps, (w.total + n_sm - 1) / n_sm);
-    w.run = std::min<uint64_t>(std::min<uint64_t>(steps, kF4MaxSteps), w.share);
-    const uint64_t grid = (w.total + w.share - 1) / w.share;
-    const uint64_t runs = (steps + w.run - 1) / w.run;
-    w.last = steps - (runs - 1) * w.run;
-    w.full = tiles * w.run * (runs - 1);
+    const F4Work w = f4_plan(d, n_words, (uint64_t)n_sm);
     const size_t smem = f4_smem_bytes();
     SG_CUDA_TRY(cudaFuncSetAttribute(cooc_f4_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    cooc_f4_kernel<<<(unsigned)grid, kF4Threads, smem, st>>>(map, w, out, dev_err);
+    cooc_f4_kernel<<<(unsigned)w.ctas, kF4Threads, smem, st>>>(map, w, out, dev_err);
     SG_CUDA_TRY(cudaGetLastError());
     if (launches) *launches += 1;
     return 0;

@@ -52,3 +52,11 @@ def test_cooc_f4_full_rows(engine, d, n_txn):
     want[d // 2, :] = half
     want[:, d // 2] = half
     assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("d,words", [(1024, 512), (1024, 514), (300, 512), (257, 966), (1051, 78), (1400, 128), (700, 10)])
+def test_cooc_f4_short_last_run(engine, d, words):
+    """Shapes whose last run of transactions is short and dealt in whole tiles."""
+    rng = np.random.default_rng(d + words)
+    bm = np.packbits(rng.random((d, words * 64)) < 0.2, axis=1, bitorder="little").view(np.uint64)
+    assert np.array_equal(_run(engine, bm, L.COOC_AUTO), _exact(bm))
