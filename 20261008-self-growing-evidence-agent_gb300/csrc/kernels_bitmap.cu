@@ -13,6 +13,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "support_rule.h"
 
 namespace sg {
 
@@ -1033,22 +1034,11 @@ bool encode_bitmap_map(CUtensorMap *map, const uint64_t *bitmaps, uint32_t d, ui
     return r == CUDA_SUCCESS;
 }
 
-// The kernel of an AUTO call (map: the rows can be staged by TMA).
-//
-// Streaming reads every row of every candidate from L2; staging reads the
-// bitmaps once per SM, whatever the number of candidates.  At 1,048,576
-// transactions, in us (streamed / k1_lane_tm), sensor rows and sparse rows alike:
-//   256 rows:    20,000 candidates 546 / 2,082; 60,000 1,489 / 2,665; 200,000 4,719 / 5,427
-//   640 rows:    20,000 701 / 3,002; 60,000 1,978 / 3,581; 200,000 6,206 / 6,354; 600,000 17,857 / 13,709
-//   1,024 rows:  20,000 626 / 3,416; 200,000 6,296 / 6,776; 600,000 18,398 / 14,119
-// and in proportion to the transactions from 20,000 on: the staged kernel pays
-// per box of 256 rows, so the line is a number of candidates and boxes.
-// Above it, calls of 2e9 candidate-words (2.4 ms) or more look whether the data
+// The kernel of an AUTO call (map: the rows can be staged by TMA).  Above the line of
+// support_rule.h, calls of 2e9 candidate-words (2.4 ms) or more look whether the data
 // are sparse (kernels_pair.cu), which costs them 40 us when they are not.
 static SupportKernel auto_kernel(uint64_t n_cand, uint32_t d, uint64_t n_words, bool map) {
-    if (!map || d == 0) return SUPPORT_STREAM;
-    const uint64_t boxes = (d + 255) / 256;
-    if (n_cand < 100000 + 30000 * boxes) return SUPPORT_STREAM;
+    if (!map || d == 0 || support_streams(n_cand, d, n_words)) return SUPPORT_STREAM;
     if (pair_supported(d, n_cand) && n_cand * n_words >= 2000000000ull) return SUPPORT_PAIR;
     return lane_supported(d) ? SUPPORT_LANE_TM : SUPPORT_STAGED4;
 }
