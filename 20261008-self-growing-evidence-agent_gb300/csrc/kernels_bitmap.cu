@@ -1034,12 +1034,10 @@ bool encode_bitmap_map(CUtensorMap *map, const uint64_t *bitmaps, uint32_t d, ui
     return r == CUDA_SUCCESS;
 }
 
-// The kernel of an AUTO call (map: the rows can be staged by TMA).  Above the line of
-// support_rule.h, calls of 2e9 candidate-words (2.4 ms) or more look whether the data
-// are sparse (kernels_pair.cu), which costs them 40 us when they are not.
+// The kernel of an AUTO call (map: the rows can be staged by TMA); the lines are in support_rule.h.
 static SupportKernel auto_kernel(uint64_t n_cand, uint32_t d, uint64_t n_words, bool map) {
     if (!map || d == 0 || support_streams(n_cand, d, n_words)) return SUPPORT_STREAM;
-    if (pair_supported(d, n_cand) && n_cand * n_words >= 2000000000ull) return SUPPORT_PAIR;
+    if (pair_supported(d, n_cand) && support_pairs(n_cand, d, n_words)) return SUPPORT_PAIR;
     return lane_supported(d) ? SUPPORT_LANE_TM : SUPPORT_STAGED4;
 }
 

@@ -1,4 +1,4 @@
-// support_rule.h -- when an AUTO support call streams its candidates' rows.
+// support_rule.h -- the kernel of an AUTO support call.
 #pragma once
 
 #include <stdint.h>
@@ -27,6 +27,22 @@ inline bool support_streams(uint64_t n_cand, uint32_t d, uint64_t n_words) {
     const double streamed = 5 + n * (0.08 + 0.44 * far * (double)((n_words + 255) / 256));
     const double staged = 25 + (double)((n_words + 15) / 16) * (0.95 + 0.47 * (double)boxes + 0.0207 * n);
     return streamed <= staged;
+}
+
+// Whether a call that does not stream looks if its data are sparse enough for pair groups
+// (kernels_pair.cu), which costs it 40 us when they are not: calls of 2e9 candidate-words
+// (2.4 ms) or more, of enough candidates.  Groups are counted 32 at a time, two units of
+// work each, by 32 warps an SM: few candidates fill few groups, and few rows make few
+// pairs, whose groups are of eight, so the line rises below 256 rows.  1,048,576 sparse
+// transactions, in us (k1_lane_tm_kernel / pair groups):
+//   64 rows:    130,000 candidates 4,116 / 8,144; 400,000 9,545 / 10,581; 600,000 13,410 / 11,926
+//   128 rows:   130,000 4,108 / 6,155; 400,000 9,545 / 10,191; 600,000 13,415 / 12,229
+//   180 rows:   200,000 5,696 / 6,414; 300,000 7,649 / 7,978; 400,000 9,547 / 8,682
+//   256 rows:   130,000 4,116 / 4,379; 200,000 5,695 / 5,077; 1,000,000 20,991 / 12,910
+//   1,024 rows: 130,000 5,524 / 5,914; 200,000 7,110 / 6,767; 1,000,000 22,349 / 12,855
+inline bool support_pairs(uint64_t n_cand, uint32_t d, uint64_t n_words) {
+    const uint64_t least = 160000 + (d < 256 ? 2000 * (uint64_t)(256 - d) : 0);
+    return n_cand >= least && n_cand * n_words >= 2000000000ull;
 }
 
 }  // namespace sg
