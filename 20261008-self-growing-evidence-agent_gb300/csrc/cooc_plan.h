@@ -10,10 +10,12 @@
 
 #include <algorithm>
 
+#ifndef SG_HOST_DEVICE
 #ifdef __CUDACC__
 #define SG_HOST_DEVICE __host__ __device__ __forceinline__
 #else
 #define SG_HOST_DEVICE inline
+#endif
 #endif
 
 namespace sg {

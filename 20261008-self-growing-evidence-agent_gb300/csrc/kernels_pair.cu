@@ -43,6 +43,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "support_rule.h"
 #include "tcgen05.cuh"
 
 namespace sg {
@@ -67,7 +68,7 @@ struct PairRec {
 // Counters of one call (device).
 struct PairCtl {
     uint32_t dense;                      // the gate: 1 = too dense for this path
-    uint32_t sampled, live;              // words sampled, and how many were not empty
+    uint32_t sampled, live, items;       // words sampled, how many were not empty, their candidates' items
     uint32_t groups[kPairGroup + 1];     // groups of each size
     uint32_t cursor[kPairGroup + 1];
     unsigned long long ovf_n;            // candidates with more items than a record holds
@@ -235,11 +236,13 @@ __global__ void __launch_bounds__(256) pair_sample_kernel(const uint64_t *__rest
     if (lane == 0) {
         atomicAdd(&s.ctl->live, live);
         atomicAdd(&s.ctl->sampled, 32u);
+        atomicAdd(&s.ctl->items, (uint32_t)k);
     }
 }
 
-// Dense when more than a sixth of the sampled words hold a bit.
-__global__ void pair_gate_kernel(PairCtl *ctl) { ctl->dense = ctl->live > ctl->sampled / 6; }
+__global__ void pair_gate_kernel(PairCtl *ctl, uint64_t n, uint32_t d) {
+    ctl->dense = pair_dense(ctl->live, ctl->sampled, ctl->items, n, d);
+}
 
 // Groups of each size over all pairs: cnt / kPairGroup full ones, and one of the rest.
 __global__ void __launch_bounds__(256) pair_sizes_kernel(PairScratch s, uint64_t pairs) {
@@ -585,7 +588,7 @@ int pair_supports_device(const CUtensorMap *map, const uint64_t *bitmaps, uint32
         pair_sample_kernel<<<kPairSamples * kPairSampleChunks / 8, 256, 0, st>>>(bitmaps, row_stride, n_words, cand_ptr,
                                                                                       cand_items, n_cand, d, s);
         SG_CUDA_TRY(cudaGetLastError());
-        pair_gate_kernel<<<1, 1, 0, st>>>(s.ctl);
+        pair_gate_kernel<<<1, 1, 0, st>>>(s.ctl, n_cand, d);
         SG_CUDA_TRY(cudaGetLastError());
     }
     pair_records_kernel<<<cand_blocks, 256, 0, st>>>(cand_ptr, cand_items, n_cand, d, n_txn, s, out);

@@ -3,6 +3,14 @@
 
 #include <stdint.h>
 
+#ifndef SG_HOST_DEVICE
+#ifdef __CUDACC__
+#define SG_HOST_DEVICE __host__ __device__ __forceinline__
+#else
+#define SG_HOST_DEVICE inline
+#endif
+#endif
+
 namespace sg {
 
 // Streaming (cand_stream_kernel) reads every row of every candidate from L2 or HBM, 256
@@ -43,6 +51,32 @@ inline bool support_streams(uint64_t n_cand, uint32_t d, uint64_t n_words) {
 inline bool support_pairs(uint64_t n_cand, uint32_t d, uint64_t n_words) {
     const uint64_t least = 160000 + (d < 256 ? 2000 * (uint64_t)(256 - d) : 0);
     return n_cand >= least && n_cand * n_words >= 2000000000ull;
+}
+
+// The gate of such a call, on the device: whether sampled candidates are too dense for pair
+// groups.  live: how many of the sampled 32-bit words of their first two rows' ANDs hold a
+// bit; items: the candidates' items, once per 32 words sampled.
+//
+// Up to a sixth of live words pays for candidates of four items and more.  Shorter ones have
+// few further rows to skip, and every word where the first four rows are left is counted on a
+// slow path: all live words for two items.  A pair group costs more the fewer candidates share
+// it, so the line falls below 400 candidates a row.  1,048,576 transactions, every row with the
+// same share of bits, in us (k1_lane_tm_kernel / pair groups):
+//   600,000 of 2 items:    300 rows, 1% 7,445 / 5,968, 4% 7,447 / 10,859; 1,024 rows, 2% 8,352 / 10,351
+//   600,000 of 3 items:    300 rows, 4% 9,370 / 7,196; 1,024 rows, 4% 10,264 / 9,966, 6% 10,266 / 12,121
+//   250,000 of 3 items:    300 rows, 4% 5,117 / 4,757; 1,024 rows, 2% 6,016 / 5,657, 4% 6,016 / 6,674
+//   600,000 of 4 items:    1,024 rows, 6% 12,133 / 10,010, 8% 12,133 / 12,140
+//   600,000 of 3..8 items: 1,024 rows, 7% (14% of the words live) 14,801 / 11,995, 10% 14,800 / 16,392
+SG_HOST_DEVICE bool pair_dense(uint32_t live, uint32_t sampled, uint32_t items, uint64_t n_cand, uint32_t d) {
+    if (sampled == 0) return false;
+    const float k = 32.f * (float)items / (float)sampled;
+    float line = 1.f / 6;
+    if (k <= 2) line = 0.0035f;
+    else if (k < 3) line = 0.0035f + 0.0565f * (k - 2) * (k - 2);
+    else if (k < 4) line = 0.06f + 0.1067f * (k - 3);
+    const float shared = (float)n_cand / (400.f * (float)d);
+    if (shared < 1) line *= shared;
+    return (float)live > line * (float)sampled;
 }
 
 }  // namespace sg
