@@ -615,6 +615,9 @@ int sgfim_ring_mine_windows(sgfim_ring *r, sgfim_handle *h, const uint64_t *star
                                     uint32_t si) -> void {
                 const uint32_t k = u32_at(R, o_k), n = (uint32_t)lens[w];
                 const uint32_t parent = rec == kWholeWindow ? w : rec;
+                // (records name their parent by window on the first level and by record on the second:
+                // the cursor stays on its level)
+                const uint32_t si_end = rec == kWholeWindow ? std::min(lvl2, (uint32_t)sub_win.size()) : (uint32_t)sub_win.size();
                 uint32_t run = 0;        // neighbours before child j that would share a task
                 double run_shared = 0.0, run_alone = 0.0;
                 auto end_run = [&](uint32_t j) {
@@ -631,7 +634,7 @@ int sgfim_ring_mine_windows(sgfim_ring *r, sgfim_handle *h, const uint64_t *star
                     run_shared = run_alone = 0.0;
                 };
                 for (uint32_t j = 0; j < k; ++j) {
-                    const bool expanded = si < sub_win.size() && sub_win[si] == w && sub_parent[si] == parent &&
+                    const bool expanded = si < si_end && sub_win[si] == w && sub_parent[si] == parent &&
                                           sub_child[si] == j;
                     const uint32_t sup = u32_at(R, o_c + 4 * j);
                     if (!expanded) {
