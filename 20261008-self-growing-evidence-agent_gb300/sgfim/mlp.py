@@ -14,6 +14,9 @@ from __future__ import annotations
 
 import numpy as np
 
+from ._lib import EDEVICE
+from .engine import SgfimError
+
 FEATURES = ("prefix_support", "item_support", "extension_support", "conditional_density", "depth",
             "min_pair_cooc", "mean_pair_cooc", "sibling_position")
 IN_DIM = len(FEATURES)
@@ -70,7 +73,15 @@ class Trainer:
     def _stream(self):
         return self.torch.cuda.current_stream(self.dev).cuda_stream
 
+    def check(self):
+        """Waits for the passes launched so far and raises when one gave up on a wait on the device (its outputs,
+        and what was computed from them, are then incomplete).  fit() asks once an epoch; a caller of forward(),
+        gradients() or step() asks when it next waits for the device anyway."""
+        if self.eng.device_status(self._stream()) != 0:
+            raise SgfimError(EDEVICE, "a scorer pass gave up on a wait on the device: its results are incomplete")
+
     def forward(self, X, keep=False):
+        """Probabilities of the rows of X (with keep also both layers' pre-activations); asynchronous, see check()."""
         torch = self.torch
         X = X.to(self.dev, torch.float32).contiguous()
         n = X.shape[0]
@@ -85,7 +96,7 @@ class Trainer:
         return (P, Z1, Z2) if keep else P
 
     def gradients(self, X, Y, WT=None):
-        """Loss and gradients of the weighted mean BCE (fp32, on the GPU)."""
+        """Loss and gradients of the weighted mean BCE (fp32, on the GPU); asynchronous, see check()."""
         torch = self.torch
         X = X.to(self.dev, torch.float32).contiguous()
         Y = Y.to(self.dev, torch.float32).contiguous()
@@ -145,4 +156,5 @@ class Trainer:
                 loss = self.step(Xd[idx], Yd[idx], Wd[idx] if Wd is not None else None, lr=lr)
                 tot += loss * len(idx)
             hist.append(float(tot.item()) / n)
+            self.check()
         return hist

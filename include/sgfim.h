@@ -86,8 +86,8 @@ const char *sgfim_last_error(const sgfim_handle *h);
 int sgfim_abi_version(void);
 
 /* Device status of the asynchronous device-pointer calls
- * (sgfim_support_batch_device, sgfim_cooccurrence_device): waits for
- * `stream`, then reads and clears the handle's device error word.  Returns
+ * (sgfim_support_batch_device, sgfim_cooccurrence_device, sgfim_mlp_forward):
+ * waits for `stream`, then reads and clears the handle's device error word.  Returns
  * SGFIM_OK, or SGFIM_EDEVICE when a kernel launched since the last check gave
  * up (a bounded wait ran out): the outputs of those calls are then
  * incomplete.  The calls with host buffers check it themselves.  The
@@ -490,7 +490,8 @@ int sgfim_load_scorer(sgfim_handle *h, uint32_t in_dim, uint32_t hidden, const u
  * `stream`).  No reference counterpart: the reference has no learned part.
  * Forward: X [n][in_dim] fp32 -> P [n] probabilities; Z1/Z2 [n][hidden]
  * receive the pre-activations when non-null.  in_dim 1..64, hidden a
- * multiple of 32 up to 256. */
+ * multiple of 32 up to 256.  A wait on the device that runs out leaves the
+ * outputs incomplete: sgfim_device_status says so. */
 int sgfim_mlp_forward(sgfim_handle *h, const float *X, uint32_t n, uint32_t in_dim, uint32_t hidden,
                       const uint16_t *W1, const float *b1, const uint16_t *W2, const float *b2, const uint16_t *w3,
                       const float *b3, float *Z1, float *Z2, float *P, void *stream);

@@ -1,0 +1,45 @@
+"""Host logic of the scorer's trainer on the CPU, with a fake engine: fit() asks for the device status once an
+epoch and raises when a forward or backward pass gave up on a wait."""
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from sgfim import _lib as L  # noqa: E402
+from sgfim.engine import SgfimError  # noqa: E402
+from sgfim.mlp import Trainer  # noqa: E402
+
+
+class FakeEngine:
+    """Counts the status calls; the one of epoch `bad` reports a wait that ran out."""
+
+    def __init__(self, bad=None):
+        self.bad, self.asked = bad, 0
+
+    def device_status(self, stream=0):
+        self.asked += 1
+        return L.EDEVICE if self.asked - 1 == self.bad else 0
+
+
+def _trainer(engine):
+    t = Trainer.__new__(Trainer)
+    t.torch, t.eng, t.dev = torch, engine, torch.device("cpu")
+    t._stream = lambda: 0
+    t.seen = []
+    t.step = lambda X, Y, WT=None, lr=1e-3: (t.seen.append(len(X)), torch.ones(1))[1]
+    return t
+
+
+def test_fit_checks_the_device_every_epoch():
+    t = _trainer(FakeEngine())
+    hist = t.fit(torch.zeros(10, 8), torch.tensor([0.0, 1.0] * 5), epochs=3, batch=4)
+    assert hist == [1.0, 1.0, 1.0] and t.seen == [4, 4, 2] * 3
+    assert t.eng.asked == 3
+
+
+@pytest.mark.parametrize("bad", [0, 2])
+def test_fit_raises_when_a_wait_ran_out(bad):
+    t = _trainer(FakeEngine(bad))
+    with pytest.raises(SgfimError) as e:
+        t.fit(torch.zeros(10, 8), torch.tensor([0.0, 1.0] * 5), epochs=3, batch=4)
+    assert e.value.code == L.EDEVICE
+    assert len(t.seen) == 3 * (bad + 1)     # no step after the epoch that failed
