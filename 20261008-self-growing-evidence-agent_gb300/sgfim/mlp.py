@@ -55,16 +55,21 @@ class Trainer:
             "b3": np.zeros(1),
         }
         self.p = {k: torch.tensor(v, dtype=torch.float32, device=self.dev).contiguous() for k, v in init.items()}
-        # the gradients are slices of one buffer (64-float boundaries), cleared by one launch per step
-        ends = np.cumsum([0] + [(v.numel() + 63) // 64 * 64 for v in self.p.values()])
-        self._g_all = torch.zeros(int(ends[-1]), dtype=torch.float32, device=self.dev)
-        self.g = {k: self._g_all[int(o):int(o) + v.numel()].view(v.shape) for (k, v), o in zip(self.p.items(), ends)}
+        self._alloc_gradients()
         self.m = {k: torch.zeros_like(v) for k, v in self.p.items()}
         self.v = {k: torch.zeros_like(v) for k, v in self.p.items()}
         self.b16 = {k: torch.zeros(v.shape, dtype=torch.int16, device=self.dev) for k, v in self.p.items()
                     if k in ("W1", "W2", "w3")}
         self._refresh_bf16()
         self.steps = 0
+
+    def _alloc_gradients(self):
+        """The gradients are slices of one buffer (64-float boundaries), cleared by one launch per step."""
+        torch = self.torch
+        ends = np.cumsum([0] + [(v.numel() + 63) // 64 * 64 for v in self.p.values()])
+        self._g_all = torch.zeros(int(ends[-1]), dtype=torch.float32, device=self.dev)
+        self.g = {k: self._g_all[int(o):int(o) + v.numel()].view(v.shape) for (k, v), o in zip(self.p.items(), ends)}
+        self._g_own = dict(self.g)
 
     def _refresh_bf16(self):
         for k, t in self.b16.items():
@@ -104,6 +109,9 @@ class Trainer:
         n = X.shape[0]
         P, Z1, Z2 = self.forward(X, keep=True)
         self._g_all.zero_()
+        for k, t in self.g.items():
+            if t is not self._g_own.get(k):   # the caller's tensor
+                t.zero_()
         loss = torch.zeros(1, dtype=torch.float32, device=self.dev)
         self.eng.mlp_backward(X.data_ptr(), n, self.in_dim, self.hidden, self.b16["W2"].data_ptr(),
                               self.b16["w3"].data_ptr(), Z1.data_ptr(), Z2.data_ptr(), P.data_ptr(), Y.data_ptr(),

@@ -43,3 +43,28 @@ def test_fit_raises_when_a_wait_ran_out(bad):
         t.fit(torch.zeros(10, 8), torch.tensor([0.0, 1.0] * 5), epochs=3, batch=4)
     assert e.value.code == L.EDEVICE
     assert len(t.seen) == 3 * (bad + 1)     # no step after the epoch that failed
+
+
+def test_gradients_clear_entries_that_a_caller_replaced():
+    """g[k] may be the caller's own tensor: every entry is cleared before the backward adds to it."""
+    class Adds:
+        def mlp_backward(self, *a):
+            for t in self.g.values():
+                t += 1.0
+    eng = Adds()
+    t = Trainer.__new__(Trainer)
+    t.torch, t.eng, t.dev, t.in_dim, t.hidden = torch, eng, torch.device("cpu"), 8, 32
+    t._stream = lambda: 0
+    t.forward = lambda X, keep=False: (torch.zeros(len(X)),) * 3
+    t.p = {"W1": torch.zeros(32, 8), "b1": torch.zeros(32), "W2": torch.zeros(32, 32), "b2": torch.zeros(32),
+           "w3": torch.zeros(32), "b3": torch.zeros(1)}
+    t.b16 = {"W2": torch.zeros(32, 32, dtype=torch.int16), "w3": torch.zeros(32, dtype=torch.int16)}
+    t._alloc_gradients()
+    eng.g = t.g
+    mine = torch.full((32, 8), 7.0)
+    t.g["W1"] = mine
+    for _ in range(3):
+        _, g = t.gradients(torch.zeros(4, 8), torch.zeros(4))
+    assert g["W1"] is mine
+    for k in t.p:
+        assert g[k].shape == t.p[k].shape and bool((g[k] == 1.0).all()), k
