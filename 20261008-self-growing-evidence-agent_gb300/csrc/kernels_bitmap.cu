@@ -1104,8 +1104,8 @@ int support_batch_device(const uint64_t *bitmaps, uint32_t d, uint64_t n_words, 
     if (kind == SUPPORT_LANE || kind == SUPPORT_LANE_TM) {
         uint32_t *ovf_l = nullptr;
         unsigned long long *ovf_c = nullptr;
-        // after a gated pair call: these kernels run when it found the data dense, and the pair
-        // kernel's events stand
+        // after a gated pair call: these kernels run when it found the data dense.  The host does not
+        // know, so the count's time spans both, from the pair kernel's first event to the end of this one
         if (!gate) mark(0);
         cudaEvent_t *lane_ev = gate ? nullptr : ev;
         int rc = -1;

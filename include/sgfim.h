@@ -225,7 +225,9 @@ typedef struct {
     uint64_t calls;          /* timed support-batch calls */
     uint64_t launches;       /* kernels launched by those calls */
     double prep_ms;          /* candidate packing */
-    double count_ms;         /* the staged (or streaming) counting kernel */
+    double count_ms;         /* the counting kernel; of an AUTO call that asked the device how dense its
+                                data are, both kernels it may take (the other one leaves at once) and what lies
+                                between them */
     double tail_ms;          /* candidates with more than 8 items */
 } sgfim_phase_stats;
 int sgfim_phase_stats_get(sgfim_handle *h, sgfim_phase_stats *out, int reset);
