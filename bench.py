@@ -16,8 +16,8 @@ in HBM (CUDA events on the launching stream, L2 flushed by a 512 MiB write
 before every step); ``e2e`` is the same metric through the C ABI with pinned
 host buffers (bitmaps and candidates copied in, supports copied out, every
 step).  ``roofline`` relates the shared-memory
-bytes that the counting kernel moves (its profiled wavefronts; the algorithmic
-k * N / 8 per candidate where no profile is committed) to the shared-memory
+bytes that the counting kernel moves (the wavefronts of its committed capture of
+this workload on one GPU; the algorithmic k * N / 8 per candidate otherwise) to the shared-memory
 bandwidth (SMs x 128 B/clk x the SM clock sampled during the timed region).
 The default kernel ANDs a pair of rows once for all candidates that share it
 and reads further rows only where bits are left, so it moves fewer than the
@@ -38,6 +38,7 @@ from __future__ import annotations
 
 import argparse
 import json
+import math
 import os
 import statistics
 import subprocess
@@ -59,7 +60,7 @@ WORKLOAD = dict(name="support-1m", n_txn=1 << 20, d=1024, n_regimes=16, dens_lo=
 METRIC = "supports/s (frac of HBM peak)"
 UNIT = "supports/s"
 SMEM_BYTES_PER_CLK = 128        # shared-memory bandwidth of one SM (32 banks x 4 B)
-KERNEL_NAMES = {"auto": "pair_lane_kernel", "pair": "pair_lane_kernel", "lane_tm": "k1_lane_tm_kernel", "lane": "k1_lane_kernel",
+KERNEL_NAMES = {"pair": "pair_lane_kernel", "lane_tm": "k1_lane_tm_kernel", "lane": "k1_lane_kernel",
                 "sorted": "k1_sorted_kernel", "staged": "k1_staged_kernel", "staged4": "k1_staged4_kernel",
                 "stream": "cand_stream_kernel"}
 LEARNED_WEIGHTS = os.path.join(ROOT, "20261008-self-growing-evidence-agent_gb300", "sgfim", "data",
@@ -77,7 +78,7 @@ def parse_args():
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-cooc", action="store_true")
     ap.add_argument("--no-configs", action="store_true", help="skip the anytime, service and learned-order keys")
-    ap.add_argument("--kernel", choices=sorted(KERNEL_NAMES), default="auto")
+    ap.add_argument("--kernel", choices=["auto", *sorted(KERNEL_NAMES)], default="auto")
     ap.add_argument("--workload", default="support-1m",
                     choices=["support-1m", "anytime-2m", "windows-4096", "learned-order", "transact-1m"])
     ap.add_argument("--floor", type=float, default=0.03, help="anytime-2m: support floor (fraction)")
@@ -112,15 +113,34 @@ def measured_peaks():
     return {"hbm_gbs": 6800.0, "bf16_tflops": 1900.0, "sm_max_mhz": 2070.0}, "fallback"
 
 
-def ncu_traffic(kernel):
-    """DRAM bytes per launch of the counting kernel from the committed ncu summary
-    (a capture of this workload: dram__bytes_read.sum + dram__bytes_write.sum), and where
-    given its shared-memory wavefronts of 128 bytes."""
-    path = os.path.join(ROOT, "profiles", f"{kernel}_support-1m.json")
-    if os.path.exists(path):
-        with open(path) as f:
-            return json.load(f)
-    return None
+def profiled(kernel, n_cand, world):
+    """(DRAM bytes, shared-memory bytes) of a launch of the counting kernel from its committed
+    ncu summary (dram__bytes_read.sum + dram__bytes_write.sum; wavefronts of 128 bytes, where
+    given).  The capture is one launch over all of this workload, so both are None for another
+    number of candidates or a rank's slice of the transactions."""
+    path = os.path.join(ROOT, "profiles", f"{kernel.replace('_kernel', '')}_support-1m.json")
+    if world != 1 or n_cand != WORKLOAD["n_cand"] or not os.path.exists(path):
+        return None, None
+    with open(path) as f:
+        c = json.load(f)
+    waves = c.get("shared_wavefronts_per_launch")
+    return c.get("dram_bytes_per_launch"), waves * SMEM_BYTES_PER_CLK if waves else None
+
+
+def dispatched(eng, call, torch, count_ms):
+    """The kernel an AUTO call counted with.  The rule is the library's, the density gate the
+    device's, so the plans AUTO chooses from are timed once each: it took as long as its own."""
+    took = {}
+    for plan in ("pair", "lane_tm", "stream"):
+        eng.set_support_plan(plan)
+        call()
+        torch.cuda.synchronize()
+        eng.phase_stats(reset=True)
+        call()
+        torch.cuda.synchronize()
+        took[plan] = eng.phase_stats(reset=True)["count_ms"]
+    eng.set_support_plan("auto")
+    return min(took, key=lambda k: abs(math.log(took[k] / count_ms)))
 
 
 class ClockSampler:
@@ -476,9 +496,12 @@ def main():
     flush = torch.empty(512 << 20, dtype=torch.uint8, device=dev)
     stream = torch.cuda.current_stream(dev)
 
-    def step():
+    def count():
         eng.support_batch_device(t_bm.data_ptr(), d, wr, bm_r.shape[1], t_cp.data_ptr(), t_ci.data_ptr(), n_cand,
                                  t_out.data_ptr(), stream.cuda_stream)
+
+    def step():
+        count()
         sharding.allreduce_counts(t_out, dist)
 
     for _ in range(args.warmup):
@@ -512,7 +535,9 @@ def main():
     value = n_cand / (ms / 1000.0)   # the whole job counts the one candidate set
     clocks = clk.summary()
 
-    # roofline of the counting kernel: algorithmic bytes of this rank's slice
+    # roofline of the counting kernel: the bytes it moves, by the counters of its capture of this very
+    # workload, or the algorithmic bytes of this rank's slice.  kernel_ms spans the whole count of an AUTO
+    # call: behind the pair groups that is also the kernels that would have counted dense data (up to 0.05 ms)
     peaks, peak_src = measured_peaks()
     k = np.diff(cp).astype(np.int64)
     alg_bytes = float(k.sum()) * (wr * 64 / 8.0)
@@ -521,10 +546,10 @@ def main():
     n_sm = torch.cuda.get_device_properties(dev).multi_processor_count
     sm_mhz = clocks["sm_mhz"] or peaks.get("sm_max_mhz", 2070.0)
     smem_peak = n_sm * SMEM_BYTES_PER_CLK * sm_mhz * 1e6 / 1e9
-    kname = KERNEL_NAMES[args.kernel]
-    tr = ncu_traffic(kname.replace("_kernel", ""))
-    traffic = tr["dram_bytes_per_launch"] if tr else None
-    moved = tr["shared_wavefronts_per_launch"] * SMEM_BYTES_PER_CLK if tr and "shared_wavefronts_per_launch" in tr else None
+    counts = t_out.clone()
+    kname = KERNEL_NAMES[dispatched(eng, count, torch, count_ms) if args.kernel == "auto" else args.kernel]
+    t_out.copy_(counts)
+    traffic, moved = profiled(kname, n_cand, world)
     achieved = moved / (count_ms / 1000.0) / 1e9 if moved else alg_rate
     roofline = {"bound": "smem", "achieved": achieved, "peak": smem_peak, "unit": "GB/s", "frac": achieved / smem_peak,
                 "traffic": traffic,
