@@ -259,8 +259,7 @@ int load_rows(sgfim_handle *h, const uint64_t *row_ptr, const uint32_t *items, u
         SG_CUDA_TRY(cudaMemcpyAsync(ds.sup.data(), ds.sup_dev.ptr, (size_t)ds.d * 4, cudaMemcpyDeviceToHost,
                                     h->stream));
         SG_CUDA_TRY(cudaStreamSynchronize(h->stream));
-        constexpr size_t kKeepLoad = 64ull << 20;
-        if (d_ptr.bytes + d_items.bytes > kKeepLoad) {
+        if (d_ptr.bytes + d_items.bytes > kept_between_calls(h->hbm_budget, 64ull << 20)) {
             d_ptr.release();
             d_items.release();
         }
@@ -396,7 +395,7 @@ int sgfim_support_batch_device(sgfim_handle *h, const uint64_t *bitmaps, uint32_
         map_ptr = map_ok ? bitmaps : nullptr;
         map_key[0] = d; map_key[1] = n_even; map_key[2] = row_stride;
     }
-    h->support_scratch.reserve(support_scratch_bytes(n_cand, d, n_even, h->plan), st);
+    h->support_scratch.reserve(support_scratch_bytes(n_cand, d, n_even, h->plan, h->hbm_budget), st);
     SupportScratch sc{h->support_scratch.ptr, h->support_scratch.bytes};
     const SupportPlan &plan = h->plan;
     const uint64_t n_txn = n_words * 64;
@@ -473,7 +472,7 @@ int sgfim_support_batch(sgfim_handle *h, const uint64_t *cand_ptr, const uint32_
         SG_CUDA_TRY(cudaStreamSynchronize(h->stream));
         if (bad_h) return fail(h, SGFIM_EINVAL, "cand_ptr must be non-decreasing");
     }
-    h->support_scratch.reserve(support_scratch_bytes(n_cand, ds.d, ds.n_words, h->plan), h->stream);
+    h->support_scratch.reserve(support_scratch_bytes(n_cand, ds.d, ds.n_words, h->plan, h->hbm_budget), h->stream);
     SupportScratch sc{h->support_scratch.ptr, h->support_scratch.bytes};
     const SupportPlan &plan = h->plan;
     const uint64_t before = h->launches;

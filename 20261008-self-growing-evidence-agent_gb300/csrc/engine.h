@@ -26,6 +26,12 @@ struct DevBuf {
     template <class T> T *as() const { return static_cast<T *>(ptr); }
 };
 
+// What a call's transient device buffers may keep of the handle's memory budget until the
+// next call: a sixteenth of it, and no more than `most`; beyond that they are given back.
+inline size_t kept_between_calls(uint64_t hbm_budget, size_t most) {
+    return hbm_budget / 16 < most ? (size_t)(hbm_budget / 16) : most;
+}
+
 // Pinned host buffer with geometric growth.
 struct HostBuf {
     void *ptr = nullptr;

@@ -82,8 +82,10 @@ struct SupportScratch {
     void *base = nullptr;
     size_t bytes = 0;
 };
-// scratch that lets every kernel the plan may choose run
-size_t support_scratch_bytes(uint64_t n_cand, uint32_t d, uint64_t n_words, const SupportPlan &plan);
+// scratch that lets every kernel the plan may choose run; the pair groups' tables, which AUTO
+// does without, only up to an eighth of the memory budget
+size_t support_scratch_bytes(uint64_t n_cand, uint32_t d, uint64_t n_words, const SupportPlan &plan,
+                             uint64_t hbm_budget);
 // ev (optional, 4 events): recorded before prep, before the counting kernel,
 // after it, and after the >8-item tail.
 int support_batch_device(const uint64_t *bitmaps, uint32_t d, uint64_t n_words, uint64_t row_stride,

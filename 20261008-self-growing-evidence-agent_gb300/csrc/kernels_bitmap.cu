@@ -1041,12 +1041,15 @@ static SupportKernel auto_kernel(uint64_t n_cand, uint32_t d, uint64_t n_words, 
     return lane_supported(d) ? SUPPORT_LANE_TM : SUPPORT_STAGED4;
 }
 
-size_t support_scratch_bytes(uint64_t n_cand, uint32_t d, uint64_t n_words, const SupportPlan &plan) {
+size_t support_scratch_bytes(uint64_t n_cand, uint32_t d, uint64_t n_words, const SupportPlan &plan,
+                             uint64_t hbm_budget) {
     const size_t base = support_scratch_bytes_for(n_cand);
-    const bool pair = plan.kernel == SUPPORT_PAIR
-                          ? pair_supported(d, n_cand)
-                          : plan.kernel == SUPPORT_AUTO && auto_kernel(n_cand, d, n_words, true) == SUPPORT_PAIR;
-    return pair ? align256(base) + pair_scratch_bytes(n_cand, d) : base;
+    if (!pair_supported(d, n_cand)) return base;
+    const size_t with_pair = align256(base) + pair_scratch_bytes(n_cand, d);
+    const bool pair = plan.kernel == SUPPORT_PAIR ||
+                      (plan.kernel == SUPPORT_AUTO && with_pair <= hbm_budget / 8 &&
+                       auto_kernel(n_cand, d, n_words, true) == SUPPORT_PAIR);
+    return pair ? with_pair : base;
 }
 
 int support_batch_device(const uint64_t *bitmaps, uint32_t d, uint64_t n_words, uint64_t row_stride,

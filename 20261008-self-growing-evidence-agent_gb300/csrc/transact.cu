@@ -571,9 +571,10 @@ template <class F> void with_median_width(uint32_t window, F &&f) {
 // stream's are given back when the call ends.
 struct TxBuffers {
     TxWorkspace &w;
-    explicit TxBuffers(TxWorkspace &ws) : w(ws) {}
+    size_t keep;
+    explicit TxBuffers(sgfim_handle *h) : w(h->tx), keep(kept_between_calls(h->hbm_budget, 1ull << 30)) {}
     ~TxBuffers() {
-        if (w.bytes() > (1ull << 30)) w.release();
+        if (w.bytes() > keep) w.release();
     }
 };
 
@@ -602,7 +603,7 @@ extern "C" int sgfim_transactionize_online(sgfim_handle *h, const double *values
     SG_CUDA_TRY(cudaSetDevice(h->device));
     cudaStream_t st = h->stream;
     const uint32_t S = n_sensors, m = n_bins - 1;
-    TxBuffers guard(h->tx);
+    TxBuffers guard(h);
     DevBuf &d_rows = h->tx.rows, &d_est = h->tx.cols, &d_out = h->tx.small, &d_anom = h->tx.anom;
     if (n_win) {
         const size_t mat = (size_t)n_rows * S * 8;
@@ -731,7 +732,7 @@ extern "C" int sgfim_transactionize(sgfim_handle *h, const double *values, uint6
     const uint32_t batch =
         (uint32_t)std::min<uint64_t>(R, std::max<uint64_t>(1, (64ull << 20) / ((uint64_t)S * kDigits * 4)));
 
-    TxBuffers guard(h->tx);
+    TxBuffers guard(h);
     DevBuf &d_rows = h->tx.rows, &d_cols = h->tx.cols, &d_small = h->tx.small, &d_anom = h->tx.anom,
            &d_items = h->tx.items;
     const size_t mat = (size_t)n_rows * S * 8;

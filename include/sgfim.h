@@ -53,7 +53,12 @@ typedef struct sgfim_handle sgfim_handle;
 
 typedef struct {
     int device;               /* CUDA device ordinal */
-    uint64_t hbm_budget;      /* bytes of device memory the engine may use; 0 = 90% of free */
+    uint64_t hbm_budget;      /* bytes of device memory the engine may use; 0 = 90% of free.  The miners'
+                                 workspaces are fractions of it and stay with the handle, as do the loaded
+                                 bitmaps and the scratch of support calls (24 bytes a candidate; in pair groups
+                                 about 110 and 12 d * d more, by AUTO only up to an eighth of the budget).  The
+                                 buffers of a transactionisation (up to 1 GB) and of a CSR being loaded (up to
+                                 64 MB) stay up to a sixteenth of it, and are given back above that */
     uint32_t wave_nodes;      /* search nodes expanded per wave; 0 = engine default */
     uint32_t flags;           /* SGFIM_F_* */
     const char *tune_cache;   /* autotuner cache file (JSON); NULL = none */
