@@ -214,7 +214,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 //   warps 0..15  expansion: a row of A (warps 0..7) or of B (8..15) per thread
 //                (half a row of the shared operand on the diagonal); wait ring_full and
 //                stage_empty, expand, fence the async proxy, arrive on
-//                ring_empty and stage_full (one arrival per warp);
+//                stage_full and ring_empty (one arrival per warp).  A ring slot is released
+//                behind the stores that used its bits: released behind the loads alone, a
+//                diagonal block now and then expanded rows of the step that refilled the
+//                slot (14 of 50,000 calls had wrong counts);
 //   warp 16      one thread issues the MMAs of a step once stage_full completes
 //                and commits them to stage_empty;
 //   warp 17      one thread keeps the TMA ring of bit slices (2 words x 256
@@ -228,7 +231,7 @@ constexpr int kT2AtomA = 256 * 128;                 // A: 256 rows x 128 B (two 
 constexpr int kT2AtomB = 256 * 128;                 // B: 256 rows x 128 B
 constexpr int kT2StageBytes = kT2AtomA + kT2AtomB;  // 64 KB
 constexpr int kT2Stages = 3;
-constexpr int kT2Ring = 3;
+constexpr int kT2Ring = 4;
 constexpr int kT2BitBox = 256 * 16;                 // one operand's slice: 256 rows x 2 words
 constexpr int kT2BitSlot = 2 * kT2BitBox;
 constexpr uint32_t kT2Idesc = (1u << 4) | ((256u >> 3) << 17) | ((128u >> 4) << 24);   // D f32, e4m3, N=256, M=128
@@ -320,8 +323,6 @@ __global__ void __launch_bounds__(kT2Threads, 1)
                     a.y = hw.y;
                 }
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&ring_empty[slot]);   // the slot's bits are in registers
             if (ok && it >= kT2Stages)
                 ok = mbar_wait_bounded(&stage_empty[s], (uint32_t)((it / kT2Stages - 1) & 1), err);
             if (!__all_sync(0xffffffffu, ok)) {
@@ -335,7 +336,10 @@ __global__ void __launch_bounds__(kT2Threads, 1)
                 expand_half(stage, r, sel, (uint64_t)a.x | ((uint64_t)a.y << 32));
             fence_proxy_async_smem();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&stage_full[s]);
+            if (lane == 0) {
+                mbar_arrive(&stage_full[s]);
+                mbar_arrive(&ring_empty[slot]);   // the slot's bits have been used (not only asked for)
+            }
         }
     } else if (warp == kT2ExpWarps) {
         // ---- MMA issue (one thread)
@@ -624,8 +628,6 @@ __global__ void __launch_bounds__(kF4Threads, 1)
                     x0 = *reinterpret_cast<const uint4 *>(src + slot * kF4RingBytes + (((group * 2) ^ sel) << 4));
                     x1 = *reinterpret_cast<const uint4 *>(src + slot * kF4RingBytes + (((group * 2 + 1) ^ sel) << 4));
                 }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&ring_empty[slot]);   // the slot's bits are in registers
                 if (ok && use) ok = mbar_wait_limit(&stage_empty[st], (use - 1) & 1, limit, err);
                 if (!__all_sync(0xffffffffu, ok)) {
                     ok = false;
@@ -644,7 +646,10 @@ __global__ void __launch_bounds__(kF4Threads, 1)
                     tc_fence_before();
                 }
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&stage_full[st]);
+                if (lane == 0) {
+                    mbar_arrive(&stage_full[st]);
+                    mbar_arrive(&ring_empty[slot]);   // the slot's bits have been used (not only asked for)
+                }
             }
             // ---- the unit's counts: warp w reads TMEM quadrant w % 4, every sixth chunk of 16 columns
             if (ok) ok = mbar_wait_limit(&done_bar, unit_n & 1, limit, err);

@@ -60,3 +60,24 @@ def test_cooc_f4_short_last_run(engine, d, words):
     rng = np.random.default_rng(d + words)
     bm = np.packbits(rng.random((d, words * 64)) < 0.2, axis=1, bitorder="little").view(np.uint64)
     assert np.array_equal(_run(engine, bm, L.COOC_AUTO), _exact(bm))
+
+
+@pytest.mark.parametrize("kind", [L.COOC_TC_F8, L.COOC_TC_F8_256, L.COOC_TC_F4])
+@pytest.mark.parametrize("d,words", [(256, 16384), (400, 4688)])
+def test_cooc_tensor_kernels_repeat_exactly(engine, kind, d, words):
+    """Thousands of calls of a tensor-core kernel agree with the popcount kernel: a ring slot that is refilled before
+    its bits are used shows in one call of a few thousand, on diagonal blocks first."""
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(d)
+    bm = torch.randint(-2**63, 2**63 - 1, (d, words), generator=g, device="cuda", dtype=torch.int64)
+    bm &= torch.randint(-2**63, 2**63 - 1, (d, words), generator=g, device="cuda", dtype=torch.int64)
+    st = torch.cuda.current_stream().cuda_stream
+    want, out = (torch.zeros((d, d), dtype=torch.int32, device="cuda") for _ in range(2))
+    engine.cooccurrence_device(bm.data_ptr(), d, words, words, want.data_ptr(), L.COOC_POPC, st)
+    bad = torch.zeros((), dtype=torch.int64, device="cuda")
+    for _ in range(8000):
+        engine.cooccurrence_device(bm.data_ptr(), d, words, words, out.data_ptr(), kind, st)
+        bad += (out != want).any()
+    assert engine.device_status(st) == 0
+    assert int(bad) == 0
