@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                   "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]),
                   "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
                 : "r"(taddr));
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            tmem_wait_ld(v);
             if (row < d) {
 #pragma unroll
                 for (int q = 0; q < 32; ++q) {
@@ -409,7 +409,7 @@ __global__ void __launch_bounds__(kT2Threads, 1)
                   "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]),
                   "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
                 : "r"(taddr));
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            tmem_wait_ld(v);
             if (row < d) {
 #pragma unroll
                 for (int c = 0; c < 32; ++c) {
@@ -677,7 +677,7 @@ __global__ void __launch_bounds__(kF4Threads, 1)
                 if (col0 >= d || row0 >= d || col0 + 15 < row0) continue;   // nothing on or above the diagonal
                 uint32_t v[16];
                 tmem_ld16(tmem + ((q * 32u) << 16) + cb, v);
-                tmem_wait_ld();
+                tmem_wait_ld(v);
                 const uint32_t row = row0 + lane;
                 __syncwarp();
 #pragma unroll

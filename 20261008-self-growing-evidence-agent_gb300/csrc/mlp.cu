@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(kFwdThreads, 2) mlp_fwd_kernel(
                 const uint32_t lanes = ((warp & 3) * 32) << 16;
                 tmem_ld16(d_top + lanes + c, t);
                 tmem_ld16(d_low + lanes + c, l);
-                tmem_wait_ld();
+                tmem_wait_ld(t, l);
 #pragma unroll
                 for (int q = 0; q < 16; q += 2)
                     unpack2(add2(pack2(__uint_as_float(t[q]), __uint_as_float(t[q + 1])),

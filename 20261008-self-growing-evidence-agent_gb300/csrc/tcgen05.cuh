@@ -44,6 +44,15 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
           "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
         : "r"(taddr));
 }
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// Waits for this warp's TMEM loads.  The arrays they filled are named: arithmetic on their
+// registers depends on the loads alone, and could be placed before a wait that does not mention them.
+template <int... N> __device__ __forceinline__ void tmem_wait_ld(uint32_t (&...v)[N]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    auto hold = [](auto &a) {
+#pragma unroll
+        for (uint32_t &x : a) asm volatile("" : "+r"(x));
+    };
+    (hold(v), ...);
+}
 
 }  // namespace sg
