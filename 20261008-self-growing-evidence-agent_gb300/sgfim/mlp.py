@@ -12,6 +12,8 @@ sgfim_mlp_backward, sgfim_adam_step).
 """
 from __future__ import annotations
 
+from operator import is_not
+
 import numpy as np
 
 from ._lib import EDEVICE
@@ -69,7 +71,7 @@ class Trainer:
         ends = np.cumsum([0] + [(v.numel() + 63) // 64 * 64 for v in self.p.values()])
         self._g_all = torch.zeros(int(ends[-1]), dtype=torch.float32, device=self.dev)
         self.g = {k: self._g_all[int(o):int(o) + v.numel()].view(v.shape) for (k, v), o in zip(self.p.items(), ends)}
-        self._g_own = dict(self.g)
+        self._g_own = tuple(self.g.values())
 
     def _refresh_bf16(self):
         for k, t in self.b16.items():
@@ -109,8 +111,8 @@ class Trainer:
         n = X.shape[0]
         P, Z1, Z2 = self.forward(X, keep=True)
         self._g_all.zero_()
-        for k, t in self.g.items():
-            if t is not self._g_own.get(k):   # the caller's tensor
+        if any(map(is_not, self.g.values(), self._g_own)):   # tensors of the caller's
+            for t in self.g.values():
                 t.zero_()
         loss = torch.zeros(1, dtype=torch.float32, device=self.dev)
         self.eng.mlp_backward(X.data_ptr(), n, self.in_dim, self.hidden, self.b16["W2"].data_ptr(),
