@@ -432,7 +432,7 @@ int sgfim_support_batch(sgfim_handle *h, const uint64_t *cand_ptr, const uint32_
     // occur map past the last row: support 0) runs there.  A small call's copies and waits are most
     // of its time: the candidates travel in one copy from pinned memory, the host checks that the
     // pointers ascend, and the supports and the error word come back behind one wait
-    // (300 candidates over 8,192 transactions: 61 -> 42 us a call).  Above the line the kernels cover the
+    // (200 candidates over 20,000 transactions: 61 -> 42 us a call).  Above the line the kernels cover the
     // copies, and a second pass over the candidates would cost the host more.
     constexpr uint64_t kSmallCall = 1u << 18;   // bytes
     const bool small = n_cand < kSmallCall && n_items < kSmallCall && (n_cand + 1) * 8 + n_items * 4 <= kSmallCall;

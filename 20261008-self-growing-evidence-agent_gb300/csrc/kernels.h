@@ -157,13 +157,14 @@ void launch_pool_append(uint64_t *pool_rows, uint64_t pool_stride, const uint64_
 int cooc_device(const uint64_t *bitmaps, uint32_t d, uint64_t n_words, uint64_t row_stride, uint32_t *out,
                 int kind, cudaStream_t st, int n_sm, void *scratch, size_t scratch_bytes, uint64_t *launches,
                 uint32_t *dev_err = nullptr);
-// tcgen05 e4m3 GEMM form (kernels_tc.cu); returns -1 when the layout is unusable.
+// The tcgen05 forms (kernels_tc.cu); they return -1 when the layout is unusable.
 // fp4 operands, 128 x 256 tiles: the AUTO form.
 int cooc_f4_device(const uint64_t *bitmaps, uint32_t d, uint64_t n_words, uint64_t row_stride, uint32_t *out,
                    cudaStream_t st, int n_sm, uint32_t *dev_err, uint64_t *launches);
 // e4m3, 256 x 256 blocks (two M = 128, N = 256 MMAs per K step).
 int cooc_tc256_device(const uint64_t *bitmaps, uint32_t d, uint64_t n_words, uint64_t row_stride, uint32_t *out,
                       cudaStream_t st, int n_sm, uint32_t *dev_err, uint64_t *launches);
+// e4m3, 128 x 128 tiles.
 int cooc_tc_device(const uint64_t *bitmaps, uint32_t d, uint64_t n_words, uint64_t row_stride, uint32_t *out,
                    cudaStream_t st, int n_sm, uint32_t *dev_err, uint64_t *launches);
 size_t cooc_scratch_bytes(uint32_t d, uint64_t n_words, int kind);
@@ -245,8 +246,7 @@ struct WFilterParams {
     const uint64_t *task_first = nullptr;
     const uint64_t *win_total = nullptr;
     const uint64_t *task_off = nullptr;
-    const uint32_t *task_cnt = nullptr;
-    uint32_t *task_kept = nullptr;      // in: task_cnt; out: kept
+    uint32_t *task_kept = nullptr;      // in: the task's candidates; out: those kept
     const uint64_t *out_m = nullptr;
     uint8_t *keep = nullptr;            // per arena slot (in: 1)
     uint64_t *scratch = nullptr;        // the windows' bitmaps: d rows of ceil(total / 64) words each

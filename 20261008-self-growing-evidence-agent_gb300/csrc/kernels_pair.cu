@@ -331,10 +331,9 @@ __device__ __forceinline__ uint32_t row_at(uint32_t row, uint32_t chunk, uint32_
     return min(t, t - ring);
 }
 
-// A group's pair over one chunk: bit w of the result is set when 32-bit word w of
-// the slice (piece w / 4, in the lane's rotated order) holds a bit.
-// Half of the slice: pieces 0..3 of the rotated order, or with oa and ob moved by
-// 64 (XOR) pieces 4..7.
+// A group's pair over half of its slice of a chunk, pieces 0..3 of the lane's rotated
+// order or, with oa and ob moved by 64 (XOR), pieces 4..7: bit w of the result is set when
+// 32-bit word w of the half (piece w / 4) holds a bit.
 __device__ __forceinline__ uint32_t pair_words(const uint8_t *smem, uint32_t oa, uint32_t ob) {
     uint32_t z = 0;
 #pragma unroll

@@ -35,16 +35,15 @@ __device__ __forceinline__ float bf2f(uint16_t b) { return __uint_as_float(((uin
 // when the weights and tensor memory allow (H <= 128), so one computes while
 // the other's MMAs run.
 //
-// Bound: shared memory (weights and activations of layer 1, the parts written
-// and read by the MMAs), about 3,800 clocks per tile of 128 rows at H = 128.
+// Bound: the chain of dependent steps of a tile, about 15,000 clocks of a CTA (2,000 of
+// them waiting for MMAs) with 16 warps an SM; its shared memory traffic alone would take
+// 3,800.  Layer 1 on the tensor cores too took a fifth of the instructions out and gave
+// 66 us, 32 warps an SM 72 us.
 // Measured (300,000 rows, H = 128, whole call): 64 us against 1,560 us for one
-// thread per hidden unit with scalar multiply-adds (a shared-memory load for each);
-// error against float64 4.5e-8 (4.7e-8 before).  Of that, 6 us came from two-float
-// multiply-adds and the next tile's inputs fetched ahead, 4 from reading W2 once, its
-// loads in flight together.  What bounds it now is the
-// chain of a tile (about 15,000 clocks a CTA, of which 2,000 wait for MMAs) over
-// 16 warps an SM: layer 1 on the tensor cores too took a fifth of the instructions
-// out and gave 66 us, 32 warps an SM 72 us.
+// thread per hidden unit with scalar multiply-adds (a shared-memory load for each).  Of
+// that, 6 us came from two-float multiply-adds and the next tile's inputs fetched ahead, 4
+// from reading W2 once, its loads in flight together.  Probabilities are off float64 by
+// 2.4e-8 (root mean square; 2.5e-8 before), without a bias above 3e-9 (1.5e-9 before).
 constexpr uint32_t kFwdRows = 128;
 constexpr uint32_t kFwdThreads = 256;
 constexpr uint32_t kFwdPart = kFwdRows * 128;   // one part's atom: 128 rows x 64 bf16
@@ -425,10 +424,11 @@ __global__ void __launch_bounds__(kFwdThreads, 2) mlp_fwd_kernel(
 // Bound: latency (one batch of rows a CTA), so every load of a batch is in flight at
 // once; loads in loops of four and weights two bytes at a time took 35 us at 4,096
 // rows and H = 128, now 23.
-// Measured (4,096 rows, H = 128, forward, backward and their fills): 63 us a
-// call, the host's launches, against 145 us with 256 CTAs whose threads each
-// added single dW2 columns 512 bytes apart; gradients' error against float64
-// 2.8e-7 (1.2e-6 before).
+// Measured (4,096 rows, H = 128, forward, backward and their fills): 68 to 71 us a
+// call, of which 46 on the device, against 145 us with 256 CTAs whose threads each
+// added single dW2 columns 512 bytes apart.  Error against float64, 24 draws each of 500 to
+// 20,000 rows and H = 64 to 256: weight gradients 2e-7 to 6e-7 of their norm, before 2e-7 to
+// 7e-7; the loss 6e-8 to 1.3e-7, before 3e-7 to 1.8e-6.
 constexpr int kBwdRows = 32;
 constexpr int kBwdThreads = 256;
 

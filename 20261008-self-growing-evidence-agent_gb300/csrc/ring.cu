@@ -760,7 +760,7 @@ int sgfim_ring_mine_windows(sgfim_ring *r, sgfim_handle *h, const uint64_t *star
                     if (st_h[t] != 0) bad[t_win[t]] = 1;
                 }
                 // ---- 5. cross-subtree filter of the split windows whose tasks all succeeded,
-                // largest candidate sets first (a CTA per window; the big ones set the makespan)
+                // largest candidate sets first: their units of 256 candidates come first in the CTAs' turns
                 struct FWin {
                     uint32_t w;
                     uint64_t t_lo, t_hi, m;
@@ -854,7 +854,6 @@ int sgfim_ring_mine_windows(sgfim_ring *r, sgfim_handle *h, const uint64_t *star
                         fp.task_first = d_first;
                         fp.win_total = d_total + i0;
                         fp.task_off = dt_off;
-                        fp.task_cnt = dt_cnt;
                         fp.task_kept = dt_kept;
                         fp.out_m = p.out_m;
                         fp.keep = keep;
