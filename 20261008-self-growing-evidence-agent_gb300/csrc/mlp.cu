@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(kFwdThreads, 2) mlp_fwd_kernel(
 // Bound: latency (one batch of rows a CTA), so every load of a batch is in flight at
 // once; loads in loops of four and weights two bytes at a time took 35 us at 4,096
 // rows and H = 128, now 23.
-// Measured (4,096 rows, H = 128, forward, backward and their fills): 68 to 71 us a
+// Measured (4,096 rows, H = 128, forward, backward and their fills): 68 to 77 us a
 // call, of which 46 on the device, against 145 us with 256 CTAs whose threads each
 // added single dW2 columns 512 bytes apart.  Error against float64, 24 draws each of 500 to
 // 20,000 rows and H = 64 to 256: weight gradients 2e-7 to 6e-7 of their norm, before 2e-7 to
